@@ -163,8 +163,10 @@ struct DevCtx {
     // Tables re-laid out on the device from P (same values, read together):
     //   ptab[med*MXGE + lgle] = {gmfp.a, gmfp.b, cohe.a, cohe.b}: the photon mean
     //     free path and Rayleigh factor of one step, the slice the photon
-    //     consumers stage in shared memory when stage_tables is set.
+    //     consumers stage in shared memory when stage_tables is set;
+    //   etab: the electron tables of a bin side by side (etab_index, dev_electron.cuh).
     const float4 *ptab;
+    const float4 *etab;
     int nmed;
     uint32_t stage_tables;          // GEGS_RUN_STAGE_TABLES of the run
     const Vox *reg;                 // nvox + 6 regions
@@ -198,7 +200,8 @@ struct DevCtx {
     float sid, iso0, iso1, iso2, z_phsp;
     float mlc_rmax, mlc_zmin, mlc_zthick, mlc_x_start, mlc_x_end, mlc_x_mid_1, mlc_x_mid_2;
     float mlc_air_gap, mlc_wl_full, mlc_wl_target, mlc_wl_isocenter, mlc_wt;
-    float2 boundaryXZ[4], boundaryYZ[4];
+    const float2 *mlc_bounds;       // [8] the MLC's bounding polygons, XZ then YZ (behind crossXZ)
+    float near_slack;               // what hownear's estimates are off by (near_error)
     int8_t module_order[8];
     uint32_t seed_lo, seed_hi;
     // beamlets: tagging grid, fluence weights (null: 1) and, in a gradient
@@ -227,22 +230,27 @@ __device__ __forceinline__ uint4 gx_philox(uint32_t c0, uint32_t c1, uint32_t c2
     return make_uint4(c0, c1, c2, c3);
 }
 
-// Per-particle stream with a window of two Philox blocks (8 words). The window
-// is refilled at one converged point per transport step (rng_window), so the
-// sampling code that draws numbers holds no inlined copy of Philox; a draw past
-// the window (rare: a step uses 5 words typically, 8 or fewer in 98 %) takes an
+// Per-particle stream with a window of two Philox blocks: eight words, word n of
+// the stream at slot n & 7 of the thread's column in shared memory. The window
+// is filled at one converged point per transport step (rng_window), so the
+// sampling code that draws numbers holds no copy of Philox; a draw past the
+// window (rare: a step uses 5 words typically, 8 or fewer in 98 %) takes an
 // out-of-line refill. Any word is a pure function of (key, counter), so where a
-// block is computed does not change the numbers.
+// block is computed does not change the numbers. In registers the window cost
+// eight of them and a selection of one of eight words at each draw, some 25
+// instructions at 5 to 30 places of a kernel.
+#define GX_MAX_THREADS 256           // threads per block of the kernels that draw
+static __shared__ uint32_t g_rng_words[8 * GX_MAX_THREADS];
+
 struct Rng {
     uint32_t hist_lo, hist_hi, sid_lo, sid_hi, ctr;
-    uint32_t wb;    // block index of w0 plus one; 0 = empty window
-    uint4 w0, w1;   // blocks wb-1 and wb
+    uint32_t wend;  // the window holds the blocks wend - 2 and wend - 1; 0 = empty
 };
 
 __device__ __forceinline__ void rng_load(Rng &r, const Part &p)
 {
     r.hist_lo = p.hist_lo; r.hist_hi = p.hist_hi; r.sid_lo = p.sid_lo; r.sid_hi = p.sid_hi;
-    r.ctr = p.ctr; r.wb = 0;
+    r.ctr = p.ctr; r.wend = 0;
 }
 
 __device__ __forceinline__ void rng_store(const Rng &r, Part &p)
@@ -250,36 +258,39 @@ __device__ __forceinline__ void rng_store(const Rng &r, Part &p)
     p.hist_lo = r.hist_lo; p.hist_hi = r.hist_hi; p.sid_lo = r.sid_lo; p.sid_hi = r.sid_hi; p.ctr = r.ctr;
 }
 
-__device__ __noinline__ uint4 rng_block(uint32_t b, uint32_t sid_lo, uint32_t sid_hi, uint32_t hist_lo,
-                                        uint32_t k0, uint32_t k1)
+__device__ __forceinline__ void rng_put(uint32_t b, uint4 x)
 {
-    return gx_philox(b, sid_lo, sid_hi, hist_lo, k0, k1);
+    uint32_t *w = g_rng_words + ((b & 1u) << 2) * GX_MAX_THREADS + threadIdx.x;
+    w[0] = x.x; w[GX_MAX_THREADS] = x.y; w[2 * GX_MAX_THREADS] = x.z; w[3 * GX_MAX_THREADS] = x.w;
+}
+
+static __device__ __noinline__ void rng_refill(uint32_t b, uint32_t sid_lo, uint32_t sid_hi, uint32_t hist_lo,
+                                               uint32_t k0, uint32_t k1)
+{
+#pragma unroll 1
+    for (uint32_t k = b; k != b + 2u; k++) rng_put(k, gx_philox(k, sid_lo, sid_hi, hist_lo, k0, k1));
 }
 
 // Make the window start at the block of the next draw (call where the warp is converged).
 __device__ __forceinline__ void rng_window(const DevCtx &C, Rng &r)
 {
     const uint32_t b = r.ctr >> 2;
-    if (r.wb == b + 1u) return;
-    if (r.wb != 0u && r.wb == b) r.w0 = r.w1;
-    else r.w0 = gx_philox(b, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi);
-    r.w1 = gx_philox(b + 1u, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi);
-    r.wb = b + 1u;
+    uint32_t k = r.wend == b + 1u ? b + 1u : b;      // the second block of the old window may be the first now
+    if (r.wend == b + 2u) return;
+#pragma unroll 1
+    for (; k != b + 2u; k++)
+        rng_put(k, gx_philox(k, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi));
+    r.wend = b + 2u;
 }
 
 __device__ __forceinline__ uint32_t rng_u32(const DevCtx &C, Rng &r)
 {
-    uint32_t k = r.ctr - ((r.wb - 1u) << 2);
-    if (r.wb == 0u || k >= 8u) {
+    if (r.wend * 4u - r.ctr - 1u >= 8u) {            // outside the window's eight words
         const uint32_t b = r.ctr >> 2;
-        r.w0 = rng_block(b, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi);
-        r.w1 = rng_block(b + 1u, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi);
-        r.wb = b + 1u;
-        k = r.ctr & 3u;
+        rng_refill(b, r.sid_lo, r.sid_hi, r.hist_lo, C.seed_lo, C.seed_hi + r.hist_hi);
+        r.wend = b + 2u;
     }
-    const uint4 w = k < 4u ? r.w0 : r.w1;
-    const uint32_t j = k & 3u;
-    const uint32_t x = j == 0 ? w.x : (j == 1 ? w.y : (j == 2 ? w.z : w.w));
+    const uint32_t x = g_rng_words[(r.ctr & 7u) * GX_MAX_THREADS + threadIdx.x];
     r.ctr++;
     return x;
 }
@@ -394,10 +405,14 @@ __device__ __forceinline__ RegInfo region_info(const DevCtx &C, uint32_t region)
     return r;
 }
 
+// Energy cuts of a region's medium (0 in vacuum).
+__device__ __forceinline__ float pcut_of(const DevCtx &C, const Vox &v) { return v.med == GX_VACUUM ? 0.0f : __ldg(&C.P->ap[v.med]); }
+__device__ __forceinline__ float ecut_of(const DevCtx &C, const Vox &v) { return v.med == GX_VACUUM ? 0.0f : __ldg(&C.P->ae[v.med]); }
+
 // Gradient replay: d(objective)/d(beamlet weight) += energy * d(objective)/d(energy in the voxel).
 // Out of line: only the replay reaches it, and inlined at every scoring site it
 // would enlarge the forward kernels.
-__device__ __noinline__ void escore_grad(const DevCtx &C, uint32_t beamlet, uint32_t region, float energy)
+static __device__ __noinline__ void escore_grad(const DevCtx &C, uint32_t beamlet, uint32_t region, float energy)
 {
     if (beamlet == GX_NO_BEAMLET) return;
     double g = (double)energy * __ldg(&C.gvm[region - GX_VAC_AND_OTH]);
@@ -431,36 +446,54 @@ __device__ __forceinline__ Part load_part(const Part *src)
     return p;
 }
 
+static __device__ __noinline__ void trace_write(TraceRec *trace, uint32_t *trace_n, uint32_t cap, TraceRec t)
+{
+    const uint32_t i = atomicAdd(trace_n, 1u);
+    if (i < cap) trace[i] = t;
+}
+
 __device__ __forceinline__ void trace_event(const DevCtx &C, uint32_t kind, int stage, const Part &p)
 {
     if (!C.trace) return;
-    uint32_t i = atomicAdd(C.trace_n, 1u);
-    if (i >= C.trace_cap) return;
     TraceRec t;
     t.kind_stage = kind | ((uint32_t)stage << 8);
     t.hist_lo = p.hist_lo; t.sid_lo = p.sid_lo; t.sid_hi = p.sid_hi; t.ctr = p.ctr;
     t.e = p.e; t.x = p.x; t.region = p.region;
-    C.trace[i] = t;
+    trace_write(C.trace, C.trace_n, C.trace_cap, t);
 }
 
-// Append one record to queue `qid`; lanes of the warp that push to the same
-// queue at the same time share one atomic.
+// A place in queue `qid` for one record of the calling lane; lanes of the warp
+// that want one of the same queue at the same time share one atomic.
+__device__ __forceinline__ uint32_t queue_place(uint32_t *count, int qid)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t same = __match_any_sync(__activemask(), qid);
+    const int leader = __ffs(same) - 1;
+    uint32_t base = 0;
+    if ((int)lane == leader) base = atomicAdd(&count[qid], (uint32_t)__popc(same));
+    return __shfl_sync(same, base, leader) + __popc(same & ((1u << lane) - 1u));
+}
+
+// Out of line, the record passed in registers: an interaction has up to ten
+// places that push.
+static __device__ __noinline__ void push_record(uint32_t *count, Part *buf, uint32_t cap, uint32_t *err, int qid, uint4 a,
+                                                uint4 b, uint4 c, uint4 d)
+{
+    const uint32_t i = queue_place(count, qid);
+    if (i < cap) {
+        uint4 *o = reinterpret_cast<uint4 *>(buf + i);
+        o[0] = a; o[1] = b; o[2] = c; o[3] = d;
+    } else atomicOr(err, GX_ERR_QUEUE_FULL);
+}
+
+// Append one record to queue `qid`.
 __device__ __forceinline__ void push(const DevCtx &C, int qid, const Part &p)
 {
-    cg::coalesced_group g = cg::coalesced_threads();
-    cg::coalesced_group sub = cg::labeled_partition(g, qid);
-    uint32_t base = 0;
-    if (sub.thread_rank() == 0) base = atomicAdd(&C.q.count[qid], (uint32_t)sub.size());
-    base = sub.shfl(base, 0);
-    uint32_t idx = base + sub.thread_rank();
-    if (idx < C.q.cap[qid]) {
-        Part r = p;
-        r.status = (uint8_t)qid;
-        store_part(&C.q.buf[qid][idx], r);
-        trace_event(C, 0u, qid, r);
-    } else {
-        atomicOr(C.err, GX_ERR_QUEUE_FULL);
-    }
+    Part r = p;
+    r.status = (uint8_t)qid;
+    trace_event(C, 0u, qid, r);
+    const uint4 *s = reinterpret_cast<const uint4 *>(&r);
+    push_record(C.q.count, C.q.buf[qid], C.q.cap[qid], C.err, qid, s[0], s[1], s[2], s[3]);
 }
 
 // push of a particle that keeps its stream (stage change)

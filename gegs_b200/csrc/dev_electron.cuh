@@ -11,7 +11,7 @@
 __device__ __forceinline__ float2 tab2(const float (*t)[2], int i) { return __ldg(reinterpret_cast<const float2 *>(t[i])); }
 __device__ __forceinline__ float ev2(float2 t, float x) { return t.x + t.y * x; }
 
-__device__ void mscat(const DevCtx &C, float lambda, float chia2, float q1, float &cost, float &sint, Rng &r)
+static __device__ void mscat(const DevCtx &C, float lambda, float chia2, float q1, float &cost, float &sint, Rng &r)
 {
     const gegs_physics *P = C.P;
     if (gx_le(lambda, 13.8)) {
@@ -117,18 +117,18 @@ __device__ __forceinline__ void sscat(const DevCtx &C, float chia2, float &cost,
     sint = sqrtf(xi * (2.0f - xi));
 }
 
-__device__ void msdist_pI(const DevCtx &C, float eloss, float tustep, Part &p0, float &ustep, const RegInfo &rd, Rng &r)
+// msdist_pI around mscat: the scattering parameters of the step, then, with the
+// sampled polar angle (ws, sint), the new direction and position.
+__device__ __forceinline__ void msdist_begin(const DevCtx &C, float eloss, float tustep, const Part &p0, float rhof,
+                                             float blccc, float xcccc, float &lambda, float &chia2, float &xi)
 {
     const gegs_physics *P = C.P;
-    unsigned medium = rd.med;
     float e0 = p0.e - P->rm;
-    float blccc = P->blcc[medium];
-    float xcccc = P->xcc[medium];
-    float e = e0 - 0.5 * eloss;
+    float e = e0 - 0.5f * eloss;              // one rounding, as in double: halving is exact
     float p2 = e * (e + P->rmt2);
-    float chia2 = xcccc / p2 / (4.0f * blccc);
+    chia2 = xcccc / p2 / (4.0f * blccc);
     float beta2 = p2 / (p2 + P->rmsq);
-    float lambda = tustep * rd.rhof * blccc / beta2;
+    lambda = tustep * rhof * blccc / beta2;
     float factor = 1 / (1 + 0.9784671 * e);
     float epsilon = eloss / e0;
     epsilon = epsilon / (1 - 0.5 * epsilon);
@@ -137,9 +137,12 @@ __device__ void msdist_pI(const DevCtx &C, float eloss, float tustep, Part &p0, 
     lambda = lambda / (1.0f + chia2);
     float chilog = gx_log(1.0f + 1.0f / chia2);
     float q1 = 2.0f * chia2 * (chilog * (1.0f + chia2) - 1.0f);
-    float xi = q1 * lambda;
-    float ws, sint;
-    mscat(C, lambda, chia2, xi, ws, sint, r);
+    xi = q1 * lambda;
+}
+
+__device__ __forceinline__ void msdist_end(const DevCtx &C, float xi, float ws, float sint, float tustep, Part &p0,
+                                           float &ustep, Rng &r)
+{
     float cphi, sphi;
     box_phi(C, r, cphi, sphi);
     float us = sint * cphi;
@@ -147,7 +150,7 @@ __device__ void msdist_pI(const DevCtx &C, float eloss, float tustep, Part &p0, 
     float z, rr, r2, z2, r2max;
     if (gx_lt(xi, 0.1)) z = 1 - xi * (0.5 - xi * (0.166666667 - 0.041666667 * xi));
     else z = (1.0f - gx_exp(-xi)) / xi;
-    rr = 0.5 * sint;
+    rr = 0.5f * sint;
     r2 = rr * rr;
     z2 = z * z;
     r2max = 1.0f - z2;
@@ -179,11 +182,14 @@ __device__ void msdist_pI(const DevCtx &C, float eloss, float tustep, Part &p0, 
     p0.w = ws;
 }
 
-__device__ __forceinline__ float range_piece(const gegs_physics *P, int qel, unsigned medium, int lel, float elk_a, float elk_b,
-                                             float e_hi, float fedep)
+// {dedx.a, dedx.b, range_ep, e_array} and {sig.a, sig.b, tmxs.a, tmxs.b} of a
+// bin (0-based) for electrons (qel 0) or positrons (1), each one 16-byte load
+// (DevCtx::etab): the tables that a step reads at one bin, side by side.
+__device__ __forceinline__ int etab_index(int qel, unsigned medium, int bin) { return ((qel * GX_MXMED + (int)medium) * GX_MXEKE + bin) * 2; }
+
+__device__ __forceinline__ float range_piece(float2 d, float elk_a, float elk_b, float e_hi, float fedep)
 {
     float elktmp = 0.5 * (elk_a + elk_b + 0.25 * fedep * fedep * (1 + fedep * (1 + 0.875 * fedep)));
-    float2 d = tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + lel - 1);
     float dedxmid = d.x + d.y * elktmp;
     dedxmid = 1.0f / dedxmid;
     float aux = d.y * dedxmid;
@@ -192,38 +198,33 @@ __device__ __forceinline__ float range_piece(const gegs_physics *P, int qel, uns
     return fedep * e_hi * dedxmid * (1.0f + aux);
 }
 
-__device__ float compute_eloss(const gegs_physics *P, int qel, unsigned medium, float step, float range, float rhof,
-                               float eke_val, float elke, int lelke)
+// Energy loss over `step`; `a` is the etab entry of the electron's own bin.
+__device__ __forceinline__ float compute_eloss(const DevCtx &C, int qel, unsigned medium, float4 a, float2 e01, float step,
+                                               float range, float rhof, float eke_val, float elke, int lelke)
 {
-    float2 ex = tab2(P->eke01, medium);
-    float de;
-    float tuss = range - __ldg(&P->range_ep[(medium * GX_MXEKE + lelke - 1) * 2 + qel]) / rhof;
-    if (tuss >= step) {
-        float2 d = tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + lelke - 1);
-        float dedxmid = d.x + d.y * elke;
-        float aux = d.y / dedxmid;
-        de = dedxmid * step * rhof;
-        float fedep = de / eke_val;
-        de = de * (1 - 0.5 * fedep * aux * (1 - 0.333333 * fedep * (aux - 1 - 0.25 * fedep * (2 - aux * (4 - aux)))));
-    } else {
-        int lelktmp = lelke;
-        tuss = (range - step) * rhof;
-        if (tuss <= 0.0f) de = eke_val - P->te[medium] * 0.99;
-        else {
-            while (lelktmp > 1 && tuss < __ldg(&P->range_ep[(medium * GX_MXEKE + lelktmp - 1) * 2 + qel])) lelktmp = lelktmp - 1;
-            float elktmp = ((float)(lelktmp + 1) - ex.x) / ex.y;
-            float eketmp = __ldg(&P->e_array[medium * GX_MXEKE + lelktmp]);
-            tuss = (__ldg(&P->range_ep[(medium * GX_MXEKE + lelktmp) * 2 + qel]) - tuss) / rhof;
-            float2 d = tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + lelktmp - 1);
-            float dedxmid = d.x + d.y * elktmp;
-            float aux = d.y / dedxmid;
-            de = dedxmid * tuss * rhof;
-            float fedep = de / eketmp;
-            de = de * (1 - 0.5 * fedep * aux * (1 - 0.333333 * fedep * (aux - 1 - 0.25 * fedep * (2 - aux * (4 - aux)))));
-            de = de + eke_val - eketmp;
+    // within the bin the loss is de(step) at the electron's energy; further, it
+    // is what is left at the bin edge reached, plus the loss down to that edge
+    float e_from = eke_val, elk = elke, len = step, below = 0.0f;
+    if (!(range - a.z / rhof >= step)) {
+        int l = lelke;
+        float left = (range - step) * rhof;
+        if (left <= 0.0f) return eke_val - C.P->te[medium] * 0.99;
+        while (l > 1 && left < a.z) {
+            l = l - 1;
+            a = __ldg(&C.etab[etab_index(qel, medium, l - 1)]);
         }
+        const float4 up = __ldg(&C.etab[etab_index(qel, medium, l)]);
+        elk = ((float)(l + 1) - e01.x) / e01.y;
+        e_from = up.w;
+        len = (up.z - left) / rhof;
+        below = 1.0f;
     }
-    return de;
+    float dedxmid = a.x + a.y * elk;
+    float aux = a.y / dedxmid;
+    float de = dedxmid * len * rhof;
+    float fedep = de / e_from;
+    de = de * (1 - 0.5 * fedep * aux * (1 - 0.333333 * fedep * (aux - 1 - 0.25 * fedep * (2 - aux * (4 - aux)))));
+    return below != 0.0f ? de + eke_val - e_from : de;
 }
 
 // state an electron carries between steps inside the electron stage
@@ -243,314 +244,282 @@ __device__ __forceinline__ void estate_init(EState &s)
 // annihilating in flight carries its total energy, above the rest mass).
 __device__ __forceinline__ bool at_rest_mark(const Part &p) { return p.e == 0.0f; }
 
-__device__ __forceinline__ void e_discard_below_cut(const DevCtx &C, Part &p, const RegInfo &rd, Rng &r)
-{
-    escore(C, p, p.region, (p.e - C.P->prm) * p.wt);
-    if (p.charge > 0) {
-        if (C.pipelined) {
-            // the photon transport of this wave runs beside this kernel and takes
-            // no new photons: the annihilation kernel, after both transports,
-            // makes them from the same random stream (region_info(p.region) is rd)
-            p.e = 0.0f;
-            push_move(C, ST_ANNIH, p, r);
-        } else annih_at_rest(C, p, rd, r);
-    }
-}
-
-// One iteration of the ELECTR loop.  Returns true when the particle has left
-// the electron stage.
-// Returns 0 while the particle stays in the electron stage, 1 when it has
-// left it, (DEFER only) 2 when the step needs howfar and (ONLY_NEAR only) 3
-// when it does not, before the step changes the particle: the caller then
-// re-queues the particle as it stood at the start of the step (howfar is the
-// first thing in the step that changes the particle; the step state and the
-// random counter are restored by the caller), and the step runs again, whole,
-// in a pass whose warps hold only such particles.
+// One iteration of the ELECTR loop (STEP_*). `vx` is the record of the
+// electron's region, kept from one step to the next. DEFER: a step that needs
+// howfar, and ONLY_NEAR: one that does not, is not taken (STEP_NEAR, STEP_FAR):
+// it returns before it changes the particle, and the caller re-queues the
+// particle as it stood at the start of the step (restoring the step state and
+// the random counter), to run it again, whole, in a pass whose warps hold only
+// such particles.
+//
+// Each routine is there once: the energy loss, the scattering angle, the
+// scoring and the ways out of all branches meet at one place each. Inlined per
+// branch they made kernels of 210 to 280 KB that waited for instructions more
+// than for anything else (22 cycles per issue in the jaws, 7 in the MLC); now
+// they take 83 to 92 KB. With the polygon routines (dev_geom.cuh) and the random
+// window in shared memory: CT head 5-field plan, 16M histories, 381 to 285 ms;
+// 1M histories 70 to 52 ms; slab, 5M histories, 96 to 90 ms.
 template <int G = GX_GEOM_ALL, bool DEFER = false, bool ONLY_NEAR = false>
-__device__ int electron_step(const DevCtx &C, Part &p, Rng &r, EState &s)
+static __device__ int electron_step(const DevCtx &C, Part &p, Rng &r, EState &s, Vox &vx, int &out)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm, rmt2 = P->rmt2, rmsq = P->rmsq;
-    uint32_t irold = p.region, irl = irold;
-    RegInfo rd = region_info(C, irl);
-    unsigned medium = rd.med;
-    float rhof = rd.rhof;
-    int lelec = p.charge;
-    int qel = (1 + lelec) / 2;
+    const uint32_t irl = p.region;
+    unsigned medium = vx.med;
+    const float rhof = vx.rhof;
+    const int qel = (1 + p.charge) / 2;
     float eie = p.e;
-    if (eie <= rd.ecut) { e_discard_below_cut(C, p, rd, r); return true; }
-    if (p.wt <= 0.0f) return true;
-    float eke_val = eie - rm;
-    if (s.is_tstep) {
-        s.compute_tstep = true;
-        if (medium != GX_VACUUM) {
-            float rnne1 = U(C, r);
-            if (rnne1 == 0.0f) rnne1 = 1.0E-30f;
-            s.demfp = fmaxf_(-gx_log(rnne1), GX_EPSEMFP);
-            s.elke = gx_log(eke_val);
-            float2 e01 = tab2(P->eke01, medium);
-            s.lelke = (int)(e01.x + e01.y * s.elke);
-            if (__ldg(&P->sig_ismonotone[medium * 2 + qel])) {
-                float sigf = ev2(tab2(P->sig, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + s.lelke - 1), s.elke);
-                float dedx0 = ev2(tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + s.lelke - 1), s.elke);
-                sigf = sigf / dedx0;
-                s.sig0 = sigf;
-            } else s.sig0 = __ldg(&P->sig_e[qel * GX_MXMED + medium]);
+    float lost = 0.0f;               // what the end of the track scores
+    bool below_cut = eie <= ecut_of(C, vx), ended = below_cut;
+    float de = 0.0f, tvstep = 0.0f, sig_val = 0.0f;
+    uint32_t irnew = irl;
+    int idisc = 0;
+    unsigned medold = medium;
+    float2 e01 = make_float2(0.0f, 0.0f);
+    if (!ended) {
+        if (p.wt <= 0.0f) return STEP_DONE;
+        float eke_val = eie - rm;
+        if (medium != GX_VACUUM) e01 = tab2(P->eke01, medium);
+        if (s.is_tstep) {
+            s.compute_tstep = true;
+            if (medium != GX_VACUUM) {
+                float rnne1 = U(C, r);
+                if (rnne1 == 0.0f) rnne1 = 1.0E-30f;
+                s.demfp = fmaxf_(-gx_log(rnne1), GX_EPSEMFP);
+                s.elke = gx_log(eke_val);
+                s.lelke = (int)(e01.x + e01.y * s.elke);
+                s.sig0 = __ldg(&P->sig_e[qel * GX_MXMED + medium]);
+            }
         }
-    }
-    const float elke = s.elke;
-    const int lelke = s.lelke;
-    float sig_val = 0.0f, dedx_val = 0.0f, tstep = 0.0f, ustep = 0.0f, tustep = 0.0f, tvstep = 0.0f, vstep = 0.0f;
-    float range = 0.0f, de = 0.0f, blccl = 0.0f, xccl = 0.0f, beta2 = 0.0f, chia2 = 0.0f, xi = 0.0f, tperp = 0.0f;
-    bool callhowfar = false, domultiple = false, dosingle = false, callmsdist = false;
-    if (medium == GX_VACUUM) {
-        tstep = GX_VACUUM_STEP;
-        ustep = tstep;
-        tustep = ustep;
-        callhowfar = true;
-    } else {
-        float2 e01 = tab2(P->eke01, medium);
-        sig_val = s.sig0;
-        if (sig_val <= 0.0f) { tstep = GX_VACUUM_STEP; s.sig0 = 1.0E-15f; }
-        else {
-            if (s.compute_tstep) {
-                float total_de = s.demfp / sig_val;
-                float ekef = eke_val - total_de;
-                if (ekef <= __ldg(&P->e_array[medium * GX_MXEKE + 0])) tstep = GX_VACUUM_STEP;
-                else {
-                    float elkef = gx_log(ekef);
-                    int lelkef = (int)(e01.x + e01.y * elkef);
-                    if (lelkef == lelke) {
-                        float fedep = 1.0f - ekef / eke_val;
-                        tstep = range_piece(P, qel, medium, lelke, elke, elkef, eke_val, fedep);
+        const float elke = s.elke;
+        const int lelke = s.lelke;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float dedx_val = 0.0f, ustep = 0.0f, tustep = 0.0f;
+        float range = 0.0f, blccl = 0.0f, xccl = 0.0f, beta2 = 0.0f, chia2 = 0.0f, xi = 0.0f, tperp = 0.0f;
+        bool callhowfar = false, domultiple = false, dosingle = false, callmsdist = false;
+        if (medium == GX_VACUUM) {
+            tustep = GX_VACUUM_STEP;
+            ustep = tustep;
+            callhowfar = true;
+        } else {
+            const float4 *bin = C.etab + etab_index(qel, medium, lelke - 1);
+            a = __ldg(bin);
+            const float4 b = __ldg(bin + 1);
+            const float dedx0 = a.x + a.y * elke;
+            if (s.is_tstep && __ldg(&P->sig_ismonotone[medium * 2 + qel])) s.sig0 = (b.x + b.y * elke) / dedx0;
+            // the range down to the bin's lower edge, and from there
+            const float to_edge = range_piece(make_float2(a.x, a.y), elke, ((float)lelke - e01.x) / e01.y, eke_val,
+                                              1.0f - a.w / eke_val);
+            float tstep;
+            sig_val = s.sig0;
+            if (sig_val <= 0.0f) { tstep = GX_VACUUM_STEP; s.sig0 = 1.0E-15f; }
+            else {
+                if (s.compute_tstep) {
+                    float ekef = eke_val - s.demfp / sig_val;
+                    if (ekef <= __ldg(&P->e_array[medium * GX_MXEKE + 0])) tstep = GX_VACUUM_STEP;
+                    else {
+                        const float elkef = gx_log(ekef);
+                        const int lelkef = (int)(e01.x + e01.y * elkef);
+                        const bool same = lelkef == lelke;
+                        float4 lo = a, up = a;
+                        float e_hi = eke_val, elk_hi = elke;
+                        if (!same) {
+                            const float4 *f = C.etab + etab_index(qel, medium, lelkef - 1);
+                            lo = __ldg(f);
+                            up = __ldg(f + 2);
+                            e_hi = up.w;
+                            elk_hi = ((float)(lelkef + 1) - e01.x) / e01.y;
+                        }
+                        tstep = range_piece(make_float2(lo.x, lo.y), elk_hi, elkef, e_hi, 1.0f - ekef / e_hi);
+                        if (!same) tstep = tstep + to_edge + a.z - up.z;
+                    }
+                    s.total_tstep = tstep;
+                    s.compute_tstep = false;
+                }
+                tstep = s.total_tstep / rhof;
+            }
+            dedx_val = rhof * dedx0;
+            float tmxs_val = (b.z + b.w * elke) / rhof;
+            range = (to_edge + a.z) / rhof;
+            tmxs_val = fminf_(tmxs_val, P->smaxir[medium]);
+            tustep = fminf_(tstep, fminf_(tmxs_val, range));
+            NearUse use;
+            use.rr = P->i_do_rr[medium] == 1 && p.e < P->e_max_rr[medium];
+            use.range = range;
+            use.tustep = tustep;
+            bool ok;
+            hownear_g<G>(C, p, tperp, ok, use);
+            if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return STEP_DONE; }
+            if (use.rr && tperp >= range) below_cut = ended = true;
+            else {
+                const float blcc = P->blcc[medium], xcc = P->xcc[medium];
+                blccl = rhof * blcc;
+                xccl = rhof * xcc;
+                float p2 = eke_val * (eke_val + rmt2);
+                beta2 = p2 / (p2 + rmsq);
+                float ssmfp = beta2 / blccl;
+                float skindepth = P->skindepth_for_bca * ssmfp;
+                tustep = fminf_(tustep, fmaxf_(tperp, skindepth));
+                if (tustep <= tperp && (!P->exact_bca || tustep > skindepth)) {
+                    if (ONLY_NEAR) return STEP_FAR;
+                    callmsdist = true;
+                } else {
+                    if (P->exact_bca) {
+                        float rnnoss = U(C, r);
+                        float lambda = -gx_log(1.0f - rnnoss);
+                        float tmp = (eke_val / rm + 1.0f);
+                        float lambda_max = 0.5 * blccl * rm / dedx_val * tmp * tmp * tmp;
+                        if (!(lambda >= 0.0f && lambda_max > 0.0f)) return STEP_DONE;
+                        float tuss;
+                        if (lambda < lambda_max) tuss = lambda * ssmfp * (1 - 0.5 * lambda / lambda_max);
+                        else tuss = 0.5 * lambda * ssmfp;
+                        if (tuss < tustep) { tustep = tuss; dosingle = true; }
+                        ustep = tustep;
                     } else {
-                        float ekei = __ldg(&P->e_array[medium * GX_MXEKE + lelke - 1]);
-                        float elkei = ((float)lelke - e01.x) / e01.y;
-                        float fedep = 1.0f - ekei / eke_val;
-                        float tuss = range_piece(P, qel, medium, lelke, elke, elkei, eke_val, fedep);
-                        ekei = __ldg(&P->e_array[medium * GX_MXEKE + lelkef]);
-                        elkei = ((float)(lelkef + 1) - e01.x) / e01.y;
-                        fedep = 1.0f - ekef / ekei;
-                        tstep = range_piece(P, qel, medium, lelkef, elkei, elkef, ekei, fedep);
-                        tstep = tstep + tuss + __ldg(&P->range_ep[(medium * GX_MXEKE + lelke - 1) * 2 + qel])
-                                - __ldg(&P->range_ep[(medium * GX_MXEKE + lelkef) * 2 + qel]);
+                        domultiple = true;
+                        float ekems = eke_val - 0.5 * tustep * dedx_val;
+                        p2 = ekems * (ekems + rmt2);
+                        beta2 = p2 / (p2 + rmsq);
+                        chia2 = xccl / (4.0f * blccl * p2);
+                        xi = 0.5 * xccl / p2 / beta2 * tustep;
+                        xi = xi * (gx_log((float)(1 + 1.0 / chia2)) - 1 / (1 + chia2));
+                        if (gx_lt(xi, 0.1)) ustep = tustep * (1 - xi * (0.5 - xi * 0.166667));
+                        else ustep = tustep * (1.0f - gx_exp(-xi)) / xi;
+                    }
+                    callhowfar = !(ustep < tperp);
+                    if (ONLY_NEAR && !callhowfar) return STEP_FAR;
+                }
+            }
+        }
+        const float ustep0 = ustep;
+        if (!ended && callhowfar) {
+            if (DEFER) return STEP_NEAR;
+            bool ok;
+            irnew = howfar_g<G>(C, p, ustep, ok);
+            if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return STEP_DONE; }
+            if (irnew == 0) {
+                if (medium == GX_VACUUM || p.leafIndex == GX_PASSMLC) { p.region = 0; return STEP_DONE; }   // left the geometry
+                idisc = -1;
+            }
+        }
+        if (!ended && !callmsdist) {
+            if (ustep <= 0.0f) ustep = 0.0f;
+            if (ustep == 0.0f || medium == GX_VACUUM) {
+                if (ustep != 0.0f) {
+                    p.x = p.x + p.u * ustep;
+                    p.y = p.y + p.v * ustep;
+                    p.z = p.z + p.w * ustep;
+                }
+                p.region = irnew;
+                vx = C.reg[irnew];
+                below_cut = eie <= ecut_of(C, vx);
+                ended = below_cut || (ustep != 0.0f && idisc < 0);
+                if (!ended) { s.is_tstep = true; return STEP_ON; }
+            }
+        }
+        if (!ended) {
+            const float vstep = ustep;
+            tvstep = tustep;
+            if (callhowfar) {
+                if (P->exact_bca) {
+                    tvstep = vstep;
+                    if (tvstep != tustep) dosingle = false;
+                } else if (vstep < ustep0) {
+                    float ekems = eke_val - 0.5 * tustep * vstep / ustep0 * dedx_val;
+                    float p2 = ekems * (ekems + rmt2);
+                    beta2 = p2 / (p2 + rmsq);
+                    chia2 = xccl / (4.0f * blccl * p2);
+                    xi = 0.5 * xccl / p2 / beta2 * vstep;
+                    xi = xi * (gx_log((float)(1 + 1.0 / chia2)) - 1 / (1 + chia2));
+                    if (gx_lt(xi, 0.1)) tvstep = vstep * (1 + xi * (0.5 + xi * 0.333333));
+                    else {
+                        if (gx_lt(xi, 0.999999)) tvstep = -vstep * gx_log(1 - xi) / xi;
+                        else return STEP_DONE;
                     }
                 }
-                s.total_tstep = tstep;
-                s.compute_tstep = false;
             }
-            tstep = s.total_tstep / rhof;
-        }
-        float dedx0 = ev2(tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + lelke - 1), elke);
-        dedx_val = rhof * dedx0;
-        float tmxs_val = ev2(tab2(P->tmxs, medium * GX_MXEKE + lelke - 1), elke);
-        tmxs_val = tmxs_val / rhof;
-        {
-            float ekei = __ldg(&P->e_array[medium * GX_MXEKE + lelke - 1]);
-            float elkei = ((float)lelke - e01.x) / e01.y;
-            float fedep = 1.0f - ekei / eke_val;
-            range = range_piece(P, qel, medium, lelke, elke, elkei, eke_val, fedep);
-            range = (range + __ldg(&P->range_ep[(medium * GX_MXEKE + lelke - 1) * 2 + qel])) / rhof;
-        }
-        tmxs_val = fminf_(tmxs_val, P->smaxir[medium]);
-        tustep = fminf_(tstep, fminf_(tmxs_val, range));
-        const bool do_rr = P->i_do_rr[medium] == 1 && p.e < P->e_max_rr[medium];
-        // In the jaws, a lower bound of hownear above the thresholds it is
-        // compared with (range for range rejection, else tustep) decides every
-        // comparison below as the exact value would, and then tustep is left
-        // unchanged: the bound stands in for the value.
-        float lb = -1.0f;
-        if (G == GX_GEOM_JAWS && (p.module == GEGS_M_SECJAWY || p.module == GEGS_M_SECJAWX))
-            lb = jaws_near_lower_bound(C, p);
-        if (lb > (do_rr ? range : tustep)) tperp = lb;
-        else {
-            bool ok;
-            hownear_g<G>(C, p, tperp, ok);
-            if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return true; }
-        }
-        if (do_rr) {
-            if (tperp >= range) { e_discard_below_cut(C, p, rd, r); return true; }
-        }
-        blccl = rhof * P->blcc[medium];
-        xccl = rhof * P->xcc[medium];
-        float p2 = eke_val * (eke_val + rmt2);
-        beta2 = p2 / (p2 + rmsq);
-        float ssmfp = beta2 / blccl;
-        float skindepth = P->skindepth_for_bca * ssmfp;
-        tustep = fminf_(tustep, fmaxf_(tperp, skindepth));
-        if (tustep <= tperp && (!P->exact_bca || tustep > skindepth)) {
-            callmsdist = true;
-            de = compute_eloss(P, qel, medium, tustep, range, rhof, eke_val, elke, lelke);
-            tvstep = tustep;
-            if (ONLY_NEAR) return 3;
-            msdist_pI(C, de, tustep, p, ustep, rd, r);
-        } else {
-            if (P->exact_bca) {
-                float rnnoss = U(C, r);
-                float lambda = -gx_log(1.0f - rnnoss);
-                float tmp = (eke_val / rm + 1.0f);
-                float lambda_max = 0.5 * blccl * rm / dedx_val * tmp * tmp * tmp;
-                if (lambda >= 0.0f && lambda_max > 0.0f) {
-                    float tuss;
-                    if (lambda < lambda_max) tuss = lambda * ssmfp * (1 - 0.5 * lambda / lambda_max);
-                    else tuss = 0.5 * lambda * ssmfp;
-                    if (tuss < tustep) { tustep = tuss; dosingle = true; } else dosingle = false;
-                } else return true;
-                ustep = tustep;
-            } else {
-                domultiple = true;
-                float ekems = eke_val - 0.5 * tustep * dedx_val;
-                p2 = ekems * (ekems + rmt2);
-                beta2 = p2 / (p2 + rmsq);
-                chia2 = xccl / (4.0f * blccl * p2);
-                xi = 0.5 * xccl / p2 / beta2 * tustep;
-                xi = xi * (gx_log((float)(1 + 1.0 / chia2)) - 1 / (1 + chia2));
-                if (gx_lt(xi, 0.1)) ustep = tustep * (1 - xi * (0.5 - xi * 0.166667));
-                else ustep = tustep * (1.0f - gx_exp(-xi)) / xi;
-            }
-            callhowfar = !(ustep < tperp);
-            if (ONLY_NEAR && !callhowfar) return 3;
-        }
-    }
-    uint32_t irnew = p.region;
-    int idisc = 0;
-    float ustep0 = ustep;
-    if (callhowfar || p.wt <= 0.0f) {
-        if (DEFER) return 2;
-        bool ok;
-        irnew = howfar_g<G>(C, p, ustep, ok);
-        if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return true; }
-    }
-    if (irnew == 0) {
-        if (rd.med == GX_VACUUM || p.leafIndex == GX_PASSMLC) idisc = 1; else idisc = -1;
-    }
-    if (idisc > 0) {
-        p.region = 0;
-        escore(C, p, 0, (p.e + (float)p.charge * prm) * p.wt);
-        return true;
-    }
-    if (ustep <= 0.0f) ustep = 0.0f;
-    if (ustep == 0.0f || medium == GX_VACUUM) {
-        if (ustep != 0.0f) {
-            vstep = ustep;
-            p.x = p.x + p.u * vstep;
-            p.y = p.y + p.v * vstep;
-            p.z = p.z + p.w * vstep;
-        }
-        p.region = irnew;
-        rd = region_info(C, irnew);
-        if (eie <= rd.ecut) { e_discard_below_cut(C, p, rd, r); return true; }
-        if (ustep != 0.0f && idisc < 0) {
-            escore(C, p, p.region, (p.e + (float)p.charge * prm) * p.wt);
-            return true;
-        }
-        s.is_tstep = true;
-        return false;
-    }
-    vstep = ustep;
-    if (callhowfar) {
-        if (P->exact_bca) {
-            tvstep = vstep;
-            if (tvstep != tustep) dosingle = false;
-        } else {
-            if (vstep < ustep0) {
-                float ekems = eke_val - 0.5 * tustep * vstep / ustep0 * dedx_val;
+            de = compute_eloss(C, qel, medium, a, e01, tvstep, range, rhof, eke_val, elke, lelke);
+            float sinthe = 0.0f, costhe = 1.0f, lambda = 0.0f;
+            if (callmsdist) msdist_begin(C, de, tustep, p, rhof, P->blcc[medium], P->xcc[medium], lambda, chia2, xi);
+            else if (domultiple) lambda = blccl * tvstep / beta2 / 1.0f / (1.0f + chia2);
+            if (callmsdist || domultiple) mscat(C, lambda, chia2, xi, costhe, sinthe, r);
+            else if (dosingle) {
+                float ekems = fmaxf_(eke_val - de, ecut_of(C, vx) - rm);
                 float p2 = ekems * (ekems + rmt2);
-                beta2 = p2 / (p2 + rmsq);
-                chia2 = xccl / (4.0f * blccl * p2);
-                xi = 0.5 * xccl / p2 / beta2 * vstep;
-                xi = xi * (gx_log((float)(1 + 1.0 / chia2)) - 1 / (1 + chia2));
-                if (gx_lt(xi, 0.1)) tvstep = vstep * (1 + xi * (0.5 + xi * 0.333333));
-                else {
-                    if (gx_lt(xi, 0.999999)) tvstep = -vstep * gx_log(1 - xi) / xi;
-                    else return true;
+                chia2 = P->xcc[medium] / (4.0f * P->blcc[medium] * p2);
+                sscat(C, chia2, costhe, sinthe, r);
+            }
+            if (callmsdist) {
+                msdist_end(C, xi, costhe, sinthe, tustep, p, ustep, r);
+                if (ustep <= 0.0f) { s.is_tstep = true; return STEP_ON; }
+            } else {
+                p.x = p.x + p.u * vstep;
+                p.y = p.y + p.v * vstep;
+                p.z = p.z + p.w * vstep;
+                if (domultiple || dosingle) {
+                    float sinphi, cosphi;
+                    uphi21(C, costhe, sinthe, cosphi, sinphi, p, r);
                 }
-            } else tvstep = tustep;
-        }
-        de = compute_eloss(P, qel, medium, tvstep, range, rhof, eke_val, elke, lelke);
-    } else {
-        tvstep = tustep;
-        if (!callmsdist) de = compute_eloss(P, qel, medium, tvstep, range, rhof, eke_val, elke, lelke);
-    }
-    float save_de = de;
-    float edep = de;
-    float ekef = eke_val - de;
-    if (!callmsdist) {
-        float sinthe = 0.0f, costhe = 0.0f;
-        if (domultiple) {
-            float lambda = blccl * tvstep / beta2 / 1.0f / (1.0f + chia2);
-            mscat(C, lambda, chia2, xi, costhe, sinthe, r);
-        } else if (dosingle) {
-            float ekems = fmaxf_(ekef, rd.ecut - rm);
-            float p2 = ekems * (ekems + rmt2);
-            beta2 = p2 / (p2 + rmsq);
-            chia2 = P->xcc[medium] / (4.0f * P->blcc[medium] * p2);
-            sscat(C, chia2, costhe, sinthe, r);
-        } else { sinthe = 0.0f; costhe = 1.0f; }
-        p.x = p.x + p.u * vstep;
-        p.y = p.y + p.v * vstep;
-        p.z = p.z + p.w * vstep;
-        if (domultiple || dosingle) {
-            float sinphi, cosphi;
-            uphi21(C, costhe, sinthe, cosphi, sinphi, p, r);
+            }
+            eie = eie - de;
+            p.e = eie;
+            escore(C, p, irl, de * p.wt);
+            below_cut = irnew == irl && eie <= ecut_of(C, vx);
+            if (!below_cut) {
+                s.elke = gx_log(eie - rm);
+                s.lelke = (int)(e01.x + e01.y * s.elke);
+                if (irnew != irl) {
+                    p.region = irnew;
+                    vx = C.reg[irnew];
+                    medium = vx.med;
+                }
+                below_cut = eie <= ecut_of(C, vx);
+            }
+            ended = below_cut || idisc < 0;
         }
     }
-    irold = p.region;
-    eie = eie - edep;
-    p.e = eie;
-    escore(C, p, irold, edep * p.wt);
-    if (irnew == irl && eie <= rd.ecut) { e_discard_below_cut(C, p, rd, r); return true; }
-    unsigned medold = medium;
-    if (medium != GX_VACUUM) {
-        eke_val = eie - rm;
-        s.elke = gx_log(eke_val);
-        float2 e01 = tab2(P->eke01, medium);
-        s.lelke = (int)(e01.x + e01.y * s.elke);
+    if (ended) {
+        // below the cut: the kinetic energy stays here, and a positron at rest goes to
+        // the annihilation kernel, which makes its photons from the same random stream
+        // (energy 0 marks it); out of the geometry: all of it
+        lost = below_cut ? p.e - prm : p.e + (float)p.charge * prm;
+        escore(C, p, p.region, lost * p.wt);
+        if (!below_cut || p.charge <= 0) return STEP_DONE;
+        p.e = 0.0f;
+        out = ST_ANNIH;
+        return STEP_QUEUE;
     }
-    if (irnew != irold) {
-        p.region = irnew;
-        irl = irnew;
-        rd = region_info(C, irl);
-        medium = rd.med;
-    }
-    if (eie <= rd.ecut) { e_discard_below_cut(C, p, rd, r); return true; }
-    if (idisc < 0) {
-        escore(C, p, p.region, (p.e + (float)p.charge * prm) * p.wt);
-        return true;
-    }
-    if (medium != medold) { s.is_tstep = true; return false; }
-    s.demfp = s.demfp - save_de * sig_val;
+    if (medium != medold) { s.is_tstep = true; return STEP_ON; }
+    s.demfp = s.demfp - de * sig_val;
     s.total_tstep = s.total_tstep - tvstep * rhof;
     if (gx_lt(s.total_tstep, 1e-9)) s.demfp = 0.0f;
-    if (gx_ge(s.demfp, GX_EPSEMFP)) { s.is_tstep = false; return false; }
-    float sigf = ev2(tab2(P->sig, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + s.lelke - 1), s.elke);
-    float dedx0 = ev2(tab2(P->dedx, qel * GX_MXEKE * GX_MXMED + medium * GX_MXEKE + s.lelke - 1), s.elke);
-    sigf = sigf / dedx0;
-    float sigratio = sigf / s.sig0;
-    float rfict = U(C, r);
-    if (rfict > sigratio) { s.is_tstep = true; return false; }
-    if (lelec < 0) {
-        float ebr1_val = ev2(tab2(P->ebr1, medium * GX_MXEKE + s.lelke - 1), s.elke);
-        float rnno24 = U(C, r);
-        if (rnno24 <= ebr1_val) { push_move(C, ST_BREMS, p, r); return true; }
-        if (p.e <= P->thmoll[medium] && P->eii_flag == 0) {
-            if (ebr1_val <= 0.0f) { s.is_tstep = true; return false; }
-            push_move(C, ST_BREMS, p, r);
-            return true;
-        }
-        push_move(C, ST_MOLLER, p, r);
-        return true;
+    if (gx_ge(s.demfp, GX_EPSEMFP)) { s.is_tstep = false; return STEP_ON; }
+    const float4 *bin = C.etab + etab_index(qel, medium, s.lelke - 1);
+    const float4 a = __ldg(bin), b = __ldg(bin + 1);
+    const float sigf = (b.x + b.y * s.elke) / (a.x + a.y * s.elke);
+    const float sigratio = sigf / s.sig0;
+    const float rfict = U(C, r);
+    s.is_tstep = true;
+    if (rfict > sigratio) return STEP_ON;
+    const int tab = medium * GX_MXEKE + s.lelke - 1;
+    if (p.charge < 0) {
+        const float ebr1_val = ev2(tab2(P->ebr1, tab), s.elke);
+        const float rnno24 = U(C, r);
+        if (rnno24 <= ebr1_val) out = ST_BREMS;
+        else if (p.e <= P->thmoll[medium] && P->eii_flag == 0) {
+            if (ebr1_val <= 0.0f) return STEP_ON;
+            out = ST_BREMS;
+        } else out = ST_MOLLER;
+        return STEP_QUEUE;
     }
-    float pbr1_val = ev2(tab2(P->pbr1, medium * GX_MXEKE + s.lelke - 1), s.elke);
-    float rnno25 = U(C, r);
-    if (rnno25 < pbr1_val) { push_move(C, ST_BREMS, p, r); return true; }
-    float pbr2_val = ev2(tab2(P->pbr2, medium * GX_MXEKE + s.lelke - 1), s.elke);
-    if (rnno25 < pbr2_val) push_move(C, ST_BHABHA, p, r);
-    else push_move(C, ST_ANNIH, p, r);
-    return true;
+    const float pbr1_val = ev2(tab2(P->pbr1, tab), s.elke);
+    const float rnno25 = U(C, r);
+    if (rnno25 < pbr1_val) out = ST_BREMS;
+    else out = rnno25 < ev2(tab2(P->pbr2, tab), s.elke) ? ST_BHABHA : ST_ANNIH;
+    return STEP_QUEUE;
 }
 
-__device__ void eii_sample(const DevCtx &C, int ish, int iz, float uj, Part &p, const RegInfo &rd, Rng &r, float &edep)
+static __device__ void eii_sample(const DevCtx &C, int ish, int iz, float uj, Part &p, const RegInfo &rd, Rng &r, float &edep)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm, rmt2 = P->rmt2;
@@ -612,7 +581,7 @@ __device__ void eii_sample(const DevCtx &C, int ish, int iz, float uj, Part &p, 
     relax(C, uj, ish, iz, edep, p, rd, r);
 }
 
-__device__ void moller(const DevCtx &C, Part p, Rng &r)
+static __device__ void moller(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -704,7 +673,7 @@ __device__ void moller(const DevCtx &C, Part p, Rng &r)
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void brems(const DevCtx &C, Part p, Rng &r)
+static __device__ void brems(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -824,7 +793,7 @@ __device__ void brems(const DevCtx &C, Part p, Rng &r)
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void bhabha(const DevCtx &C, Part p, Rng &r)
+static __device__ void bhabha(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -885,7 +854,7 @@ __device__ void bhabha(const DevCtx &C, Part p, Rng &r)
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void annih(const DevCtx &C, Part p, Rng &r)
+static __device__ void annih(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;

@@ -46,7 +46,7 @@ __device__ __forceinline__ int is_where(float p, uint32_t nreg, const float *bou
     return mu - 1;
 }
 
-__device__ uint32_t howfar_phantom(const DevCtx &C, const Part &p0, float &t)
+static __device__ uint32_t howfar_phantom(const DevCtx &C, const Part &p0, float &t)
 {
     const float *xb = C.xb, *yb = C.yb, *zb = C.zb;
     uint32_t Nx = (uint32_t)C.nx, Ny = (uint32_t)C.ny, Nz = (uint32_t)C.nz;
@@ -124,7 +124,7 @@ __device__ uint32_t howfar_phantom(const DevCtx &C, const Part &p0, float &t)
     return 0;
 }
 
-__device__ void hownear_phantom(const DevCtx &C, const Part &p0, float &tperp)
+static __device__ void hownear_phantom(const DevCtx &C, const Part &p0, float &tperp)
 {
     const float *xb = C.xb, *yb = C.yb, *zb = C.zb;
     uint32_t Nx = (uint32_t)C.nx, Ny = (uint32_t)C.ny, Nz = (uint32_t)C.nz;
@@ -155,28 +155,31 @@ __device__ void hownear_phantom(const DevCtx &C, const Part &p0, float &tperp)
 }
 
 // ---- polygons (2-D points as float2) ----------------------------------------
+// The instruction cache is the scarcest resource of the beam-line kernels: with
+// each polygon test inlined and unrolled where it is used they took 80 to 280 KB
+// of code and waited for instructions first of all. So each routine has one
+// loop over its polygons, the loops over edges stay rolled and without
+// branches, and what only few edges need (the divisions) follows for those
+// edges alone, picked out by a bit mask. The photon kernels of the jaws and the
+// MLC went from 97 and 83 KB to 30 and 33 KB (times: electron_step).
 __device__ __forceinline__ float2 ld2(const float2 *a) { return __ldg(a); }
 
-__device__ int point_in_polygon(float2 p, const float2 *poly, int n)
+static __device__ __noinline__ int point_in_polygon(float px, float py, const float2 *poly, int n)
 {
-    int j = n - 1, odd = 0;
+    uint32_t cross = 0;
+    float2 b = ld2(&poly[n - 1]);
+#pragma unroll 2
     for (int i = 0; i < n; i++) {
-        float2 a = ld2(&poly[i]), b = ld2(&poly[j]);
-        if (((a.y < p.y && b.y >= p.y) || (b.y < p.y && a.y >= p.y)) && (a.x <= p.x || b.x <= p.x))
-            odd ^= (a.x + (p.y - a.y) / (b.y - a.y) * (b.x - a.x) < p.x);
-        j = i;
+        const float2 a = ld2(&poly[i]);
+        if ((a.y < py) != (b.y < py) && (a.y >= py || b.y >= py) && (a.x <= px || b.x <= px)) cross |= 1u << i;
+        b = a;
     }
-    return odd;
-}
-
-__device__ int point_in_polygon_local(float2 p, const float2 *poly, int n)
-{
-    int j = n - 1, odd = 0;
-    for (int i = 0; i < n; i++) {
-        float2 a = poly[i], b = poly[j];
-        if (((a.y < p.y && b.y >= p.y) || (b.y < p.y && a.y >= p.y)) && (a.x <= p.x || b.x <= p.x))
-            odd ^= (a.x + (p.y - a.y) / (b.y - a.y) * (b.x - a.x) < p.x);
-        j = i;
+    int odd = 0;
+    while (cross) {
+        const int i = __ffs(cross) - 1;
+        cross &= cross - 1u;
+        const float2 a = ld2(&poly[i]), c = ld2(&poly[i ? i - 1 : n - 1]);
+        odd ^= (a.x + (py - a.y) / (c.y - a.y) * (c.x - a.x) < px);
     }
     return odd;
 }
@@ -186,15 +189,15 @@ __device__ __forceinline__ const float2 *endnode_of(const DevCtx &C, int field, 
     return reinterpret_cast<const float2 *>(&C.fields[field].endnode[leaf][0][0]);
 }
 
-__device__ int point_in_leaf(float2 p, const float2 *endn)
+static __device__ int point_in_leaf(float2 p, const float2 *endn)
 {
     int bank = 0;
-    if (point_in_polygon(p, endn, 17)) bank = 1;
-    else if (point_in_polygon(p, endn + 17, 17)) bank = 2;
+    if (point_in_polygon(p.x, p.y, endn, 17)) bank = 1;
+    else if (point_in_polygon(p.x, p.y, endn + 17, 17)) bank = 2;
     return bank;
 }
 
-__device__ int index_of_leaf(const DevCtx &C, float2 p)
+static __device__ __noinline__ int index_of_leaf(const DevCtx &C, float2 p)
 {
     int i = GX_OUTMLC, index = GX_OUTMLC;
     float x = p.x / p.y * C.mlc_zmin;
@@ -215,59 +218,73 @@ __device__ int index_of_leaf(const DevCtx &C, float2 p)
     else if (x <= C.mlc_x_end)
         i = 58;
     if (i >= 0) {
-        if (point_in_polygon(p, C.crossXZ + i * 16, 14)) index = i;
+        if (point_in_polygon(p.x, p.y, C.crossXZ + i * 16, 14)) index = i;
         else if (i < 59) {
-            if (point_in_polygon(p, C.crossXZ + (i + 1) * 16, 14)) index = i + 1;
+            if (point_in_polygon(p.x, p.y, C.crossXZ + (i + 1) * 16, 14)) index = i + 1;
             else index = -(i + 1);
         } else index = GX_OUTMLC;
     }
     return index;
 }
 
-// (u >= 0 && u < 1) for u = fl(num / den), den != 0, deciding from num and
-// den without the division where the outcome is certain and dividing
-// otherwise, so the decision is always that of the rounded quotient:
-// with n = num * sign(den) and d = |den| (exact), fl(num / den) = fl(n / d);
-// n < -d * 1e-30 gives a negative quotient that does not round to zero; n >= d
-// a quotient >= 1; 0 <= n <= d * (1 - 2^-20) a quotient below 1 - 2^-21.
-__device__ __forceinline__ bool edge_param_in_unit(float num, float den)
+// An edge's terms in the ray's intersection with it: the edge parameter is
+// num / den, the distance dn / den (rayIntersectPolygon, geom.cu; the
+// differences are taken the other way round, which changes no rounding).
+__device__ __forceinline__ void ray_edge(float2 p0, float2 v, float2 a, float2 b, float &num, float &den, float &dn)
 {
-    float n = den > 0.0f ? num : -num;
-    float d = fabsf(den);
-    if (n < -d * 1e-30f) return false;
-    if (n >= d) return false;
-    if (n >= 0.0f && n <= d * 0.99999904632568359375f) return true;
-    float u = num / den;
-    return (u >= 0) && (u < 1);
+    const float ex = b.x - a.x, ey = b.y - a.y, dx = a.x - p0.x, dy = a.y - p0.y;
+    den = v.x * ey - v.y * ex;
+    num = dx * v.y - dy * v.x;
+    dn = ey * dx - ex * dy;
 }
 
-template <bool LOCAL>
-__device__ float ray_intersect_polygon(float2 p0, float2 v, const float2 *poly, int n, int &inside)
+// The nearest edge in front of the ray, and the parity of the edges hit. An
+// edge is hit where u = fl(num / den) lies in [0, 1) and fl(dn / den) >= 0.
+// First the edges for which that is possible, from the signs and sizes of num,
+// den and dn alone: with d = |den| and the others carrying den's sign, n >= d
+// makes u >= 1, and n or m below -d * 1e-30 makes a quotient negative that does
+// not round to zero. Then the quotients of those edges, one or two of a
+// polygon; u only where n is not certainly below d (1 - 2^-20).
+__device__ __forceinline__ float ray_intersect_polygon(float2 p0, float2 v, const float2 *poly, int n, int &inside)
 {
+    uint32_t hit = 0;
+    const float2 first = ld2(poly);
+    float2 a = first;
+#pragma unroll 2
+    for (int i = 0; i < n; i++) {
+        const float2 b = i + 1 < n ? ld2(&poly[i + 1]) : first;
+        float num, den, dn;
+        ray_edge(p0, v, a, b, num, den, dn);
+        const uint32_t sign = __float_as_uint(den) & 0x80000000u;
+        const float d = fabsf(den), least = d * -1e-30f;
+        const float u = __uint_as_float(__float_as_uint(num) ^ sign), m = __uint_as_float(__float_as_uint(dn) ^ sign);
+        if (u >= least && u < d && m >= least) hit |= 1u << i;
+        a = b;
+    }
     float minDist = GX_INFI_DIST + 1;
     int count = 0;
-    for (int i = 0; i < n; i++) {
-        int j = i + 1;
-        if (j >= n) j = 0;
-        float2 a = LOCAL ? poly[i] : ld2(&poly[i]);
-        float2 b = LOCAL ? poly[j] : ld2(&poly[j]);
-        float tmp1 = v.x * (b.y - a.y) - v.y * (b.x - a.x);
-        if (tmp1 != 0) {
-            // the edge parameter first: most edges fail it, and then the distance is not needed
-            if (edge_param_in_unit(((a.x - p0.x) * v.y - (a.y - p0.y) * v.x), tmp1)) {
-                float dist = ((b.x - a.x) * (p0.y - a.y) - (b.y - a.y) * (p0.x - a.x)) / tmp1;
-                if (dist >= 0) {
-                    count++;
-                    if (dist < minDist) minDist = dist;
-                }
-            }
+    while (hit) {
+        const int i = __ffs(hit) - 1;
+        hit &= hit - 1u;
+        float num, den, dn;
+        ray_edge(p0, v, ld2(&poly[i]), i + 1 < n ? ld2(&poly[i + 1]) : first, num, den, dn);
+        const float d = fabsf(den);
+        const float u = den > 0.0f ? num : -num;
+        if (!(u >= 0.0f && u <= d * 0.99999904632568359375f)) {
+            const float q = num / den;
+            if (!(q >= 0 && q < 1)) continue;
+        }
+        const float dist = dn / den;
+        if (dist >= 0) {
+            count++;
+            if (dist < minDist) minDist = dist;
         }
     }
     inside = count & 1;
     return minDist;
 }
 
-__device__ uint32_t inwhere_mlc(const DevCtx &C, int field, float qx, float qy, float qz, int &index, int &bank)
+static __device__ uint32_t inwhere_mlc(const DevCtx &C, int field, float qx, float qy, float qz, int &index, int &bank)
 {
     uint32_t inew = 1;
     float2 p = make_float2(qx, qz);
@@ -280,83 +297,88 @@ __device__ uint32_t inwhere_mlc(const DevCtx &C, int field, float qx, float qy, 
     return inew;
 }
 
-__device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
+static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
 {
     const Part p = p0;
     uint32_t inew = p.region;
     int bank = p.bank;
     int index = p.leafIndex;
-    int indexLimit1 = 0, indexLimit2 = 60;
     if (p.y < -C.mlc_rmax || p.y > C.mlc_rmax) return 0;
-    float minDist, minBoundaryDist;
-    float dis_xz, dis_yz, temp1 = GX_INFI_DIST + 1;
-    float2 p1 = make_float2(p.x, p.z), p2 = make_float2(p.y, p.z);
-    float2 dir1 = make_float2(p.u, p.w), dir2 = make_float2(p.v, p.w), p3;
-    int inside_XZ, inside_YZ;
-    dis_xz = ray_intersect_polygon<true>(p1, dir1, C.boundaryXZ, 4, inside_XZ);
-    dis_yz = ray_intersect_polygon<true>(p2, dir2, C.boundaryYZ, 4, inside_YZ);
-    if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
-    if (dis_xz < dis_yz) minBoundaryDist = dis_xz; else minBoundaryDist = dis_yz;
-    bool to_new_region = false;
-    if (inside_XZ && inside_YZ) {
-        p3.x = p1.x + dis_xz * dir1.x;
-        p3.y = p1.y + (dis_xz - 0.001) * dir1.y;   // in double, as geom.cu:591
-        indexLimit1 = index_of_leaf(C, p3);
-        if (indexLimit1 < 0) indexLimit1 = -indexLimit1;
-    } else {
-        inew = 0;
-        if (minBoundaryDist >= GX_INFI_DIST) return inew;
-        if (t > minBoundaryDist) { t = minBoundaryDist + GX_EPSTEP; to_new_region = true; }
-        else return inew;
-    }
-    if (!to_new_region) {
-        if (p.leafIndex > -60) index = p.leafIndex;
-        else index = index_of_leaf(C, p1);
-        // In a leaf: the ray against the leaf's XZ cross section, then against
-        // its YZ leaf-end outline. In an air gap: against the XZ cross sections
-        // of the leaves the ray walks through, from the nearest, until one is
-        // hit or the walk leaves the limits. One loop serves both, one polygon
-        // per pass, so leaf and gap lanes of a warp intersect together (each
-        // lane keeps the reference's polygons, points and order).
-        if (index > -60) {
-            const bool leaf = index >= 0;
-            const float2 *yzp = nullptr;
-            int nv = 17, sx = 1, sl = 16, i = 0, lp = 0;
+    const float2 p1 = make_float2(p.x, p.z), p2 = make_float2(p.y, p.z);
+    const float2 dir1 = make_float2(p.u, p.w), dir2 = make_float2(p.v, p.w);
+    // One polygon per turn of one loop, so that lanes with different polygons
+    // intersect together and the code is there once: the MLC's bounds in XZ and
+    // in YZ; then, inside them, in a leaf the leaf's XZ cross section and its
+    // YZ leaf-end outline; in an air gap the XZ cross sections of the leaves
+    // that the ray walks through, from the nearest, until one is hit or the
+    // walk leaves the limits (each lane keeps the reference's polygons, points
+    // and order).
+    float dis_xz = 0.0f, dis_yz = 0.0f, minBoundaryDist = 0.0f, temp1 = GX_INFI_DIST + 1;
+    float leaf_xz = 0.0f;
+    int limit1 = 0, limit2 = 60, sx = 1, i = 0, inside_xz = 0;
+    bool leaf = false, to_new_region = false;
+    const float2 *poly = C.mlc_bounds, *yzp = nullptr;
+    int n = 4, nvyz = 17;
+    bool yz = false;
+    for (int turn = 0;; turn++) {
+        int ins;
+        const float d = ray_intersect_polygon(yz ? p2 : p1, yz ? dir2 : dir1, poly, n, ins);
+        if (turn == 0) {
+            dis_xz = d;
+            inside_xz = ins;
+            poly = C.mlc_bounds + 4;
+            yz = true;
+        } else if (turn == 1) {
+            dis_yz = d;
+            if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
+            minBoundaryDist = dis_xz < dis_yz ? dis_xz : dis_yz;
+            if (!(inside_xz && ins)) {
+                if (!(t > minBoundaryDist)) return 0;
+                inew = 0;
+                t = minBoundaryDist + GX_EPSTEP;
+                to_new_region = true;
+                break;
+            }
+            if (p.leafIndex <= -60) index = index_of_leaf(C, p1);
+            if (index <= -60) break;
+            leaf = index >= 0;
+            yz = false;
+            n = 14;
             if (leaf) {
+                poly = C.crossXZ + index * 16;
                 yzp = endnode_of(C, p.field, index);
-                if (p.bank == 0) { yzp += 2; nv = 30; }
-                else if (p.bank == 2) { yzp += 17; }
+                if (p.bank == 0) { yzp += 2; nvyz = 30; }
+                else if (p.bank == 2) yzp += 17;
             } else {
-                if (dir1.x < 0) { sx = -1; sl = -16; if (indexLimit1 > 0) indexLimit1 -= 1; indexLimit2 = -index + 1; }
-                else { indexLimit2 = indexLimit1; indexLimit1 = -index - 1; }
+                // the leaf (or gap) where the ray leaves the MLC; in double, as geom.cu:591
+                const float2 p3 = make_float2(p1.x + dis_xz * dir1.x, p1.y + (dis_xz - 0.001) * dir1.y);
+                limit1 = index_of_leaf(C, p3);
+                if (limit1 < 0) limit1 = -limit1;
+                if (dir1.x < 0) { sx = -1; if (limit1 > 0) limit1 -= 1; limit2 = -index + 1; }
+                else { limit2 = limit1; limit1 = -index - 1; }
                 i = -index - sx;
-                if (indexLimit1 < 0) indexLimit1 = 0;
-                if (indexLimit2 > 59) indexLimit2 = 59;
+                if (limit1 < 0) limit1 = 0;
+                if (limit2 > 59) limit2 = 59;
                 if (i < 0) i = 0;
                 if (i > 59) i = 59;
-                lp = i * 16;
+                poly = C.crossXZ + i * 16;
             }
-            float leaf_xz = 0.0f, leaf_yz = 0.0f;
-            int ins, pass = 0;
-            bool more = true;
-            while (more) {
-                const bool yz = leaf && pass == 1;
-                const float2 *poly = leaf ? (pass == 0 ? C.crossXZ + index * 16 : yzp) : C.crossXZ + lp;
-                float d = ray_intersect_polygon<false>(yz ? p2 : p1, yz ? dir2 : dir1, poly, yz ? nv : 14, ins);
-                if (leaf) {
-                    if (pass == 0) leaf_xz = d;
-                    else { leaf_yz = d; more = false; }
-                } else {
-                    temp1 = d;
-                    i += sx;
-                    lp += sl;
-                    more = i >= indexLimit1 && i <= indexLimit2 && temp1 >= GX_INFI_DIST;
-                }
-                pass++;
-            }
+        } else if (leaf) {
+            if (turn == 3) { dis_xz = leaf_xz; dis_yz = d; break; }
+            leaf_xz = d;
+            poly = yzp;
+            n = nvyz;
+            yz = true;
+        } else {
+            temp1 = d;
+            i += sx;
+            poly += 16 * sx;
+            if (!(i >= limit1 && i <= limit2 && temp1 >= GX_INFI_DIST)) break;
+        }
+    }
+    if (!to_new_region) {
+        if (index > -60) {
             if (leaf) {
-                dis_xz = leaf_xz;
-                dis_yz = leaf_yz;
                 if (dis_yz > dis_xz) {
                     if (dir1.x < 0 && index > 0) index = -index;
                     else if (index < 59) index = -(index + 1);
@@ -369,7 +391,7 @@ __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
                 p0.module = (uint8_t)C.module_order[GEGS_M_VARMLC];
             }
         }
-        if (dis_xz < dis_yz) minDist = dis_xz; else minDist = dis_yz;
+        float minDist = dis_xz < dis_yz ? dis_xz : dis_yz;
         bool steppingOut = false;
         if ((minDist + GX_EPSTEP) >= minBoundaryDist) { minDist = minBoundaryDist; steppingOut = true; }
         if (t > minDist) {
@@ -390,105 +412,82 @@ __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
 
 __device__ __forceinline__ const float2 *fpoly(const float (*a)[2]) { return reinterpret_cast<const float2 *>(a); }
 
-__device__ uint32_t howfar_secjaws_y(const DevCtx &C, Part &p, float &t)
+// The polygons of one pair of jaws: bounding polygons, and the opening with the
+// two jaws around it (the opening is the polygon from vertex 2, the jaws those
+// from vertices 0 and 4).
+struct JawPolys { const float2 *bmax, *bmin, *geom; };
+
+__device__ __forceinline__ JawPolys jaw_polys(const DevCtx &C, int field, bool xjaw)
 {
-    const gegs_field *F = &C.fields[p.field];
-    uint32_t inew = 0;
-    float2 p0, p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
-    float2 dir1 = make_float2(p.v, p.w), dir2 = make_float2(p.u, p.w);
-    int inside_XZ, inside_YZ;
-    float dis_xz = ray_intersect_polygon<false>(p1, dir1, fpoly(F->boundMaxY), 4, inside_XZ);
-    float dis_yz = ray_intersect_polygon<false>(p2, dir2, fpoly(F->boundMaxY), 4, inside_YZ);
-    float minBoundaryDist;
-    if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return inew;
-    if (dis_xz < dis_yz) minBoundaryDist = dis_xz; else minBoundaryDist = dis_yz;
-    if (inside_XZ && inside_YZ) {
-        if (point_in_polygon(p2, fpoly(F->jawsGeomY) + 2, 4)) {
-            inew = 1;
-            dis_xz = ray_intersect_polygon<false>(p2, dir2, fpoly(F->jawsGeomY), 4, inside_YZ);
-            dis_yz = ray_intersect_polygon<false>(p2, dir2, fpoly(F->jawsGeomY) + 4, 4, inside_YZ);
-            if (dis_xz < GX_INFI_DIST) {
-                if (t > dis_xz) { inew = 2; t = dis_xz + GX_EPSTEP; }
-            } else if (dis_yz < GX_INFI_DIST) {
-                if (t > dis_yz) { inew = 2; t = dis_yz + GX_EPSTEP; }
-            } else {
-                if (t > minBoundaryDist) { t = minBoundaryDist + GX_EPSTEP; p.module = (uint8_t)C.module_order[GEGS_M_SECJAWY]; }
-            }
-        } else {
-            inew = 2;
-            dis_yz = ray_intersect_polygon<false>(p2, dir2, fpoly(F->jawsGeomY) + 2, 4, inside_YZ);
-            if (dis_yz < GX_INFI_DIST) {
-                if (t > dis_yz) { inew = 1; t = dis_yz + GX_EPSTEP; }
-            } else {
-                if (t > minBoundaryDist) { inew = 0; t = minBoundaryDist + GX_EPSTEP; }
-            }
-        }
-    } else {
-        inew = 1;
-        if (t > minBoundaryDist) {
-            t = minBoundaryDist + GX_EPSTEP;
-            p0.x = p.y + t * p.v;
-            p0.y = p.x + t * p.u;
-            if (!point_in_polygon(p0, fpoly(F->boundMinY), 4)) inew = 0;
-            else {
-                p0.x = p0.y;
-                p0.y = p.z + t * p.w;
-                if (point_in_polygon(p0, fpoly(F->jawsGeomY) + 2, 4)) inew = 1;
-                else inew = 2;
-            }
-        }
-    }
-    return inew;
+    const gegs_field *F = &C.fields[field];
+    JawPolys j;
+    j.bmax = fpoly(xjaw ? F->boundMaxX : F->boundMaxY);
+    j.bmin = fpoly(xjaw ? F->boundMinX : F->boundMinY);
+    j.geom = fpoly(xjaw ? F->jawsGeomX : F->jawsGeomY);
+    return j;
 }
 
-__device__ uint32_t howfar_secjaws_x(const DevCtx &C, Part &p, float &t)
+// howfar_SecJawsY and howfar_SecJawsX (geom.cu:793-1035) in one: the Y jaws
+// open in x, the X jaws in y. The reference's X routine steps to the opening
+// from the tungsten by the distance to the bounds in YZ; kept.
+static __device__ uint32_t howfar_secjaws(const DevCtx &C, Part &p, float &t)
 {
-    const gegs_field *F = &C.fields[p.field];
-    uint32_t inew = 0;
-    float2 p0, p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
-    float2 dir1 = make_float2(p.v, p.w), dir2 = make_float2(p.u, p.w);
-    int inside_XZ, inside_YZ;
-    float dis_xz = ray_intersect_polygon<false>(p1, dir1, fpoly(F->boundMaxX), 4, inside_XZ);
-    float dis_yz = ray_intersect_polygon<false>(p2, dir2, fpoly(F->boundMaxX), 4, inside_YZ);
-    float minBoundaryDist;
-    if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return inew;
-    if (dis_xz < dis_yz) minBoundaryDist = dis_xz; else minBoundaryDist = dis_yz;
-    if (inside_XZ && inside_YZ) {
-        if (point_in_polygon(p1, fpoly(F->jawsGeomX) + 2, 4)) {
-            inew = 1;
-            dis_xz = ray_intersect_polygon<false>(p1, dir1, fpoly(F->jawsGeomX), 4, inside_XZ);
-            dis_yz = ray_intersect_polygon<false>(p1, dir1, fpoly(F->jawsGeomX) + 4, 4, inside_XZ);
-            if (dis_xz < GX_INFI_DIST) {
-                if (t > dis_xz) { inew = 2; t = dis_xz + GX_EPSTEP; }
-            } else if (dis_yz < GX_INFI_DIST) {
-                if (t > dis_yz) { inew = 2; t = dis_yz + GX_EPSTEP; }
-            } else {
-                if (t > minBoundaryDist) { t = minBoundaryDist + GX_EPSTEP; p.module = (uint8_t)C.module_order[GEGS_M_SECJAWX]; }
+    const bool xjaw = p.module == GEGS_M_SECJAWX;
+    const JawPolys J = jaw_polys(C, p.field, xjaw);
+    const float2 p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
+    const float2 dir1 = make_float2(p.v, p.w), dir2 = make_float2(p.u, p.w);
+    const float2 q = xjaw ? p1 : p2, dq = xjaw ? dir1 : dir2;
+    // one polygon per turn: the bounds seen from (y, z) and from (x, z); then
+    // from the opening the two jaws around it, from a jaw the opening
+    float dis_xz = 0.0f, dis_yz = 0.0f, minBoundaryDist = 0.0f, jaw0 = 0.0f, d;
+    int inside_xz = 0, ins;
+    bool open = false;
+    float2 o = p1, v = dir1;
+    const float2 *poly = J.bmax;
+    for (int turn = 0;; turn++) {
+        d = ray_intersect_polygon(o, v, poly, 4, ins);
+        if (turn == 0) {
+            dis_xz = d;
+            inside_xz = ins;
+            o = p2;
+            v = dir2;
+        } else if (turn == 1) {
+            dis_yz = d;
+            if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
+            minBoundaryDist = dis_xz < dis_yz ? dis_xz : dis_yz;
+            if (!(inside_xz && ins)) {
+                if (!(t > minBoundaryDist)) return 1;
+                t = minBoundaryDist + GX_EPSTEP;
+                const float y = p.y + t * p.v, x = p.x + t * p.u;
+                if (!point_in_polygon(y, x, J.bmin, 4)) return 0;
+                return point_in_polygon(xjaw ? y : x, p.z + t * p.w, J.geom + 2, 4) ? 1 : 2;
             }
-        } else {
-            inew = 2;
-            dis_xz = ray_intersect_polygon<false>(p1, dir1, fpoly(F->jawsGeomX) + 2, 4, inside_XZ);
-            if (dis_xz < GX_INFI_DIST) {
-                if (t > dis_xz) { inew = 1; t = dis_yz + GX_EPSTEP; }
-            } else {
-                if (t > minBoundaryDist) { inew = 0; t = minBoundaryDist + GX_EPSTEP; }
-            }
-        }
-    } else {
-        inew = 1;
-        if (t > minBoundaryDist) {
-            t = minBoundaryDist + GX_EPSTEP;
-            p0.x = p.y + t * p.v;
-            p0.y = p.x + t * p.u;
-            if (!point_in_polygon(p0, fpoly(F->boundMinX), 4)) inew = 0;
-            else {
-                p0.y = p.z + t * p.w;
-                if (point_in_polygon(p0, fpoly(F->jawsGeomX) + 2, 4)) inew = 1;
-                else inew = 2;
-            }
-        }
+            open = point_in_polygon(q.x, q.y, J.geom + 2, 4);
+            o = q;
+            v = dq;
+            poly = open ? J.geom : J.geom + 2;
+        } else if (turn == 2 && open) {
+            jaw0 = d;
+            poly = J.geom + 4;
+        } else break;
     }
-    return inew;
+    if (open) {
+        const float jaw = jaw0 < GX_INFI_DIST ? jaw0 : d;
+        if (jaw < GX_INFI_DIST) {
+            if (t > jaw) { t = jaw + GX_EPSTEP; return 2; }
+        } else if (t > minBoundaryDist) {
+            t = minBoundaryDist + GX_EPSTEP;
+            p.module = (uint8_t)C.module_order[xjaw ? GEGS_M_SECJAWX : GEGS_M_SECJAWY];
+        }
+        return 1;
+    }
+    if (d < GX_INFI_DIST) {
+        if (t > d) { t = (xjaw ? dis_yz : d) + GX_EPSTEP; return 1; }
+    } else if (t > minBoundaryDist) {
+        t = minBoundaryDist + GX_EPSTEP;
+        return 0;
+    }
+    return 2;
 }
 
 // ---- hownear -----------------------------------------------------------------
@@ -513,117 +512,154 @@ __device__ __forceinline__ float point_dist2_to_segment(float2 p, float2 v, floa
     return dist2p(p, a);
 }
 
-// Minimum edge distance of the polygon, capped at 1e9 (pointMinDistToPolygon,
-// geom.cu:1175-1191). sqrtf is correctly rounded and monotonic, so the
-// minimum of the edges' sqrtf equals sqrtf of the minimum squared distance:
-// one square root per polygon instead of one per edge, same result.
-template <bool LOCAL>
-__device__ float point_min_dist_to_polygon(float2 p0, const float2 *poly, int n)
+// What an electron step does with hownear: compares it with the range (where
+// range rejection is on) and with the step tustep, which it limits when it is
+// smaller. A value known to within a slack often decides that, and then stands
+// in for the exact one.
+struct NearUse { bool rr; float range, tustep; };
+
+__device__ __forceinline__ NearUse near_exactly()
+{
+    NearUse u;
+    u.rr = false; u.range = 0.0f; u.tustep = __int_as_float(0x7f800000);
+    return u;
+}
+
+// lo <= hownear <= hi: is the step's outcome (beyond the range; or within it
+// and beyond tustep) certain?
+__device__ __forceinline__ bool near_decided(const NearUse &u, float lo, float hi)
+{
+    return u.rr ? lo > u.range || (lo > u.tustep && hi < u.range) : lo > u.tustep;
+}
+
+// Squared distances to the polygon's edges, without their roundings: lowers
+// `best` to the smallest and marks the edges that come within `slack` (cm) of
+// the smallest found so far, which include every edge whose exact distance can
+// be the smallest. (sqrt(m) + s)^2 <= m (1 + s) + s + s^2.
+__device__ __forceinline__ void near_edges(float2 p0, const float2 *poly, int n, float slack, float &best, uint32_t &cand)
+{
+    cand = 0;
+    const float grow = 1.0f + slack, add = slack + slack * slack;
+    const float2 first = ld2(poly);
+    float2 a = first;
+#pragma unroll 2
+    for (int i = 0; i < n; i++) {
+        const float2 b = i + 1 < n ? ld2(&poly[i + 1]) : first;
+        const float ex = b.x - a.x, ey = b.y - a.y, dx = p0.x - a.x, dy = p0.y - a.y;
+        const float t = __saturatef(__fdividef(__fmaf_rn(dx, ex, dy * ey), __fmaf_rn(ex, ex, ey * ey)));
+        const float rx = __fmaf_rn(-t, ex, dx), ry = __fmaf_rn(-t, ey, dy);
+        const float d2 = __fmaf_rn(rx, rx, ry * ry);
+        if (d2 <= __fmaf_rn(best, grow, add)) cand |= 1u << i;
+        best = fminf(best, d2);
+        a = b;
+    }
+}
+
+// Exact distance to the polygon (pointMinDistToPolygon, geom.cu:1175-1191,
+// capped at 1e9) from its marked edges; infinite without any. sqrtf is
+// correctly rounded and monotonic, so the root of the smallest square is the
+// smallest root.
+__device__ __forceinline__ float near_exact(float2 p0, const float2 *poly, int n, uint32_t cand)
 {
     float min2 = __int_as_float(0x7f800000);
-    for (int i = 0; i < n; i++) {
-        int j = i + 1;
-        if (j >= n) j = 0;
-        float2 a = LOCAL ? poly[i] : ld2(&poly[i]);
-        float2 b = LOCAL ? poly[j] : ld2(&poly[j]);
-        float d2 = point_dist2_to_segment(p0, a, b);
+    while (cand) {
+        const int i = __ffs(cand) - 1;
+        cand &= cand - 1u;
+        const float d2 = point_dist2_to_segment(p0, ld2(&poly[i]), ld2(&poly[i + 1 < n ? i + 1 : 0]));
         if (d2 < min2) min2 = d2;
     }
-    float d = sqrtf(min2);
+    const float d = sqrtf(min2);
     return d < 1e9f ? d : 1e9f;
 }
 
-__device__ void hownear_mlc(const DevCtx &C, Part &p, float &tperp)
+// How far near_edges can be from the exact distance, as computed in float: some
+// 1e-6 of the coordinates and of the polygons' extent (C.near_slack holds 10 um
+// and 1e-5 of the latter).
+__device__ __forceinline__ float near_error(const DevCtx &C, const Part &p)
 {
-    float2 p1 = make_float2(p.x, p.z), p2 = make_float2(p.y, p.z);
-    int index;
-    float tperp_xz = GX_INFI_DIST + 1, tperp_yz = GX_INFI_DIST + 1, bound;
-    int inside_XZ, inside_YZ;
-    if (p.leafIndex < -60) {
-        inside_XZ = point_in_polygon_local(p1, C.boundaryXZ, 4);
-        inside_YZ = point_in_polygon_local(p2, C.boundaryYZ, 4);
-    } else { inside_XZ = 1; inside_YZ = 1; }
-    // the distance to the MLC boundary is needed only outside the MLC (the
-    // reference computes it first in every case; the result is the same)
-    if (inside_XZ && inside_YZ) {
+    return C.near_slack + 1e-5f * (fabsf(p.x) + fabsf(p.y) + fabsf(p.z));
+}
+
+static __device__ void hownear_mlc(const DevCtx &C, Part &p, float &tperp, const NearUse &use)
+{
+    const float2 p1 = make_float2(p.x, p.z), p2 = make_float2(p.y, p.z);
+    const float err = near_error(C, p);
+    // Two polygons in every case, one per turn, so that the lanes of all cases
+    // share the loops: outside the MLC its bounds in XZ and in YZ; in a leaf
+    // column the leaf's XZ cross section and its YZ leaf-end outline; in an air
+    // gap the XZ cross sections of the leaves on either side.
+    const float2 *poly0 = C.mlc_bounds, *poly1 = C.mlc_bounds + 4;
+    int n0 = 4, n1 = 4;
+    bool second_yz = true, gap = false;
+    bool inside = true;
+    if (p.leafIndex < -60)
+        inside = point_in_polygon(p1.x, p1.y, C.mlc_bounds, 4) && point_in_polygon(p2.x, p2.y, C.mlc_bounds + 4, 4);
+    if (inside) {
+        int index;
         if (p.leafIndex > GX_PASSMLC) index = p.leafIndex;
         else { index = index_of_leaf(C, p1); p.leafIndex = (int8_t)index; }
-        // In a leaf column: the leaf's XZ cross section, then its YZ leaf-end
-        // outline; in an air gap: the XZ cross sections of the two leaves on
-        // either side. Two polygon distances either way, taken in one loop so
-        // that lanes of both cases share it (each lane keeps the reference's
-        // polygons and order).
-        if (index >= 0 && p.bank < 0) p.bank = (int8_t)point_in_leaf(p2, endnode_of(C, p.field, index));
-        if (index > -60) {
-            const bool leaf = index >= 0;
-            const float2 *yzp = nullptr;
-            int nvyz = 17;
-            if (leaf) {
-                yzp = endnode_of(C, p.field, index);
-                if (p.bank == 0) { yzp += 2; nvyz = 30; }
-                else if (p.bank == 2) { yzp += 17; }
-            }
-            float dd[2];
-            for (int k = 0; k < 2; k++) {
-                const bool yz = leaf && k == 1;
-                const float2 *poly = leaf ? (k == 0 ? C.crossXZ + index * 16 : yzp) : C.crossXZ + (-index - k) * 16;
-                dd[k] = point_min_dist_to_polygon<false>(yz ? p2 : p1, poly, yz ? nvyz : 14);
-            }
-            if (leaf) { tperp_xz = dd[0]; tperp_yz = dd[1]; }
-            else tperp_xz = dd[0] < dd[1] ? dd[0] : dd[1];
-        }
-        if (tperp_xz < tperp_yz) tperp = tperp_xz; else tperp = tperp_yz;
-    } else {
-        float bxz = point_min_dist_to_polygon<true>(p1, C.boundaryXZ, 4);
-        float byz = point_min_dist_to_polygon<true>(p2, C.boundaryYZ, 4);
-        if (bxz < byz) bound = bxz; else bound = byz;
-        tperp = bound;
-    }
-}
-
-__device__ void hownear_secjaws_y(const DevCtx &C, const Part &p, float &tperp)
-{
-    const gegs_field *F = &C.fields[p.field];
-    float2 p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
-    int inside_XZ = point_in_polygon(p1, fpoly(F->boundMaxY), 4);
-    int inside_YZ = point_in_polygon(p2, fpoly(F->boundMaxY), 4);
-    float bound_xz = point_min_dist_to_polygon<false>(p1, fpoly(F->boundMaxY), 4);
-    float bound_yz = point_min_dist_to_polygon<false>(p2, fpoly(F->boundMaxY), 4);
-    if (inside_XZ && inside_YZ) {
-        float dist_yz = point_min_dist_to_polygon<false>(p2, fpoly(F->jawsGeomY) + 2, 4);
-        if (point_in_polygon(p2, fpoly(F->jawsGeomY) + 2, 4)) {
-            if (dist_yz < bound_xz) tperp = dist_yz; else tperp = bound_xz;
+        if (index <= -60) { tperp = GX_INFI_DIST + 1; return; }
+        if (index >= 0) {
+            const float2 *yzp = endnode_of(C, p.field, index);
+            if (p.bank < 0) p.bank = (int8_t)point_in_leaf(p2, yzp);
+            poly0 = C.crossXZ + index * 16;
+            poly1 = yzp + (p.bank == 0 ? 2 : p.bank == 2 ? 17 : 0);
+            n1 = p.bank == 0 ? 30 : 17;
         } else {
-            if (dist_yz > bound_yz) dist_yz = bound_yz;
-            if (dist_yz < bound_xz) tperp = dist_yz; else tperp = bound_xz;
+            gap = true;
+            second_yz = false;
+            poly0 = C.crossXZ + -index * 16;
+            poly1 = C.crossXZ + (-index - 1) * 16;
+            n1 = 14;
         }
-    } else {
-        if (bound_xz < bound_yz) tperp = bound_xz; else tperp = bound_yz;
+        n0 = 14;
+    }
+    float best = 1e30f;
+    uint32_t cand0 = 0, cand1 = 0;
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        cand0 = cand1;
+        near_edges(k && second_yz ? p2 : p1, k ? poly1 : poly0, k ? n1 : n0, 2.0f * err, best, cand1);
+    }
+    const float d = sqrtf(best);
+    if (near_decided(use, d - err, d + err)) { tperp = d - err; return; }
+    tperp = gap ? GX_INFI_DIST + 1 : __int_as_float(0x7f800000);
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const float e = near_exact(k && second_yz ? p2 : p1, k ? poly1 : poly0, k ? n1 : n0, k ? cand1 : cand0);
+        if (e < tperp) tperp = e;
     }
 }
 
-__device__ void hownear_secjaws_x(const DevCtx &C, const Part &p, float &tperp)
+// hownear_SecJawsY and hownear_SecJawsX (geom.cu:1288-1374) in one: distances to
+// the bounding polygon seen from (y, z) and from (x, z), and to the opening.
+static __device__ void hownear_secjaws(const DevCtx &C, const Part &p, float &tperp)
 {
-    const gegs_field *F = &C.fields[p.field];
-    float2 p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
-    int inside_XZ = point_in_polygon(p1, fpoly(F->boundMaxX), 4);
-    int inside_YZ = point_in_polygon(p2, fpoly(F->boundMaxX), 4);
-    float bound_xz = point_min_dist_to_polygon<false>(p1, fpoly(F->boundMaxX), 4);
-    float bound_yz = point_min_dist_to_polygon<false>(p2, fpoly(F->boundMaxX), 4);
-    if (inside_XZ && inside_YZ) {
-        float dist_xz = point_min_dist_to_polygon<false>(p1, fpoly(F->jawsGeomX) + 2, 4);
-        if (point_in_polygon(p1, fpoly(F->jawsGeomX) + 2, 4)) {
-            if (dist_xz < bound_yz) tperp = dist_xz; else tperp = bound_yz;
-        } else {
-            if (dist_xz > bound_xz) dist_xz = bound_xz;
-            if (dist_xz < bound_yz) tperp = dist_xz; else tperp = bound_yz;
-        }
-    } else {
-        if (bound_xz < bound_yz) tperp = bound_xz; else tperp = bound_yz;
+    const bool xjaw = p.module == GEGS_M_SECJAWX;
+    const JawPolys J = jaw_polys(C, p.field, xjaw);
+    const float err = near_error(C, p);
+    const float2 p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
+    float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f;
+    int in0 = 0, in1 = 0, in2 = 0;
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+        const float2 o = k == 0 || (k == 2 && xjaw) ? p1 : p2;
+        const float2 *poly = k < 2 ? J.bmax : J.geom + 2;
+        float best = 1e30f;
+        uint32_t cand;
+        near_edges(o, poly, 4, 2.0f * err, best, cand);
+        d0 = d1; d1 = d2; d2 = near_exact(o, poly, 4, cand);
+        in0 = in1; in1 = in2; in2 = point_in_polygon(o.x, o.y, poly, 4);
     }
+    const float along = xjaw ? d1 : d0, across = xjaw ? d0 : d1;
+    if (in0 && in1) {
+        float d = d2;
+        if (!in2 && d > across) d = across;
+        tperp = d < along ? d : along;
+    } else tperp = d0 < d1 ? d0 : d1;
 }
 
-// Lower bound on hownear_secjaws_y / _x: their result is a minimum over
+// Lower bound on hownear_secjaws: its result is a minimum over
 // distances to some of three (point, polygon) pairs -- the bounding polygon
 // seen from (y, z) and from (x, z), and the jaw opening seen from (x, z) for
 // the Y jaws or from (y, z) for the X jaws -- and a distance to a polygon is
@@ -658,8 +694,8 @@ __device__ __forceinline__ uint32_t howfar(const DevCtx &C, Part &p, float &t, b
     switch (p.module) {
     case GEGS_M_PHANTOM: return howfar_phantom(C, p, t);
     case GEGS_M_VARMLC: return howfar_mlc(C, p, t);
-    case GEGS_M_SECJAWY: return howfar_secjaws_y(C, p, t);
-    case GEGS_M_SECJAWX: return howfar_secjaws_x(C, p, t);
+    case GEGS_M_SECJAWY:
+    case GEGS_M_SECJAWX: return howfar_secjaws(C, p, t);
     default: ok = false; return 0;
     }
 }
@@ -669,9 +705,9 @@ __device__ __forceinline__ void hownear(const DevCtx &C, Part &p, float &tperp, 
     ok = true;
     switch (p.module) {
     case GEGS_M_PHANTOM: hownear_phantom(C, p, tperp); return;
-    case GEGS_M_VARMLC: hownear_mlc(C, p, tperp); return;
-    case GEGS_M_SECJAWY: hownear_secjaws_y(C, p, tperp); return;
-    case GEGS_M_SECJAWX: hownear_secjaws_x(C, p, tperp); return;
+    case GEGS_M_VARMLC: hownear_mlc(C, p, tperp, near_exactly()); return;
+    case GEGS_M_SECJAWY:
+    case GEGS_M_SECJAWX: hownear_secjaws(C, p, tperp); return;
     default: ok = false; tperp = 0; return;
     }
 }
@@ -711,25 +747,29 @@ __device__ __forceinline__ uint32_t howfar_g(const DevCtx &C, Part &p, float &t,
     } else if (G == GX_GEOM_MLC) {
         if (p.module == GEGS_M_VARMLC) return howfar_mlc(C, p, t);
     } else {
-        if (p.module == GEGS_M_SECJAWY) return howfar_secjaws_y(C, p, t);
-        if (p.module == GEGS_M_SECJAWX) return howfar_secjaws_x(C, p, t);
+        if (p.module == GEGS_M_SECJAWY || p.module == GEGS_M_SECJAWX) return howfar_secjaws(C, p, t);
     }
     ok = false;
     return 0;
 }
 
+// Distance to the nearest boundary, as far as `use` needs it.
 template <int G>
-__device__ __forceinline__ void hownear_g(const DevCtx &C, Part &p, float &tperp, bool &ok)
+__device__ __forceinline__ void hownear_g(const DevCtx &C, Part &p, float &tperp, bool &ok, const NearUse &use)
 {
     if (G == GX_GEOM_ALL) { hownear(C, p, tperp, ok); return; }
     ok = true;
     if (G == GX_GEOM_PHANTOM) {
         if (p.module == GEGS_M_PHANTOM) { hownear_phantom(C, p, tperp); return; }
     } else if (G == GX_GEOM_MLC) {
-        if (p.module == GEGS_M_VARMLC) { hownear_mlc(C, p, tperp); return; }
+        if (p.module == GEGS_M_VARMLC) { hownear_mlc(C, p, tperp, use); return; }
     } else {
-        if (p.module == GEGS_M_SECJAWY) { hownear_secjaws_y(C, p, tperp); return; }
-        if (p.module == GEGS_M_SECJAWX) { hownear_secjaws_x(C, p, tperp); return; }
+        if (p.module == GEGS_M_SECJAWY || p.module == GEGS_M_SECJAWX) {
+            tperp = jaws_near_lower_bound(C, p);
+            if (near_decided(use, tperp, __int_as_float(0x7f800000))) return;
+            hownear_secjaws(C, p, tperp);
+            return;
+        }
     }
     ok = false;
     tperp = 0;

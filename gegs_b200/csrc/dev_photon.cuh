@@ -90,13 +90,13 @@ __device__ __forceinline__ void relax_direction(const DevCtx &C, Rng &r, Part &p
     }
 }
 
-__constant__ short c_first_transition[5] = {1, 20, 27, 33, 38};
-__constant__ short c_last_transition[5] = {19, 26, 32, 37, 39};
-__constant__ short c_final_state[39] = {4, 3, 5, 6, 202, 302, 402, 404, 403, 303, 502, 503, 504, 602, 603, 604, 505, 605, 606,
+static __constant__ short c_first_transition[5] = {1, 20, 27, 33, 38};
+static __constant__ short c_last_transition[5] = {19, 26, 32, 37, 39};
+static __constant__ short c_final_state[39] = {4, 3, 5, 6, 202, 302, 402, 404, 403, 303, 502, 503, 504, 602, 603, 604, 505, 605, 606,
                                         13, 14, 5, 6, 505, 605, 606, 14, 5, 6, 505, 605, 606, 5, 6, 505, 605, 606, 6, 606};
 
 // Fluorescence / Auger / Coster-Kronig cascade for a vacancy in shell n of element iz.
-__device__ void relax(const DevCtx &C, float energy, int n, int iz, float &edep, Part p, const RegInfo &rd, Rng &r)
+static __device__ void relax(const DevCtx &C, float energy, int n, int iz, float &edep, Part p, const RegInfo &rd, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -194,76 +194,78 @@ __device__ __forceinline__ void stage_photon_tables(const DevCtx &C)
     __syncthreads();
 }
 
-// One iteration of the PHOTON loop.  Returns true when the photon has left
-// the photon stage (absorbed, escaped or queued for an interaction).
+// What became of a particle in a transport step.
+enum : int {
+    STEP_ON = 0,      // it goes on in this stage
+    STEP_DONE = 1,    // it is gone
+    STEP_QUEUE = 2,   // it goes to the stage that the step names
+    STEP_NEAR = 3,    // (electron first passes) the step needs howfar: not taken
+    STEP_FAR = 4      // (near-boundary passes) it does not: not taken
+};
+
+// One iteration of the PHOTON loop. `vx` is the record of the photon's region,
+// kept from one step to the next. Every way out that scores or queues shares
+// one place, and the queueing itself is the caller's, so that the code is small.
 // SH: the {gmfp, cohe} table is staged in shared memory (stage_photon_tables).
 template <int G = GX_GEOM_ALL, bool SH = false>
-__device__ bool photon_step(const DevCtx &C, Part &p, Rng &r)
+static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, int &out)
 {
     const gegs_physics *P = C.P;
-    RegInfo rd = region_info(C, p.region);
-    if (p.e <= rd.pcut) { escore(C, p, p.region, p.e * p.wt); return true; }
-    if (p.wt <= 0.0f) return true;
-    float r1 = U(C, r);
-    float dpmfp = -gx_log(r1);
-    float gle = gx_log(p.e);
-    int lgle = 0;
-    float tstep, gmfp_val = 0.0f, cohfac = 0.0f;
-    unsigned med = rd.med;
-    if (med == GX_VACUUM) tstep = GX_VACUUM_STEP;
-    else {
-        float2 ge = __ldg(reinterpret_cast<const float2 *>(P->ge[med]));
-        lgle = (int)(ge.x + ge.y * gle);
-        float4 t;
-        if (SH && C.stage_tables) t = g_smem_ptab[med * GX_MXGE + lgle];
-        else {
-            const float2 g = __ldg(reinterpret_cast<const float2 *>(P->gmfp[med * GX_MXGE + lgle]));
-            t.x = g.x; t.y = g.y;
-        }
-        float gmfpr0 = t.x + t.y * gle;
-        gmfp_val = gmfpr0 / rd.rhof;
-        if (rd.flags & GEGS_F_RAYLEIGH) {
-            if (!(SH && C.stage_tables)) {
-                const float2 c = __ldg(reinterpret_cast<const float2 *>(P->cohe[med * GX_MXGE + lgle]));
-                t.z = c.x; t.w = c.y;
-            }
-            cohfac = t.z + t.w * gle;
-            gmfp_val = gmfp_val * cohfac;
-        }
-        tstep = gmfp_val * dpmfp;
-    }
-    bool ok;
-    uint32_t new_region = howfar_g<G>(C, p, tstep, ok);
-    if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return true; }
+    const unsigned med = vx.med;
     int idisc = 0;
-    if (new_region == 0) {
-        if (med == GX_VACUUM || p.leafIndex == GX_PASSMLC) idisc = 1; else idisc = -1;
+    bool absorbed = p.e <= pcut_of(C, vx);
+    float dpmfp = 0.0f, cohfac = 0.0f, gle = 0.0f;
+    int lgle = 0;
+    if (!absorbed) {
+        if (p.wt <= 0.0f) return STEP_DONE;
+        float r1 = U(C, r);
+        dpmfp = -gx_log(r1);
+        gle = gx_log(p.e);
+        float tstep, gmfp_val = 0.0f;
+        if (med == GX_VACUUM) tstep = GX_VACUUM_STEP;
+        else {
+            float2 ge = __ldg(reinterpret_cast<const float2 *>(P->ge[med]));
+            lgle = (int)(ge.x + ge.y * gle);
+            const float4 t = SH && C.stage_tables ? g_smem_ptab[med * GX_MXGE + lgle] : __ldg(&C.ptab[med * GX_MXGE + lgle]);
+            float gmfpr0 = t.x + t.y * gle;
+            gmfp_val = gmfpr0 / vx.rhof;
+            if (vx.flags & GEGS_F_RAYLEIGH) {
+                cohfac = t.z + t.w * gle;
+                gmfp_val = gmfp_val * cohfac;
+            }
+            tstep = gmfp_val * dpmfp;
+        }
+        bool ok;
+        const uint32_t new_region = howfar_g<G>(C, p, tstep, ok);
+        if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return STEP_DONE; }
+        if (new_region != p.region) vx = C.reg[new_region];
+        if (new_region == 0) {
+            if (med == GX_VACUUM || p.leafIndex == GX_PASSMLC) { p.region = 0; return STEP_DONE; }   // left the geometry
+            idisc = -1;
+        }
+        p.x = p.x + p.u * tstep;
+        p.y = p.y + p.v * tstep;
+        p.z = p.z + p.w * tstep;
+        if (med != GX_VACUUM) dpmfp = fmaxf_(0.0f, dpmfp - tstep / gmfp_val);
+        p.region = new_region;
+        absorbed = p.e <= pcut_of(C, vx) || idisc < 0;
     }
-    if (idisc > 0) { p.region = 0; escore(C, p, 0, p.e * p.wt); return true; }
-    p.x = p.x + p.u * tstep;
-    p.y = p.y + p.v * tstep;
-    p.z = p.z + p.w * tstep;
-    if (med != GX_VACUUM) dpmfp = fmaxf_(0.0f, dpmfp - tstep / gmfp_val);
-    unsigned old_medium = med;
-    if (new_region != p.region) { p.region = new_region; rd = region_info(C, new_region); }
-    if (p.e <= rd.pcut || idisc < 0) { escore(C, p, p.region, p.e * p.wt); return true; }
-    if ((rd.med != old_medium) || (rd.med == GX_VACUUM) || gx_ge(dpmfp, GX_EPSGMFP)) return false;
-    if (rd.flags & GEGS_F_RAYLEIGH) {
-        r1 = U(C, r);
-        if (r1 < 1.0f - cohfac) { push_move(C, ST_RAYLEIGH, p, r); return true; }
+    if (absorbed) { escore(C, p, p.region, p.e * p.wt); return STEP_DONE; }
+    if ((vx.med != med) || (vx.med == GX_VACUUM) || gx_ge(dpmfp, GX_EPSGMFP)) return STEP_ON;
+    if (vx.flags & GEGS_F_RAYLEIGH) {
+        const float r1 = U(C, r);
+        if (r1 < 1.0f - cohfac) { out = ST_RAYLEIGH; return STEP_QUEUE; }
     }
-    float2 b1 = __ldg(reinterpret_cast<const float2 *>(P->gbr1[rd.med * GX_MXGE + lgle]));
-    float2 b2 = __ldg(reinterpret_cast<const float2 *>(P->gbr2[rd.med * GX_MXGE + lgle]));
+    float2 b1 = __ldg(reinterpret_cast<const float2 *>(P->gbr1[vx.med * GX_MXGE + lgle]));
+    float2 b2 = __ldg(reinterpret_cast<const float2 *>(P->gbr2[vx.med * GX_MXGE + lgle]));
     float gbr1_val = b1.x + b1.y * gle;
     float gbr2_val = b2.x + b2.y * gle;
-    r1 = U(C, r);
-    if ((r1 <= gbr1_val) && (p.e > 2.0f * P->rm)) push_move(C, ST_PAIR, p, r);
-    else if (r1 < gbr2_val) push_move(C, ST_COMPTON, p, r);
-    else push_move(C, ST_PHOTO, p, r);
-    return true;
+    const float r1 = U(C, r);
+    out = (r1 <= gbr1_val) && (p.e > 2.0f * P->rm) ? ST_PAIR : r1 < gbr2_val ? ST_COMPTON : ST_PHOTO;
+    return STEP_QUEUE;
 }
 
-__device__ void compton(const DevCtx &C, Part p, Rng &r)
+static __device__ void compton(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -445,7 +447,7 @@ __device__ void compton(const DevCtx &C, Part p, Rng &r)
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void photo(const DevCtx &C, Part p, Rng &r)
+static __device__ void photo(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm;
@@ -569,7 +571,7 @@ __device__ void photo(const DevCtx &C, Part p, Rng &r)
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void rayleigh(const DevCtx &C, Part p, Rng &r)
+static __device__ void rayleigh(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     RegInfo rd = region_info(C, p.region);
@@ -618,7 +620,7 @@ __device__ void rayleigh(const DevCtx &C, Part p, Rng &r)
     else push_spawn(C, ST_PHOTON, p, r);
 }
 
-__device__ void annih_at_rest(const DevCtx &C, Part &p, const RegInfo &rd, Rng &r)
+static __device__ void annih_at_rest(const DevCtx &C, Part &p, const RegInfo &rd, Rng &r)
 {
     const gegs_physics *P = C.P;
     float edep = 0.0f;
@@ -644,7 +646,7 @@ __device__ void annih_at_rest(const DevCtx &C, Part &p, const RegInfo &rd, Rng &
     escore(C, p, p.region, edep * p.wt);
 }
 
-__device__ void pair_angle(const DevCtx &C, Rng &r, int use, float ese, float eig, unsigned medium, float &costhe, float &sinthe)
+static __device__ void pair_angle(const DevCtx &C, Rng &r, int use, float ese, float eig, unsigned medium, float &costhe, float &sinthe)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm;
@@ -701,7 +703,7 @@ __device__ void pair_angle(const DevCtx &C, Rng &r, int use, float ese, float ei
     }
 }
 
-__device__ void pair(const DevCtx &C, Part p, Rng &r)
+static __device__ void pair(const DevCtx &C, Part p, Rng &r)
 {
     const gegs_physics *P = C.P;
     const float rm = P->rm, prm = P->prm, rmt2 = P->rmt2;

@@ -43,6 +43,10 @@ static_assert(GX_NQ == GEGS_NQUEUES, "gegs_run_stats reports every queue");
 // eight interaction kernels: the engine's stream and seven more)
 static constexpr int kAux = 7;
 
+// Spare entries around the re-laid tables: the reference's tables end where
+// another begins, so a bin past an end reads something; here it reads these.
+static constexpr size_t kTablePad = 4096;
+
 struct gegs_engine {
     int device = 0;
     int nsm = 0;
@@ -56,7 +60,8 @@ struct gegs_engine {
     std::string err;
 
     gegs_physics *d_P = nullptr;
-    float4 *d_ptab = nullptr;          // {gmfp, cohe} per (medium, energy bin) (DevCtx::ptab)
+    float4 *d_ptab = nullptr;          // {gmfp, cohe} per (medium, energy bin) (DevCtx::ptab, kTablePad entries in)
+    float4 *d_etab = nullptr;          // electron tables per bin (DevCtx::etab, kTablePad entries in)
     Vox *d_reg = nullptr;
     float *d_xb = nullptr, *d_yb = nullptr, *d_zb = nullptr;
     gegs_field *d_fields = nullptr;
@@ -168,6 +173,25 @@ static std::vector<float4> jaw_edge_lines(const gegs_field *F, int nfields)
     return out;
 }
 
+// The slack of hownear's estimates over the polygons so far: 10 um, and 1e-5 of
+// the largest coordinate (near_error). True if these polygons widened it.
+static bool widen_near_slack(gegs_engine *e, const float *xy, size_t n)
+{
+    float most = 0.0f;
+    for (size_t i = 0; i < n; i++)
+        if (fabsf(xy[i]) > most) most = fabsf(xy[i]);
+    const float slack = 1e-3f + 1e-5f * most;
+    if (!(slack > e->ctx.near_slack)) return false;
+    e->ctx.near_slack = slack;
+    return true;
+}
+
+static bool widen_near_slack(gegs_engine *e, const gegs_field &F)
+{
+    const float *first = &F.boundMinY[0][0], *end = (const float *)(&F + 1);
+    return widen_near_slack(e, first, (size_t)(end - first));
+}
+
 extern "C" {
 
 const char *gegs_version(void) { return "gegs_b200 0.1 (sm_100a)"; }
@@ -213,7 +237,7 @@ void gegs_destroy(gegs_engine *e)
     if (e->stream) cudaStreamSynchronize(e->stream);
     for (int k = 0; k < 2; k++) if (e->gexec[k]) cudaGraphExecDestroy(e->gexec[k]);
     cudaFree(e->d_blw); cudaFree(e->d_gvm); cudaFree(e->d_grad);
-    cudaFree(e->d_P); cudaFree(e->d_ptab); cudaFree(e->d_reg); cudaFree(e->d_xb); cudaFree(e->d_yb); cudaFree(e->d_zb);
+    cudaFree(e->d_P); cudaFree(e->d_ptab); cudaFree(e->d_etab); cudaFree(e->d_reg); cudaFree(e->d_xb); cudaFree(e->d_yb); cudaFree(e->d_zb);
     cudaFree(e->d_timeline);
     cudaFree(e->d_fields); cudaFree(e->d_cross); cudaFree(e->d_jaw_lines); cudaFree(e->d_phsp); cudaFree(e->d_tally);
     cudaFree(e->d_err); cudaFree(e->d_stats); cudaFree(e->d_sched); cudaFree(e->d_qmeta);
@@ -277,12 +301,31 @@ gegs_status gegs_set_physics(gegs_engine *e, const gegs_physics *P)
     std::vector<float4> ptab(ng);
     for (size_t i = 0; i < ng; i++)
         ptab[i] = make_float4(P->gmfp[i][0], P->gmfp[i][1], P->cohe[i][0], P->cohe[i][1]);
-    if (!e->d_ptab) CK(cudaMalloc(&e->d_ptab, ng * sizeof(float4)), "photon tables");
-    CK(cudaMemcpyAsync(e->d_ptab, ptab.data(), ng * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "tables H2D");
+    if (!e->d_ptab) {
+        CK(cudaMalloc(&e->d_ptab, (ng + 2 * kTablePad) * sizeof(float4)), "photon tables");
+        CK(cudaMemsetAsync(e->d_ptab, 0, (ng + 2 * kTablePad) * sizeof(float4), e->stream), "photon tables");
+    }
+    CK(cudaMemcpyAsync(e->d_ptab + kTablePad, ptab.data(), ng * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "tables H2D");
+    // the electron tables of a bin side by side (etab_index)
+    const size_t ne = (size_t)2 * GEGS_MXMED * GEGS_MXEKE;
+    std::vector<float4> etab(ne * 2);
+    for (size_t q = 0; q < 2; q++)
+        for (size_t i = 0; i < ne / 2; i++) {
+            const size_t k = q * (ne / 2) + i;
+            etab[2 * k] = make_float4(P->dedx[k][0], P->dedx[k][1], P->range_ep[2 * i + q], P->e_array[i]);
+            etab[2 * k + 1] = make_float4(P->sig[k][0], P->sig[k][1], P->tmxs[i][0], P->tmxs[i][1]);
+        }
+    if (!e->d_etab) {
+        CK(cudaMalloc(&e->d_etab, (2 * ne + 2 * kTablePad) * sizeof(float4)), "electron tables");
+        CK(cudaMemsetAsync(e->d_etab, 0, (2 * ne + 2 * kTablePad) * sizeof(float4), e->stream), "electron tables");
+    }
+    CK(cudaMemcpyAsync(e->d_etab + kTablePad, etab.data(), etab.size() * sizeof(float4), cudaMemcpyHostToDevice, e->stream),
+       "tables H2D");
     CK(cudaStreamSynchronize(e->stream), "physics sync");
     e->have_physics = true;
     e->ctx.P = e->d_P;
-    e->ctx.ptab = e->d_ptab;
+    e->ctx.ptab = e->d_ptab + kTablePad;
+    e->ctx.etab = e->d_etab + kTablePad;
     e->ctx.nmed = P->nmed;
     e->ctx_gen++;
     return GEGS_OK;
@@ -349,8 +392,10 @@ gegs_status gegs_set_scene(gegs_engine *e, const gegs_scene *S)
         CK(cudaMemcpy(e->d_jaw_lines, lines.data(), lines.size() * sizeof(float4), cudaMemcpyHostToDevice),
            "jaw lines H2D");
     }
-    if (!e->d_cross) CK(cudaMalloc(&e->d_cross, sizeof(float2) * 960), "crossXZ");
+    if (!e->d_cross) CK(cudaMalloc(&e->d_cross, sizeof(float2) * 968), "crossXZ");
     CK(cudaMemcpy(e->d_cross, S->crossXZ, sizeof(float2) * 960, cudaMemcpyHostToDevice), "crossXZ H2D");
+    CK(cudaMemcpy(e->d_cross + 960, S->boundaryXZ, sizeof(float2) * 4, cudaMemcpyHostToDevice), "MLC bounds H2D");
+    CK(cudaMemcpy(e->d_cross + 964, S->boundaryYZ, sizeof(float2) * 4, cudaMemcpyHostToDevice), "MLC bounds H2D");
     if (nvox != e->nvox || !e->d_tally) {
         CK(realloc_dev(&e->d_tally, nvox), "tally");
         e->nvox = nvox;
@@ -384,10 +429,12 @@ gegs_status gegs_set_scene(gegs_engine *e, const gegs_scene *S)
     C.mlc_x_start = S->mlc_x_start; C.mlc_x_end = S->mlc_x_end; C.mlc_x_mid_1 = S->mlc_x_mid_1;
     C.mlc_x_mid_2 = S->mlc_x_mid_2; C.mlc_air_gap = S->mlc_air_gap; C.mlc_wl_full = S->mlc_wl_full;
     C.mlc_wl_target = S->mlc_wl_target; C.mlc_wl_isocenter = S->mlc_wl_isocenter; C.mlc_wt = S->mlc_wt;
-    for (int i = 0; i < 4; i++) {
-        C.boundaryXZ[i] = make_float2(S->boundaryXZ[i][0], S->boundaryXZ[i][1]);
-        C.boundaryYZ[i] = make_float2(S->boundaryYZ[i][0], S->boundaryYZ[i][1]);
-    }
+    C.mlc_bounds = e->d_cross + 960;
+    C.near_slack = 0.0f;
+    widen_near_slack(e, &S->crossXZ[0][0], 960 * 2);
+    widen_near_slack(e, &S->boundaryXZ[0][0], 8);
+    widen_near_slack(e, &S->boundaryYZ[0][0], 8);
+    for (int f = 0; f < S->nfields; f++) widen_near_slack(e, S->fields[f]);
     for (int i = 0; i < 8; i++) C.module_order[i] = S->module_order[i];
     C.seed_lo = (uint32_t)S->seed;
     C.seed_hi = (uint32_t)(S->seed >> 32);
@@ -910,6 +957,7 @@ extern "C" gegs_status gegs_set_field(gegs_engine *e, int32_t index, const gegs_
     }
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     e->host_fields[(size_t)index] = *F;
+    if (widen_near_slack(e, *F)) e->ctx_gen++;
     std::vector<float4> lines = jaw_edge_lines(e->host_fields.data(), e->nfields);
     // the device arrays keep their addresses: graphs built before stay valid
     CK(cudaMemcpyAsync(e->d_fields + index, F, sizeof(gegs_field), cudaMemcpyHostToDevice, e->stream), "field H2D");

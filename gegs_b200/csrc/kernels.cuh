@@ -11,7 +11,7 @@
 // with a global atomic, and the host synchronises and reads the queue counters
 // back after every launch (CUDA_EGS.cu:226-365, 498-799).
 #pragma once
-#include "dev_electron.cuh"
+#include "dev_run.cuh"
 #include "../../include/gegs.h"     // gegs_probe_state
 
 // Step budgets in the tail of a run (fewer than batch / GX_TAIL_DIV particles
@@ -30,36 +30,6 @@
 // and GX_ERR_STEP_BUDGET is raised (guards the persistent loops against a
 // particle that stops making progress)
 #define GX_STEP_BUDGET 4000000u
-
-struct SchedState {
-    unsigned long long next, end;     // history cursor
-    unsigned long long h0, h1;        // histories injected by the current wave
-    uint32_t batch, waves, max_waves, pending;
-    uint32_t refill_below;
-    uint32_t photon_done;             // photon MLC and phantom consumers finished in this wave
-    uint32_t electron_done;           // electron branches finished in this wave
-    uint32_t budget_shift;            // step budgets of the next wave are shifted left by this (tail of a run)
-};
-
-// ---- wave timeline (tracing; off unless DevCtx::timeline is set) ------------
-// Kernel ids: 0 source; 1-3 photon jaws / MLC / phantom; 4-7 Compton, photo,
-// Rayleigh, pair; 8-10 electron jaws / MLC / phantom; 11-14 Moller, brems,
-// Bhabha, annihilation. Each block's thread 0 lowers the kernel's start stamp
-// of this wave when the block begins and raises its end stamp once the block
-// is done (after the block's barrier).
-enum : int { TL_SOURCE = 0, TL_PHOTON = 1, TL_PINT = 4, TL_ELECTRON = 8, TL_EINT = 11, TL_ENEAR = 15, TL_PLONG = 16 };
-
-__device__ __forceinline__ void timeline_mark(const DevCtx &C, int kernel, bool end)
-{
-    if (C.timeline == nullptr || threadIdx.x != 0) return;
-    uint32_t w = *((volatile const uint32_t *)C.wave);
-    if (w >= C.timeline_waves) return;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    unsigned long long *slot = C.timeline + ((size_t)w * GX_TL_KERNELS + (size_t)kernel) * 2;
-    if (end) atomicMax(slot + 1, t);
-    else atomicMin(slot, t);
-}
 
 __device__ __forceinline__ void consumer_done(const DevCtx &C, int q, int q2 = -1, uint32_t *finished = nullptr)
 {
@@ -82,47 +52,23 @@ __device__ __forceinline__ void consumer_done(const DevCtx &C, int q, int q2 = -
     }
 }
 
-// Re-queue a particle whose per-launch step budget ran out (same stream, same
-// state: the result does not depend on where a track is split).
-__device__ __forceinline__ void push_cont(const DevCtx &C, int qid, Part p, const Rng &r, const EStatePk *st)
+// Queue a particle of a transport for a stage, or for the next wave as it
+// stands (electrons with their step state), into `qid`.
+template <bool ELEC>
+__device__ __forceinline__ void queue_particle(const DevCtx &C, int qid, Part &p, const Rng &r, const EState &s)
 {
     rng_store(r, p);
-    // lanes of a warp may push to different queues here: one atomic per queue
-    cg::coalesced_group g = cg::labeled_partition(cg::coalesced_threads(), qid);
-    uint32_t base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(&C.q.count[qid], (uint32_t)g.size());
-    base = g.shfl(base, 0);
-    uint32_t idx = base + g.thread_rank();
-    if (idx < C.q.cap[qid]) {
-        store_part(&C.q.buf[qid][idx], p);
-        if (st) C.q.estate[qid - GX_Q_ECONT][idx] = *st;
+    if (qid < GX_NSTAGE) {
+        p.status = (uint8_t)qid;
+        trace_event(C, 0u, qid, p);
+    }
+    const uint32_t i = queue_place(C.q.count, qid);
+    if (i < C.q.cap[qid]) {
+        store_part(&C.q.buf[qid][i], p);
+        if (ELEC && qid >= GX_Q_ECONT) C.q.estate[qid - GX_Q_ECONT][i] = pack_estate(s);
     } else {
         atomicOr(C.err, GX_ERR_QUEUE_FULL);
     }
-}
-
-__device__ __forceinline__ EStatePk pack_estate(const EState &s)
-{
-    EStatePk k;
-    k.elke = s.elke; k.demfp = s.demfp; k.sig0 = s.sig0; k.total_tstep = s.total_tstep;
-    k.lelke = s.lelke;
-    k.flags = (s.compute_tstep ? 1u : 0u) | (s.is_tstep ? 2u : 0u);
-    k.pad0 = 0; k.pad1 = 0;
-    return k;
-}
-
-__device__ __forceinline__ void unpack_estate(const EStatePk &k, EState &s)
-{
-    s.elke = k.elke; s.demfp = k.demfp; s.sig0 = k.sig0; s.total_tstep = k.total_tstep;
-    s.lelke = k.lelke;
-    s.compute_tstep = (k.flags & 1u) != 0;
-    s.is_tstep = (k.flags & 2u) != 0;
-}
-
-__device__ __forceinline__ uint32_t queue_len(const DevCtx &C, int q)
-{
-    uint32_t n = *((volatile uint32_t *)&C.q.count[q]);
-    return n < C.q.cap[q] ? n : C.q.cap[q];
 }
 
 __device__ __forceinline__ void block_stat_add(const DevCtx &C, int slot, unsigned long long v)
@@ -132,58 +78,7 @@ __device__ __forceinline__ void block_stat_add(const DevCtx &C, int slot, unsign
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(&C.stats[slot], v);
 }
 
-// ---- source: history index -> primary (CUDA_EGS.cu:52-131) -----------------
-__device__ bool make_primary(const DevCtx &C, unsigned long long h, Part &p)
-{
-    int f;
-    for (f = 0; f < C.nfields; f++) {
-        unsigned long long hb = C.fields[f].hist_begin, he = C.fields[f].hist_end;
-        if (h >= hb && h < he) break;
-    }
-    if (f == C.nfields) return false;
-    const gegs_field *F = &C.fields[f];
-    unsigned long long j = (h - F->hist_begin) / (unsigned long long)(F->nrepeat + 1);
-    const gegs_phsp_record *rec = &C.phsp[j % C.nphsp];
-    uint32_t latch = __ldg(&rec->latch);
-    float re = __ldg(&rec->e), rx = __ldg(&rec->x), ry = __ldg(&rec->y);
-    float ru = __ldg(&rec->u), rv = __ldg(&rec->v), rwt = __ldg(&rec->wt);
-    int q;
-    if (latch & 0x40000000u) q = -1;
-    else if (latch & 0x20000000u) q = 1;
-    else q = 0;
-    float w2 = 1.0f - ru * ru - rv * rv;
-    float w = sqrtf(w2 > 0.0f ? w2 : 0.0f);
-    float wt = rwt;
-    if (wt < 0.0f) { w = -w; wt = -wt; }
-    p.charge = (int8_t)q;
-    p.e = re < 0.0f ? -re : re;
-    p.wt = wt;
-    p.region = 0;
-    p.leafIndex = GX_OUTMLC;
-    p.bank = -1;
-    p.module = (uint8_t)C.module_order[0];
-    p.field = (uint8_t)f;
-    p.x = rx; p.y = ry; p.z = C.z_phsp;
-    p.u = ru; p.v = rv; p.w = w;
-    p.hist_lo = (uint32_t)h;
-    p.hist_hi = (uint32_t)(h >> 32);
-    p.sid_lo = 0; p.sid_hi = 0; p.ctr = 0;
-    p.status = 0;
-    // beamlet: the bixel of the isocentre plane on the primary's straight line
-    p.beamlet = GX_NO_BEAMLET;
-    if (C.bl_nx > 0 && w > 0.0f) {
-        float t = (C.sid - C.z_phsp) / w;
-        float xi = rx + ru * t, yi = ry + rv * t;
-        float fx = (xi - C.bl_x0) / C.bl_dx, fy = (yi - C.bl_y0) / C.bl_dy;
-        if (fx >= 0.0f && fy >= 0.0f && fx < (float)C.bl_nx && fy < (float)C.bl_ny) {
-            int b = f * C.bl_nx * C.bl_ny + (int)fy * C.bl_nx + (int)fx;
-            p.beamlet = (uint16_t)b;
-            if (C.bl_weight) p.wt = wt * __ldg(&C.bl_weight[b]);
-        }
-    }
-    return true;
-}
-
+// ---- source ------------------------------------------------------------------
 __global__ void k_source(const __grid_constant__ DevCtx C, const SchedState *st)
 {
     timeline_mark(C, TL_SOURCE, false);
@@ -206,7 +101,7 @@ __global__ void k_source(const __grid_constant__ DevCtx C, const SchedState *st)
 // counter `hq`; idle lanes of a warp are refilled with one atomic.
 template <int Q, bool ELEC>
 __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont, uint32_t n, int qc, bool &exhausted,
-                                       bool active, Part &p, Rng &r, EState *s, unsigned long long &taken)
+                                       bool active, Part &p, Rng &r, EState &s, Vox &vx, unsigned long long &taken)
 {
     const uint32_t lane = threadIdx.x & 31u;
     unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -219,14 +114,14 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
     if (!active) {
         uint32_t idx = base + __popc(need & ((1u << lane) - 1u));
         if (idx < n) {
-            if (idx < n_cont) {
-                p = load_part(&C.q.buf[qc][idx]);
-                rng_load(r, p);
-                if (ELEC) unpack_estate(C.q.estate[qc - GX_Q_ECONT][idx], *s);
+            const bool cont = idx < n_cont;
+            p = load_part(cont ? &C.q.buf[qc][idx] : &C.q.buf[Q][idx - n_cont]);
+            rng_load(r, p);
+            vx = C.reg[p.region];
+            if (cont) {
+                if (ELEC) unpack_estate(C.q.estate[qc - GX_Q_ECONT][idx], s);
             } else {
-                p = load_part(&C.q.buf[Q][idx - n_cont]);
-                rng_load(r, p);
-                if (ELEC) estate_init(*s);
+                if (ELEC) estate_init(s);
                 trace_event(C, 1u, Q, p);
                 taken++;
             }
@@ -325,48 +220,41 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
     Part p;
     Rng r;
     EState s;
+    Vox vx;
     bool active = false, exhausted = false;
     unsigned long long taken = 0, steps = 0;
     uint32_t nst = 0;
     for (;;) {
-        bool was = active;
-        active = refill<Q, ELEC>(C, hq, n_cont, n, qc_in, exhausted, active, p, r, &s, taken);
+        const bool was = active;
+        active = refill<Q, ELEC>(C, hq, n_cont, n, qc_in, exhausted, active, p, r, s, vx, taken);
         if (active && !was) nst = 0;
         if (!__any_sync(0xffffffffu, active)) break;
         if (active) {
-            if (!in_geom_class<G>(p)) {
-                const int tq = base + 2 * (geom_class_of(p.module) - GX_GEOM_JAWS) + (int)(par ^ 1u);
-                if (ELEC) { EStatePk k = pack_estate(s); push_cont(C, tq, p, r, &k); }
-                else push_cont(C, tq, p, r, nullptr);
-                active = false;
-            } else {
+            int tq = -1;                          // the queue the particle leaves for
+            if (!in_geom_class<G>(p)) tq = base + 2 * (geom_class_of(p.module) - GX_GEOM_JAWS) + (int)(par ^ 1u);
+            else {
                 steps++;
                 rng_window(C, r);
-                bool done;
-                if (DEFER || (ELEC && NEAR)) {
-                    const uint32_t ctr0 = r.ctr;
-                    const EState s0 = s;
-                    const int code = DEFER ? electron_step<G, true, false>(C, p, r, s)
-                                           : electron_step<G, false, true>(C, p, r, s);
-                    if (code >= 2) {
-                        // needs howfar (to the near-boundary pass) or, in that pass, does
-                        // not (back to the first pass of the next wave): re-queued as it stood
-                        r.ctr = ctr0;
-                        EStatePk k = pack_estate(s0);
-                        push_cont(C, code == 2 ? GX_Q_ENEAR + cls : qc_out, p, r, &k);
-                        steps--;
-                    }
-                    done = code != 0;                 // leaves this pass either way
-                } else done = ELEC ? electron_step<G>(C, p, r, s) != 0 : photon_step<G, true>(C, p, r);
-                if (done) active = false;
-                else if (++nst >= budget &&
-                         (!JAWS_PHOTON || !C.overlap || nst >= 64u * budget ||
-                          (((nst - budget) & 15u) == 0u &&
-                           *others_done + (C.pipelined && !LONG ? *others_done2 : 0u) >= others))) {
-                    if (ELEC) { EStatePk k = pack_estate(s); push_cont(C, qc_out, p, r, &k); }
-                    else push_cont(C, q_limit, p, r, nullptr);
-                    active = false;
-                }
+                const uint32_t ctr0 = r.ctr;
+                const EState s0 = s;
+                const int code = ELEC ? electron_step<G, DEFER, ELEC && NEAR>(C, p, r, s, vx, tq) : photon_step<G, true>(C, p, r, vx, tq);
+                if (code == STEP_DONE) active = false;
+                else if ((DEFER && code == STEP_NEAR) || (ELEC && NEAR && code == STEP_FAR)) {
+                    // needs howfar (to the near-boundary pass) or, in that pass, does
+                    // not (back to the first pass of the next wave): as it stood
+                    r.ctr = ctr0;
+                    s = s0;
+                    tq = DEFER ? GX_Q_ENEAR + cls : qc_out;
+                    steps--;
+                } else if (code == STEP_ON && ++nst >= budget &&
+                           (!JAWS_PHOTON || !C.overlap || nst >= 64u * budget ||
+                            (((nst - budget) & 15u) == 0u &&
+                             *others_done + (C.pipelined && !LONG ? *others_done2 : 0u) >= others)))
+                    tq = ELEC ? qc_out : q_limit;
+            }
+            if (tq >= 0) {
+                queue_particle<ELEC>(C, tq, p, r, s);
+                active = false;
             }
         }
     }
@@ -429,32 +317,6 @@ __global__ void __launch_bounds__(256, GX_EPHANTOM_MIN_BLOCKS) k_electron(const 
 }
 
 template <int Q>
-__device__ __forceinline__ void run_interaction(const DevCtx &C, const Part &p, Rng &r)
-{
-    if (Q == ST_COMPTON) compton(C, p, r);
-    else if (Q == ST_PHOTO) photo(C, p, r);
-    else if (Q == ST_RAYLEIGH) rayleigh(C, p, r);
-    else if (Q == ST_PAIR) pair(C, p, r);
-    else if (Q == ST_MOLLER) moller(C, p, r);
-    else if (Q == ST_BREMS) brems(C, p, r);
-    else if (Q == ST_BHABHA) bhabha(C, p, r);
-    else if (Q == ST_ANNIH) {
-        if (at_rest_mark(p)) {
-            Part q = p;
-            annih_at_rest(C, q, region_info(C, q.region), r);
-        } else annih(C, p, r);
-    }
-}
-
-// Entries an interaction kernel counts as processed: all but the positrons
-// handed over at rest (counted nowhere in the serial form either).
-template <int Q>
-__device__ __forceinline__ unsigned counted(const Part &p)
-{
-    return (Q == ST_ANNIH && at_rest_mark(p)) ? 0u : 1u;
-}
-
-template <int Q>
 __global__ void __launch_bounds__(256) k_interact(const __grid_constant__ DevCtx C)
 {
     constexpr int tl = Q < ST_ELECTRON ? TL_PINT + (Q - ST_COMPTON) : TL_EINT + (Q - ST_MOLLER);
@@ -489,22 +351,18 @@ __global__ void __launch_bounds__(256) k_plain(const __grid_constant__ DevCtx C)
         rng_load(r, p);
         trace_event(C, 1u, Q, p);
         taken += counted<Q>(p);
-        if (Q == ST_PHOTON) {
-            uint32_t nst = 0;
-            while (!photon_step(C, p, r)) {
-                steps++;
-                if (++nst > GX_STEP_BUDGET) { atomicOr(C.err, GX_ERR_STEP_BUDGET); break; }
-            }
-            steps++;
-        } else if (Q == ST_ELECTRON) {
+        if (Q == ST_PHOTON || Q == ST_ELECTRON) {
             EState s;
             estate_init(s);
+            Vox vx = C.reg[p.region];
             uint32_t nst = 0;
-            while (!electron_step(C, p, r, s)) {
+            int code, out = 0;
+            do {
+                code = Q == ST_PHOTON ? photon_step(C, p, r, vx, out) : electron_step(C, p, r, s, vx, out);
                 steps++;
                 if (++nst > GX_STEP_BUDGET) { atomicOr(C.err, GX_ERR_STEP_BUDGET); break; }
-            }
-            steps++;
+            } while (code == STEP_ON);
+            if (code == STEP_QUEUE) push_move(C, out, p, r);
         } else {
             run_interaction<Q>(C, p, r);
         }

@@ -60,3 +60,63 @@ def test_device_geometry_equals_the_oracle(engine, name):
         want = pair.geom(parts, t_in)
         res = engine.probe_geometry(parts, t_in)
         _compare(res, want["region"], want["t"], want["particle"], want["tperp"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0.0, 1e-6, 1e-4, 2e-3])
+def test_device_geometry_at_polygon_vertices_and_edges(engine, offset):
+    """Where the polygon routines pick out the edges that they divide for:
+    points on, and `offset` cm around, the vertices and edge midpoints of the
+    leaf cross sections, the leaf-end outlines and the jaws, with directions
+    along the axes (edges parallel to the ray) and oblique ones, in a leaf, in a
+    gap, outside, and with the bank known or not. Bit for bit as the oracle."""
+    from oracle import refpin as R
+    job = RC.job("c3")
+    sh = _engine(engine, job)
+    pair = R.OraclePair(job.physics, sh)
+    cap = pair.capture(0, 2000, every=1, cap_n=20000)
+    base = np.concatenate([cap[0], cap[5]])
+    rng = np.random.default_rng(29)
+    cross = np.ctypeslib.as_array(sh.scene.crossXZ).reshape(60, 16, 2)[:, :14]
+    out = []
+    for module, n in ((3, 6000), (1, 2000), (2, 2000)):
+        have = base[base["module"] == module]
+        p = have[rng.integers(0, len(have), n)].copy()
+        f = p["field"] = rng.integers(0, len(job.fields), n)
+        k = rng.integers(0, 60, n)
+        if module == 3:
+            leaf = k.astype(np.int8)
+            end = np.stack([np.ctypeslib.as_array(sh.scene.fields[i].endnode) for i in range(len(job.fields))])
+            a, b = cross[k, k % 14], cross[k, (k + 1) % 14]
+            mid = rng.integers(0, 2, n)[:, None] / 2.0
+            xz = a + (b - a) * mid
+            yz = end[f, k, rng.integers(0, 34, n)]
+            on_x = rng.integers(0, 2, n) == 0
+            p["x"] = np.where(on_x, xz[:, 0], cross[k].mean(1)[:, 0])
+            p["y"] = np.where(on_x, rng.uniform(-8, 8, n), yz[:, 0])
+            p["z"] = np.where(on_x, xz[:, 1], yz[:, 1])
+            p["leafIndex"] = np.choose(rng.integers(0, 4, n), [leaf, leaf, -np.maximum(leaf, 1), -99])
+            p["bank"] = np.choose(rng.integers(0, 4, n), [-1, 0, 1, 2])
+            p["region"] = np.where(p["bank"] > 0, 3, 1)
+        else:
+            geo = "jawsGeomX" if module == 2 else "jawsGeomY"
+            v = np.stack([np.ctypeslib.as_array(getattr(sh.scene.fields[i], geo)) for i in range(len(job.fields))])
+            q = v[f, rng.integers(0, 8, n)]
+            p["y" if module == 2 else "x"] = q[:, 0]
+            p["x" if module == 2 else "y"] = rng.uniform(-4, 4, n)
+            p["z"] = q[:, 1]
+            p["region"] = rng.integers(1, 3, n)
+        for c in ("x", "y", "z"):
+            p[c] = (p[c] + offset * rng.integers(-1, 2, n)).astype(np.float32)
+        d = rng.normal(size=(n, 3)).astype(np.float32)
+        d[np.arange(n), rng.integers(0, 3, n)] *= rng.integers(0, 2, n)
+        d[np.arange(n), rng.integers(0, 3, n)] *= rng.integers(0, 2, n)
+        d[(d == 0).all(1)] = (0, 0, 1)
+        d /= np.linalg.norm(d, axis=1, keepdims=True)
+        p["u"], p["v"], p["w"] = d[:, 0], d[:, 1], d[:, 2]
+        out.append(p)
+    parts = np.concatenate(out)
+    for t_in in (np.full(len(parts), 1e3, np.float32), rng.exponential(0.3, len(parts)).astype(np.float32)):
+        want = pair.geom(parts, t_in)
+        res = engine.probe_geometry(parts, t_in)
+        _compare(res, want["region"], want["t"], want["particle"], want["tperp"])
