@@ -44,7 +44,7 @@ STAGES = ["photon", "compton", "photo", "rayleigh", "pair", "electron", "moller"
 
 def build(force=False):
     """Build the harness from the reference sources when they are present."""
-    if not REF_DIR.is_dir():
+    if not (REF_DIR / "geom.cu").is_file():
         return None
     srcs = [p for p in (HERE / "ref").rglob("*") if p.is_file()] + [HERE / "ora_base.c", HERE / "gegs_oracle.h"]
     if force or not REF_LIB.exists() or any(s.stat().st_mtime > REF_LIB.stat().st_mtime for s in srcs):
