@@ -9,6 +9,7 @@ from __future__ import annotations
 import os
 import pathlib
 import subprocess
+import tempfile
 
 PKG = pathlib.Path(__file__).resolve().parent
 SRC = PKG / "csrc"
@@ -19,7 +20,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
     "-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
 ]
 
 
@@ -39,14 +40,18 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
     if not force and not needs_build():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc, *NVCC_FLAGS, "-Xcompiler", "-ffp-contract=off", "-o", str(LIB), str(SRC / "engine.cu"),
-           str(SRC / "postproc.cu"), str(SRC / "plan_host.cpp")]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    tmp = LIB.with_suffix(".so.tmp")
-    cmd[cmd.index(str(LIB))] = str(tmp)
-    subprocess.run(cmd, check=True)
-    os.replace(tmp, LIB)
+    units = sorted(list(SRC.glob("*.cu")) + list(SRC.glob("*.cpp")))
+    flags = [*(["-Xptxas=-v"] if verbose else []), *NVCC_FLAGS, "-Xcompiler", "-ffp-contract=off"]
+    with tempfile.TemporaryDirectory() as tmp:
+        # the translation units side by side: each holds kernels that take a minute or two
+        objs = [pathlib.Path(tmp) / (u.name + ".o") for u in units]
+        jobs = [subprocess.Popen([nvcc, *flags, "-c", str(u), "-o", str(o)]) for u, o in zip(units, objs)]
+        for u, j in zip(units, [j.wait() for j in jobs]):
+            if j != 0:
+                raise subprocess.CalledProcessError(j, f"nvcc -c {u}")
+        out = LIB.with_suffix(".so.tmp")
+        subprocess.run([nvcc, *NVCC_FLAGS, "-shared", "-o", str(out), *map(str, objs)], check=True)
+    os.replace(out, LIB)
     return LIB
 
 

@@ -58,6 +58,14 @@ static_assert(sizeof(gegs_field) % 16 == 0, "field record size");
 #define GX_NQ 25
 #define GX_NESTATE 8
 #define GX_TL_KERNELS 32   // wave timeline slots per wave
+// The drain kernel's particle types: photons and electrons of each geometry
+// class, then the eight interactions in stage order; and the records of one
+// type that a warp's stack holds (fewer than 32 when a warp claims 32 more).
+#define GX_DT_P 0
+#define GX_DT_E 3
+#define GX_DT_I 6
+#define GX_DT_N 14
+#define GX_DRAIN_CAP 64
 #define GX_LOOP_CAP 1000
 // The reference's step constants are double literals (EGSnrc_Parameters.h:91-92,
 // CUDA_EGS.h:34): a step that adds EPSTEP, and a comparison with EPSGMFP or
@@ -190,6 +198,8 @@ struct DevCtx {
                                     // phases (persistent form); a positron that stops in the electron
                                     // transport annihilates at rest in the annihilation kernel
     uint32_t photon_budget, electron_budget;   // steps per particle per launch before continuation
+    Part *drain_part;       // the drain kernel's stacks: [warp][GX_DT_N][GX_DRAIN_CAP]
+    EStatePk *drain_estate; // [warp][3][GX_DRAIN_CAP], step states of the electrons on them
     unsigned long long *timeline;   // [timeline_waves][16][2] first start / last end (ns) per kernel; null: off
     uint32_t timeline_waves;
     QueueSet q;
@@ -462,6 +472,10 @@ __device__ __forceinline__ void trace_event(const DevCtx &C, uint32_t kind, int 
     trace_write(C.trace, C.trace_n, C.trace_cap, t);
 }
 
+#ifdef GX_WARP_STACKS
+// In the drain kernel a particle made by a warp stays with it (drain.cu).
+__device__ __forceinline__ void push(const DevCtx &C, int qid, const Part &p);
+#else
 // A place in queue `qid` for one record of the calling lane; lanes of the warp
 // that want one of the same queue at the same time share one atomic.
 __device__ __forceinline__ uint32_t queue_place(uint32_t *count, int qid)
@@ -495,6 +509,7 @@ __device__ __forceinline__ void push(const DevCtx &C, int qid, const Part &p)
     const uint4 *s = reinterpret_cast<const uint4 *>(&r);
     push_record(C.q.count, C.q.buf[qid], C.q.cap[qid], C.err, qid, s[0], s[1], s[2], s[3]);
 }
+#endif
 
 // push of a particle that keeps its stream (stage change)
 __device__ __forceinline__ void push_move(const DevCtx &C, int qid, Part p, const Rng &r)

@@ -11,6 +11,9 @@ struct SchedState {
     uint32_t refill_below;
     uint32_t photon_done;             // photon MLC and phantom consumers finished in this wave
     uint32_t electron_done;           // electron branches finished in this wave
+    uint32_t drain_below;             // the drain kernel takes over at this many particles and histories left (0: never)
+    uint32_t drain;                   // 1: it does, after this plan
+    unsigned long long drain_hist;    // histories it has claimed
     uint32_t budget_shift;            // step budgets of the next wave are shifted left by this (tail of a run)
 };
 
@@ -20,7 +23,7 @@ struct SchedState {
 // Bhabha, annihilation. Each block's thread 0 lowers the kernel's start stamp
 // of this wave when the block begins and raises its end stamp once the block
 // is done (after the block's barrier).
-enum : int { TL_SOURCE = 0, TL_PHOTON = 1, TL_PINT = 4, TL_ELECTRON = 8, TL_EINT = 11, TL_ENEAR = 15, TL_PLONG = 16 };
+enum : int { TL_SOURCE = 0, TL_PHOTON = 1, TL_PINT = 4, TL_ELECTRON = 8, TL_EINT = 11, TL_ENEAR = 15, TL_PLONG = 16, TL_DRAIN = 17 };
 
 __device__ __forceinline__ void timeline_mark(const DevCtx &C, int kernel, bool end)
 {

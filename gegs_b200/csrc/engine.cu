@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 #include "kernels.cuh"
+#include "drain.cuh"
 #include "../../include/gegs.h"
 
 namespace {
@@ -86,6 +87,12 @@ struct gegs_engine {
     uint32_t qcap[GX_NQ] = {};
     uint32_t batch = 0;
     uint32_t queue_cap = 0;            // gegs_run_opts::queue_cap of the current queues
+
+    // drain kernel (drain.cu): its stacks and the grid they are sized for
+    Part *d_drain_part = nullptr;
+    EStatePk *d_drain_estate = nullptr;
+    int drain_grid = 0;
+    bool has_head = true;              // the scene's modules include jaws or an MLC (or one this path does not model)
 
     DevCtx ctx{};
     bool have_physics = false, have_scene = false;
@@ -245,6 +252,7 @@ void gegs_destroy(gegs_engine *e)
     cudaFree(e->d_stat_s1); cudaFree(e->d_stat_s2); cudaFree(e->d_stat_snap);
     for (int q = 0; q < GX_NQ; q++) cudaFree(e->d_qbuf[q]);
     for (int k = 0; k < GX_NESTATE; k++) cudaFree(e->d_estate[k]);
+    cudaFree(e->d_drain_part); cudaFree(e->d_drain_estate);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     for (int k = 0; k < kAux; k++) {
@@ -436,6 +444,7 @@ gegs_status gegs_set_scene(gegs_engine *e, const gegs_scene *S)
     widen_near_slack(e, &S->boundaryYZ[0][0], 8);
     for (int f = 0; f < S->nfields; f++) widen_near_slack(e, S->fields[f]);
     for (int i = 0; i < 8; i++) C.module_order[i] = S->module_order[i];
+    e->has_head = C.module_order[0] != GEGS_M_PHANTOM;   // a beam line of the phantom alone?
     C.seed_lo = (uint32_t)S->seed;
     C.seed_hi = (uint32_t)(S->seed >> 32);
     // beamlet grid and fluence weights
@@ -476,8 +485,9 @@ constexpr unsigned long long kQueueBytesPerParticle =
     cap_factor_sum() * sizeof(Part) + estate_factor_sum() * sizeof(EStatePk);
 
 // In-flight batch when the caller leaves it at 0: 60 % of the run's histories
-// in steps of 64K, between 64K and 30M (about 157 GB of queues), and within
-// 85 % of the device memory that is free once this engine's current queues are
+// (all of them up to 1M: a small run fills no SM as it is, and every injection
+// costs it a build-up and a decline of short waves) in steps of 64K, between
+// 64K and 30M (about 157 GB of queues), and within 85 % of the device memory that is free once this engine's current queues are
 // counted as free. More particles in flight keep more lanes busy and need
 // fewer waves: on the CT 5-field plan's 40M-history steps, 24M in flight is
 // 2.9 % faster than 16M, 16M 7 % faster than 6M, and 26M to 30M gain nothing
@@ -486,8 +496,10 @@ constexpr unsigned long long kQueueBytesPerParticle =
 static uint32_t default_batch(gegs_engine *e, uint64_t histories)
 {
     const uint64_t step = 1ull << 16, most = 30ull << 20;
+    const uint64_t small = 1ull << 20;
     uint64_t want = histories / 5 * 3;
     want = want / step * step;
+    if (want < small) want = histories < small ? (histories + step - 1) / step * step : small;
     if (want < step) want = step;
     if (want > most) want = most;
     size_t free_b = 0, total_b = 0;
@@ -559,6 +571,9 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
     };
     k_source<<<grid, threads, 0, s>>>(C, e->d_sched);
     const size_t ps = C.stage_tables ? photon_smem_bytes(C.nmed) : 0;   // the staged {gmfp, cohe} table
+    // A beam line of the phantom alone leaves the queues of the jaws and the MLC
+    // empty: their kernels, six of a wave's eight transports, are not launched.
+    const bool head = e->has_head;
     if (C.pipelined) {
         // Both transport phases at once: the photon consumers read the photon
         // queues, the electron consumers the electron queues, and neither
@@ -572,16 +587,21 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
         // Measured on the 40M-history C3 step against the order jaws, MLC,
         // phantom with photons and electrons interleaved: 1.7 % faster; the
         // jaws photons created last: 6 % slower.
-        fork(5);
-        k_photon_jaws<<<grid, threads, ps, a[0]>>>(C);
-        k_photon_mlc<<<grid, threads, ps, a[1]>>>(C);
+        const int branches = head ? 5 : 1;
+        fork(branches);
+        if (head) {
+            k_photon_jaws<<<grid, threads, ps, a[1]>>>(C);
+            k_photon_mlc<<<grid, threads, ps, a[2]>>>(C);
+        }
         k_photon<<<grid, threads, ps, s>>>(C);
-        k_electron<<<grid, threads, 0, a[4]>>>(C);
-        k_electron_mlc<<<grid, threads, 0, a[3]>>>(C);
-        k_electron_mlc_near<<<grid, threads, 0, a[3]>>>(C);
-        k_electron_jaws<<<grid, threads, 0, a[2]>>>(C);
-        k_electron_jaws_near<<<grid, threads, 0, a[2]>>>(C);
-        join(5);
+        k_electron<<<grid, threads, 0, a[0]>>>(C);
+        if (head) {
+            k_electron_mlc<<<grid, threads, 0, a[3]>>>(C);
+            k_electron_mlc_near<<<grid, threads, 0, a[3]>>>(C);
+            k_electron_jaws<<<grid, threads, 0, a[4]>>>(C);
+            k_electron_jaws_near<<<grid, threads, 0, a[4]>>>(C);
+        }
+        join(branches);
         fork(7);
         k_interact<ST_COMPTON><<<grid, threads, 0, s>>>(C);
         k_interact<ST_PHOTO><<<grid, threads, 0, a[0]>>>(C);
@@ -595,8 +615,10 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
         return;
     }
     fork(2);
-    k_photon_jaws<<<grid, threads, ps, a[0]>>>(C);
-    k_photon_mlc<<<grid, threads, ps, a[1]>>>(C);
+    if (head) {
+        k_photon_jaws<<<grid, threads, ps, a[0]>>>(C);
+        k_photon_mlc<<<grid, threads, ps, a[1]>>>(C);
+    }
     k_photon<<<grid, threads, ps, s>>>(C);
     join(2);
     fork(3);
@@ -606,11 +628,13 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
     k_interact<ST_PAIR><<<grid, threads, 0, a[2]>>>(C);
     join(3);
     fork(3);
-    k_photon_jaws_long<<<grid, threads, ps, a[2]>>>(C);
-    k_electron_jaws<<<grid, threads, 0, a[0]>>>(C);
-    k_electron_jaws_near<<<grid, threads, 0, a[0]>>>(C);
-    k_electron_mlc<<<grid, threads, 0, a[1]>>>(C);
-    k_electron_mlc_near<<<grid, threads, 0, a[1]>>>(C);
+    if (head) {
+        k_photon_jaws_long<<<grid, threads, ps, a[2]>>>(C);
+        k_electron_jaws<<<grid, threads, 0, a[0]>>>(C);
+        k_electron_jaws_near<<<grid, threads, 0, a[0]>>>(C);
+        k_electron_mlc<<<grid, threads, 0, a[1]>>>(C);
+        k_electron_mlc_near<<<grid, threads, 0, a[1]>>>(C);
+    }
     k_electron<<<grid, threads, 0, s>>>(C);
     join(3);
     fork(3);
@@ -621,36 +645,40 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
     join(3);
 }
 
-// Adds an engine's wave loop to g: a WHILE node whose body is one wave and
-// whose condition k_plan_cond sets on the device. With a planner, the loop is
-// preceded by the k_plan node that plans the first wave (a run launched on
-// its own launches k_plan before the graph instead).
-static gegs_status add_wave_loop(gegs_engine *e, cudaGraph_t g, int grid, int threads, bool with_planner)
+// Adds an engine's run to g: the first plan, a WHILE node whose body is one
+// wave and whose condition k_plan_cond sets on the device, then the drain
+// kernel for what the plan left to it.
+static gegs_status add_wave_loop(gegs_engine *e, cudaGraph_t g, int grid, int threads)
 {
+    cudaGraphConditionalHandle handle;
+    CK(cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault), "conditional handle");
     cudaGraphNode_t pnode = nullptr;
-    if (with_planner) {
-        void *args[] = {(void *)&e->ctx, (void *)&e->d_sched};
+    {
+        void *args[] = {(void *)&e->ctx, (void *)&e->d_sched, (void *)&handle};
         cudaKernelNodeParams kp = {};
-        kp.func = (void *)k_plan;
+        kp.func = (void *)k_plan_cond;
         kp.gridDim = dim3(1);
-        kp.blockDim = dim3(1);
+        kp.blockDim = dim3(32);
         kp.kernelParams = args;
         CK(cudaGraphAddKernelNode(&pnode, g, nullptr, 0, &kp), "planner node");
     }
-    cudaGraphConditionalHandle handle;
-    CK(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault), "conditional handle");
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
     cudaGraphNode_t cnode;
-    CK(cudaGraphAddNode(&cnode, g, pnode ? &pnode : nullptr, pnode ? 1 : 0, &cp), "conditional node");
+    CK(cudaGraphAddNode(&cnode, g, &pnode, 1, &cp), "conditional node");
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(e->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
     launch_wave_kernels(e, grid, threads);
-    k_plan_cond<<<1, 1, 0, e->stream>>>(e->ctx, e->d_sched, handle);
+    k_plan_cond<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched, handle);
     cudaGraph_t captured;
+    CK(cudaStreamEndCapture(e->stream, &captured), "end capture");
+    if (!e->drain_grid) return GEGS_OK;     // no run of this engine has left anything to the drain kernel yet
+    CK(cudaStreamBeginCaptureToGraph(e->stream, g, &cnode, nullptr, 1, cudaStreamCaptureModeThreadLocal), "capture");
+    launch_drain(e->ctx, e->d_sched, e->has_head, e->drain_grid, e->stream);
+    k_drain_end<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
     CK(cudaStreamEndCapture(e->stream, &captured), "end capture");
     return GEGS_OK;
 }
@@ -663,7 +691,7 @@ static gegs_status build_graph(gegs_engine *e, int grid, int threads)
     if (e->gexec[k]) { cudaGraphExecDestroy(e->gexec[k]); e->gexec[k] = nullptr; }
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0), "graph create");
-    gegs_status st = add_wave_loop(e, g, grid, threads, false);
+    gegs_status st = add_wave_loop(e, g, grid, threads);
     if (st != GEGS_OK) { cudaGraphDestroy(g); return st; }
     CK(cudaGraphInstantiate(&e->gexec[k], g, 0), "graph instantiate");
     cudaGraphDestroy(g);
@@ -689,6 +717,37 @@ struct GroupRun {
 
 static gegs_status run_finish(gegs_engine *e);
 
+// The drain kernel takes over at this many particles and histories left: where
+// the waves' fixed cost (some 100 us) weighs more than the lanes that a warp
+// working by itself leaves idle. Device ms with 0 / 2000 / 4000 / 8000 / 12000:
+// water, 10 000 histories 3.62 / 2.19 / 2.16 / 2.14 / 3.83 (there all of them
+// go to it); slab, 200 000: 11.7 / 9.8 / 9.5 / 10.1 / 10.5; CT head 5-field
+// plan, 1M: 36.1 / 33.4 / 33.5 / 33.3 / 34.1, 16M: 258.2 / 255.5 / 255.6 /
+// 256.0 / 255.9. Never for a run that says how it is to be divided into waves
+// (step or wave budgets, serial waves) or that tests its queues, and at most
+// half the in-flight batch, so that a small batch still runs as asked.
+static uint32_t drain_threshold(const gegs_run_opts &o, uint32_t batch)
+{
+    if (o.mode != GEGS_MODE_PERSISTENT || (o.flags & GEGS_RUN_SERIAL_WAVES) || o.step_budget || o.max_waves || o.queue_cap)
+        return 0u;
+    const uint32_t most = 4000u;
+    return most < batch / 2u ? most : batch / 2u;
+}
+
+static gegs_status ensure_drain(gegs_engine *e)
+{
+    const int grid = e->nsm * drain_blocks_per_sm(e->has_head);
+    if (e->drain_grid == grid) return GEGS_OK;
+    const size_t warps = (size_t)grid * (kDrainThreads / 32);
+    CK(realloc_dev(&e->d_drain_part, warps * GX_DT_N * GX_DRAIN_CAP), "drain stacks");
+    CK(realloc_dev(&e->d_drain_estate, warps * 3 * GX_DRAIN_CAP), "drain stacks");
+    e->drain_grid = grid;
+    e->ctx.drain_part = e->d_drain_part;
+    e->ctx.drain_estate = e->d_drain_estate;
+    e->ctx_gen++;
+    return GEGS_OK;
+}
+
 // Everything a run needs before its kernels: options resolved into the
 // context, queues sized, the scheduler state and the counters reset on the
 // engine's stream.
@@ -696,6 +755,7 @@ struct RunSetup {
     gegs_run_opts o;
     int grid, threads;
     uint32_t max_waves;
+    uint32_t drain_below;
 };
 
 static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t hist_end, const gegs_run_opts *opts,
@@ -727,6 +787,8 @@ static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t his
     }
     gegs_status st = ensure_queues(e, batch, o.queue_cap);
     if (st != GEGS_OK) return st;
+    const uint32_t drain_below = drain_threshold(o, batch);
+    if (drain_below) { st = ensure_drain(e); if (st != GEGS_OK) return st; }
     fill_queue_ctx(e);
 
     SchedState hs = {};
@@ -734,6 +796,7 @@ static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t his
     hs.end = hist_end;
     hs.batch = batch;
     hs.max_waves = max_waves;
+    hs.drain_below = drain_below;
     hs.refill_below = o.refill_below ? o.refill_below : (batch / 4u > 0u ? batch / 4u : 1u);
     CK(cudaMemcpyAsync(e->d_sched, &hs, sizeof hs, cudaMemcpyHostToDevice, e->stream), "sched H2D");
     CK(cudaMemsetAsync(e->d_qmeta, 0, sizeof(uint32_t) * 4 * GX_NQ, e->stream), "qmeta reset");
@@ -753,6 +816,7 @@ static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t his
     R.grid = grid;
     R.threads = threads;
     R.max_waves = max_waves;
+    R.drain_below = drain_below;
     return GEGS_OK;
 }
 
@@ -768,11 +832,17 @@ static gegs_status run_impl(gegs_engine *e, uint64_t hist_begin, uint64_t hist_e
     const int grid = R.grid, threads = R.threads;
     const uint32_t max_waves = R.max_waves;
     for (int k = 0; k < 16; k++) { e->last.stage_ms[k] = 0.0; e->last.stage_launches[k] = 0; }
-    if (o.mode == GEGS_MODE_PERSISTENT) {
+    if (o.mode == GEGS_MODE_PERSISTENT && hist_end - hist_begin <= R.drain_below) {
+        // the whole run goes to the drain kernel: no wave loop, so no graph
+        CK(cudaEventRecord(e->ev0, e->stream), "event");
+        k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
+        launch_drain(e->ctx, e->d_sched, e->has_head, e->drain_grid, e->stream);
+        k_drain_end<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
+        CK(cudaEventRecord(e->ev1, e->stream), "event");
+    } else if (o.mode == GEGS_MODE_PERSISTENT) {
         st = build_graph(e, grid, threads);
         if (st != GEGS_OK) return st;
         CK(cudaEventRecord(e->ev0, e->stream), "event");
-        k_plan<<<1, 1, 0, e->stream>>>(e->ctx, e->d_sched);
         CK(cudaGraphLaunch(e->gexec[e->slot], e->stream), "graph launch");
         CK(cudaEventRecord(e->ev1, e->stream), "event");
     } else if (o.mode == GEGS_MODE_TIMED) {
@@ -786,7 +856,7 @@ static gegs_status run_impl(gegs_engine *e, uint64_t hist_begin, uint64_t hist_e
         unsigned long long nl[16] = {0};
         for (uint32_t w = 0; w < max_waves; w++) {
             CK(cudaEventRecord(evs[30], e->stream), "event");
-            k_plan<<<1, 1, 0, e->stream>>>(e->ctx, e->d_sched);
+            k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
             CK(cudaEventRecord(evs[31], e->stream), "event");
             CK(cudaMemcpyAsync(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost, e->stream), "sched D2H");
             CK(cudaStreamSynchronize(e->stream), "timed sync");
@@ -845,7 +915,7 @@ static gegs_status run_impl(gegs_engine *e, uint64_t hist_begin, uint64_t hist_e
         uint32_t counts[GX_NQ];
         SchedState hsr;
         for (uint32_t w = 0; w < max_waves; w++) {
-            k_plan<<<1, 1, 0, e->stream>>>(e->ctx, e->d_sched);
+            k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
             CK(cudaMemcpyAsync(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost, e->stream), "sched D2H");
             CK(cudaStreamSynchronize(e->stream), "plain sync");
             if (!hsr.pending) break;
@@ -912,14 +982,22 @@ static gegs_status run_finish(gegs_engine *e)
     e->in_flight = false;
     CK(cudaStreamSynchronize(e->stream), "run sync");
     e->group.reset();
+    SchedState hsr;
+    CK(cudaMemcpy(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost), "sched D2H");
+    while (hsr.pending) {
+        // what the drain kernel's full stacks sent to the event queues: further waves
+        launch_wave_kernels(e, e->nsm * 2, 256);
+        k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
+        CK(cudaEventRecord(e->ev1, e->stream), "event");
+        CK(cudaMemcpyAsync(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost, e->stream), "sched D2H");
+        CK(cudaStreamSynchronize(e->stream), "run sync");
+    }
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e->ev0, e->ev1);
     uint32_t errbits = 0;
     unsigned long long stats[16];
-    SchedState hsr;
     CK(cudaMemcpy(&errbits, e->d_err, sizeof errbits, cudaMemcpyDeviceToHost), "err D2H");
     CK(cudaMemcpy(stats, e->d_stats, sizeof stats, cudaMemcpyDeviceToHost), "stats D2H");
-    CK(cudaMemcpy(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost), "sched D2H");
     CK(cudaMemcpy(e->last.queue_peak, e->d_qmeta + 3 * GX_NQ, sizeof(uint32_t) * GX_NQ, cudaMemcpyDeviceToHost),
        "queue peaks D2H");
     for (int q = 0; q < GX_NQ; q++) e->last.queue_cap[q] = e->qcap[q];
@@ -1009,7 +1087,7 @@ extern "C" gegs_status gegs_launch_group(gegs_engine *const *engines, int32_t n,
         cudaGraph_t g;
         CK(cudaGraphCreate(&g, 0), "graph create");
         for (int i = 0; i < n; i++) {
-            gegs_status st = add_wave_loop(engines[i], g, R[i].grid, R[i].threads, true);
+            gegs_status st = add_wave_loop(engines[i], g, R[i].grid, R[i].threads);
             if (st != GEGS_OK) { cudaGraphDestroy(g); if (engines[i] != e) e->err = engines[i]->err; return st; }
         }
         grp = std::make_shared<GroupRun>();
@@ -1340,7 +1418,7 @@ extern "C" gegs_status gegs_run_noalloc(gegs_engine *e, uint64_t hist_begin, uin
         // gated planner injects nothing and counts no wave, and the kernels of
         // the remaining waves find empty queues
         for (int k = 0; k < 8 && w < hs.max_waves; k++, w++) {
-            k_plan_gated<<<1, 1, 0, s>>>(c, sched);
+            k_plan_gated<<<1, 32, 0, s>>>(c, sched);
             k_source<<<grid, threads, 0, s>>>(c, sched);
             k_photon_jaws<<<grid, threads, 0, s>>>(c);
             k_photon_mlc<<<grid, threads, 0, s>>>(c);
@@ -1426,6 +1504,8 @@ extern "C" gegs_status gegs_backward(gegs_engine *e, uint64_t hist_begin, uint64
     e->ctx.q = after.q;                          // queue buffers may have been re-sized by the run
     e->ctx.photon_budget = after.photon_budget;
     e->ctx.electron_budget = after.electron_budget;
+    e->ctx.drain_part = after.drain_part;
+    e->ctx.drain_estate = after.drain_estate;
     if (fresh) e->ctx_gen++;
     if (st != GEGS_OK) return st;
     std::vector<double> g((size_t)n * GX_GRAD_COPIES);

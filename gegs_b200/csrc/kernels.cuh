@@ -31,13 +31,14 @@
 // particle that stops making progress)
 #define GX_STEP_BUDGET 4000000u
 
-__device__ __forceinline__ void consumer_done(const DevCtx &C, int q, int q2 = -1, uint32_t *finished = nullptr)
+// The last of the `blocks` that took part in draining a queue resets it.
+__device__ __forceinline__ void consumer_done(const DevCtx &C, uint32_t blocks, int q, int q2 = -1, uint32_t *finished = nullptr)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         uint32_t prev = atomicAdd(&C.q.done[q], 1u);
-        if (prev == gridDim.x - 1) {
+        if (prev == blocks - 1) {
             if (C.q.peak) {
                 atomicMax(&C.q.peak[q], *((volatile uint32_t *)&C.q.count[q]));
                 if (q2 >= 0) atomicMax(&C.q.peak[q2], *((volatile uint32_t *)&C.q.count[q2]));
@@ -105,8 +106,8 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
 {
     const uint32_t lane = threadIdx.x & 31u;
     unsigned need = __ballot_sync(0xffffffffu, !active);
-    if (need == 0u || exhausted) return active;
     uint32_t cnt = __popc(need);
+    if (cnt == 0u || exhausted) return active;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&C.q.head[hq], cnt);
     base = __shfl_sync(0xffffffffu, base, 0);
@@ -188,14 +189,25 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
     // the photon jaws kernel's second form (NEAR): the long tracks, beside the electron phase
     constexpr bool LONG = !ELEC && G == GX_GEOM_JAWS && NEAR;
     constexpr int tl = LONG ? TL_PLONG : NEAR ? TL_ENEAR : (ELEC ? TL_ELECTRON : TL_PHOTON) + cls;
-    timeline_mark(C, tl, false);
-    if (!ELEC) stage_photon_tables(C);
     const uint32_t par = *C.wave & 1u;
     const int qc_in = LONG ? GX_Q_PLONG : NEAR ? GX_Q_ENEAR + cls : base + 2 * cls + (int)par;
     const int qc_out = base + 2 * cls + (int)(par ^ 1u);
     const int hq = FIRST ? Q : qc_in;
     const uint32_t n_cont = queue_len(C, qc_in);
     const uint32_t n = n_cont + (FIRST ? queue_len(C, Q) : 0u);
+    // the last kernel of each photon branch but the jaws (MLC, phantom), and of
+    // each electron branch (jaws and MLC near-boundary passes, phantom)
+    uint32_t *fin = (!ELEC && G != GX_GEOM_JAWS) ? C.photon_done
+                  : (ELEC && (NEAR || G == GX_GEOM_PHANTOM)) ? C.electron_done : nullptr;
+    // Only the blocks that have work take part: a launch of 888 blocks that found
+    // nothing and counted themselves off took 10 to 25 us, now 3 to 4.
+    const uint32_t blocks = min(gridDim.x, n / blockDim.x + (n % blockDim.x ? 1u : 0u));
+    if (blockIdx.x >= blocks) {
+        if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0 && fin) atomicAdd(fin, 1u);
+        return;
+    }
+    timeline_mark(C, tl, false);
+    if (!ELEC) stage_photon_tables(C);
     // per-class budgets (measured on the CT 5-field plan): photons take 8x their
     // budget in the jaws and MLC, where a few bounce along leaf gaps for many
     // steps; electrons take 2x theirs in the phantom
@@ -262,12 +274,8 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
     block_stat_add(C, GX_NSTAGE + (ELEC ? 1 : 0), steps);
     // steps in the jaws and the MLC (slots 12-15; the phantom's are the rest)
     if (cls < 2) block_stat_add(C, GX_NSTAGE + 2 + 2 * (ELEC ? 1 : 0) + cls, steps);
-    // the last kernel of each photon branch but the jaws (MLC, phantom), and of
-    // each electron branch (jaws and MLC near-boundary passes, phantom)
-    uint32_t *fin = (!ELEC && G != GX_GEOM_JAWS) ? C.photon_done
-                  : (ELEC && (NEAR || G == GX_GEOM_PHANTOM)) ? C.electron_done : nullptr;
-    if (FIRST) consumer_done(C, Q, qc_in, fin);
-    else consumer_done(C, qc_in, -1, fin);
+    if (FIRST) consumer_done(C, blocks, Q, qc_in, fin);
+    else consumer_done(C, blocks, qc_in, -1, fin);
     timeline_mark(C, tl, true);
 }
 
@@ -320,8 +328,10 @@ template <int Q>
 __global__ void __launch_bounds__(256) k_interact(const __grid_constant__ DevCtx C)
 {
     constexpr int tl = Q < ST_ELECTRON ? TL_PINT + (Q - ST_COMPTON) : TL_EINT + (Q - ST_MOLLER);
-    timeline_mark(C, tl, false);
     const uint32_t n = queue_len(C, Q);
+    const uint32_t blocks = min(gridDim.x, n / blockDim.x + (n % blockDim.x ? 1u : 0u));
+    if (blockIdx.x >= blocks) return;
+    timeline_mark(C, tl, false);
     unsigned long long taken = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         Part p = load_part(&C.q.buf[Q][i]);
@@ -333,7 +343,7 @@ __global__ void __launch_bounds__(256) k_interact(const __grid_constant__ DevCtx
         taken += counted<Q>(p);
     }
     block_stat_add(C, Q, taken);
-    consumer_done(C, Q);
+    consumer_done(C, blocks, Q);
     timeline_mark(C, tl, true);
 }
 
@@ -370,41 +380,51 @@ __global__ void __launch_bounds__(256) k_plain(const __grid_constant__ DevCtx C)
     block_stat_add(C, Q, taken);
     if (Q == ST_PHOTON) block_stat_add(C, GX_NSTAGE, steps);
     if (Q == ST_ELECTRON) block_stat_add(C, GX_NSTAGE + 1, steps);
-    consumer_done(C, Q);
+    consumer_done(C, gridDim.x, Q);
 }
 
 // ---- planner: next wave's injection and the loop condition -----------------
+// One warp: a lane per queue reads its count (one thread reading the 25 one
+// after another took most of the 9 to 12 us between two waves).
 __device__ __forceinline__ uint32_t plan_wave(const DevCtx &C, SchedState *st)
 {
-    uint32_t inflight = 0;
-    for (int q = 0; q < GX_NQ; q++) inflight += *((volatile uint32_t *)&C.q.count[q]);
-    uint32_t main_q = *((volatile uint32_t *)&C.q.count[ST_PHOTON]) + *((volatile uint32_t *)&C.q.count[ST_ELECTRON]);
-    for (int q = GX_Q_PCONT; q < GX_NQ; q++) main_q += *((volatile uint32_t *)&C.q.count[q]);
-    // once the population falls below `refill_below`, top it up to `batch`
-    unsigned long long remaining = st->end - st->next;
-    unsigned long long inject = 0;
-    if (remaining > 0 && main_q < st->refill_below && main_q < st->batch) {
-        inject = st->batch - main_q;
-        if (inject > remaining) inject = remaining;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t count = lane < GX_NQ ? *((volatile uint32_t *)&C.q.count[lane]) : 0u;
+    const bool is_main = lane == ST_PHOTON || lane == ST_ELECTRON || lane >= GX_Q_PCONT;
+    const uint32_t inflight = __reduce_add_sync(0xffffffffu, count);
+    const uint32_t main_q = __reduce_add_sync(0xffffffffu, is_main ? count : 0u);
+    const uint32_t side_q = __reduce_add_sync(0xffffffffu, lane >= GX_Q_ENEAR ? count : 0u);   // empty between waves
+    uint32_t pending = 0;
+    if (lane == 0) {
+        const uint32_t err = *((volatile uint32_t *)C.err);
+        const unsigned long long remaining = st->end - st->next;
+        unsigned long long inject = 0;
+        // what is left is small: the drain kernel takes all of it, and the waves end
+        st->drain = main_q + remaining > 0 && main_q == inflight && side_q == 0u && main_q + remaining <= st->drain_below && err == 0u;
+        // once the population falls below `refill_below`, top it up to `batch`
+        if (!st->drain && remaining > 0 && main_q < st->refill_below && main_q < st->batch) {
+            inject = st->batch - main_q;
+            if (inject > remaining) inject = remaining;
+        }
+        st->h0 = st->next;
+        st->h1 = st->next + inject;
+        st->next += inject;
+        // The tail of a run: every history injected and few particles left. The
+        // waves are then short and their fixed cost (launches, the step chains of
+        // single particles) dominates; larger step budgets take fewer of them.
+        st->budget_shift = (st->next >= st->end && main_q < st->batch / GX_TAIL_DIV) ? GX_TAIL_SHIFT : 0u;
+        st->waves++;
+        st->photon_done = 0u;
+        st->electron_done = 0u;
+        pending = (inflight > 0 || inject > 0 || st->next < st->end) ? 1u : 0u;
+        if (pending && st->waves >= st->max_waves) {
+            atomicOr(C.err, GX_ERR_STEP_BUDGET);
+            pending = 0;
+        }
+        if ((err & GX_ERR_QUEUE_FULL) || st->drain) pending = 0;
+        st->pending = pending;
     }
-    st->h0 = st->next;
-    st->h1 = st->next + inject;
-    st->next += inject;
-    // The tail of a run: every history injected and few particles left. The
-    // waves are then short and their fixed cost (launches, the step chains of
-    // single particles) dominates; larger step budgets take fewer of them.
-    st->budget_shift = (st->next >= st->end && main_q < st->batch / GX_TAIL_DIV) ? GX_TAIL_SHIFT : 0u;
-    st->waves++;
-    st->photon_done = 0u;
-    st->electron_done = 0u;
-    uint32_t pending = (inflight > 0 || inject > 0 || st->next < st->end) ? 1u : 0u;
-    if (pending && st->waves >= st->max_waves) {
-        atomicOr(C.err, GX_ERR_STEP_BUDGET);
-        pending = 0;
-    }
-    if (*((volatile uint32_t *)C.err) & GX_ERR_QUEUE_FULL) pending = 0;
-    st->pending = pending;
-    return pending;
+    return __shfl_sync(0xffffffffu, pending, 0);
 }
 
 __global__ void k_plan(const __grid_constant__ DevCtx C, SchedState *st)
@@ -418,17 +438,41 @@ __global__ void k_plan(const __grid_constant__ DevCtx C, SchedState *st)
 // histories are those of the graph form, which stops at that plan.
 __global__ void k_plan_gated(const __grid_constant__ DevCtx C, SchedState *st)
 {
-    if (st->pending == 0u) {
-        st->h0 = st->h1 = st->next;
+    const uint32_t pending = *((volatile uint32_t *)&st->pending);
+    __syncwarp();
+    if (pending == 0u) {
+        if (threadIdx.x == 0) st->h0 = st->h1 = st->next;
         return;
     }
+    plan_wave(C, st);
+}
+
+// Ends a run: if the drain kernel ran, the queues it emptied are reset (their
+// peaks recorded) and the plan says whether it left anything (`pending`).
+__global__ void k_drain_end(const __grid_constant__ DevCtx C, SchedState *st)
+{
+    const uint32_t drained = *((volatile uint32_t *)&st->drain);
+    __syncwarp();
+    if (drained == 0u) return;
+    if (threadIdx.x < 8u) {
+        const int k = (int)threadIdx.x, q = k < 6 ? GX_Q_PCONT + 2 * k + (int)(*C.wave & 1u) : k == 6 ? ST_PHOTON : ST_ELECTRON;
+        if (C.q.peak && C.q.count[q] > C.q.peak[q]) C.q.peak[q] = C.q.count[q];
+        C.q.count[q] = 0;
+        C.q.head[q] = 0;
+    }
+    if (threadIdx.x == 0) {
+        st->next = st->end;
+        st->drain_below = 0u;
+        st->drain_hist = 0ull;
+    }
+    __syncwarp();
     plan_wave(C, st);
 }
 
 __global__ void k_plan_cond(const __grid_constant__ DevCtx C, SchedState *st, cudaGraphConditionalHandle handle)
 {
     uint32_t pending = plan_wave(C, st);
-    cudaGraphSetConditional(handle, pending);
+    if (threadIdx.x == 0) cudaGraphSetConditional(handle, pending);
 }
 
 // ---- geometry probe (gegs_probe_geometry) ----------------------------------

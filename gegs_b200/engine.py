@@ -255,7 +255,7 @@ class Engine:
 
     TIMELINE_KERNELS = ["source", "photon_jaws", "photon_mlc", "photon", "compton", "photo", "rayleigh", "pair",
                         "electron_jaws", "electron_mlc", "electron", "moller", "brems", "bhabha", "annih",
-                        "electron_near", "photon_jaws_long"]
+                        "electron_near", "photon_jaws_long", "drain"]
     TIMELINE_SLOTS = 32
 
     def set_timeline(self, max_waves: int):

@@ -81,7 +81,8 @@ def timeline_summary(eng, args, dims):
     e = np.where(ran, (tl[:, :, 1] - t0) / 1e6, np.nan)
     names = eng.TIMELINE_KERNELS
     groups = {"source": [0], "photon transport": [1, 2, 3], "photon interactions": [4, 5, 6, 7],
-              "electron transport": [8, 9, 10, 15], "long jaws-photon tracks": [16], "electron interactions": [11, 12, 13, 14]}
+              "electron transport": [8, 9, 10, 15], "long jaws-photon tracks": [16], "electron interactions": [11, 12, 13, 14],
+              "drain": [17]}
     import warnings
     with np.errstate(all="ignore"), warnings.catch_warnings():
         warnings.simplefilter("ignore", RuntimeWarning)          # waves in which a group did not run

@@ -270,8 +270,9 @@ gegs_status gegs_tally_device_ptr(gegs_engine *e, void **out);
  * 4-7 Compton, photo, Rayleigh, pair; 8-10 electron jaws, MLC, phantom;
  * 11-14 Moller, brems, Bhabha, annihilation; 15 the near-boundary passes of
  * the jaws and MLC electrons (together); 16 the long jaws-photon tracks run
- * beside the electron phase; 17-31 unused. A kernel that did not
- * run in a wave keeps start = UINT64_MAX, end = 0. 0 turns it off. */
+ * beside the electron phase; 17 the drain kernel (in the wave after the last);
+ * 18-31 unused. A kernel that did not run, or found nothing to do, in a wave
+ * keeps start = UINT64_MAX, end = 0. 0 turns it off. */
 gegs_status gegs_set_timeline(gegs_engine *e, uint32_t max_waves);
 gegs_status gegs_get_timeline(gegs_engine *e, uint64_t *out, uint32_t max_waves);
 

@@ -1,0 +1,77 @@
+"""The drain kernel (small runs, and the end of every other one) against the
+oracle, bit for bit, and against the waves in what it counts. Its edges: fewer
+histories than warps, one more than a warp or than all warps' lanes hold, runs
+just below and above the population at which it takes over, and a gradient
+replay through it."""
+import numpy as np
+import pytest
+
+from gegs_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+WAVES = dict(photon_budget=32, electron_budget=4)      # a run that names its step budgets is run in waves
+
+
+def _load(engine, job):
+    sh = job.scene()
+    engine.set_physics(job.physics)
+    engine.set_scene(sh)
+    return sh
+
+
+@pytest.mark.parametrize("histories", [1, 31, 33, 3553, 4000, 4001, 20000, 70000])
+@pytest.mark.parametrize("scene", ["slab", "head"])
+def test_drain_is_the_oracle_and_counts_like_the_waves(engine, oracle, scene, histories):
+    if scene == "slab":
+        job = W.config2(histories=histories, nphsp=20000, n=30)
+    else:
+        job = W.config3(histories=histories, nphsp=20000, dims=(48, 40, 24), angles=(0.0, 72.0, 200.0))
+    sh = _load(engine, job)
+    drained = engine.run(0, histories)
+    a = engine.tally()
+    engine.reset_tally()
+    waves = engine.run(0, histories, **WAVES)
+    b = engine.tally()
+    ref, _ = oracle.run(job.physics, sh, 0, histories)
+    np.testing.assert_array_equal(a, ref)
+    np.testing.assert_array_equal(b, ref)
+    assert drained["error_bits"] == waves["error_bits"] == 0
+    if histories <= 4000:
+        assert drained["waves"] == 2                   # the plan before the drain kernel and the one after it
+    for key in ("processed", "photon_steps", "electron_steps", "photon_steps_class", "electron_steps_class"):
+        assert drained[key] == waves[key], key
+
+
+def test_a_history_range_and_several_runs_on_one_engine(engine, oracle):
+    """Drained runs of part of a plan, one after another and beside a run in
+    waves, add up to the plan's tally."""
+    job = W.config3(histories=9000, nphsp=5000, dims=(40, 40, 20))
+    sh = _load(engine, job)
+    for lo, hi, kw in ((0, 7, {}), (7, 3000, {}), (3000, 6001, WAVES), (6001, 9000, dict(batch=512))):
+        engine.run(lo, hi, **kw)
+    ref, _ = oracle.run(job.physics, sh, 0, 9000)
+    np.testing.assert_array_equal(engine.tally(), ref)
+
+
+def test_a_gradient_replay_drains_and_leaves_the_forward_run_as_it_was(engine):
+    """The first run of an engine being a replay, then a forward run, then a
+    replay again: the same gradient (double sums in any order) and the tally."""
+    from gegs_b200.engine import Engine
+    job = W.config4(histories=5000, nphsp=5000, dims=(40, 40, 20), nb=6, bixel=1.5)
+    sh = _load(engine, job)
+    g = np.random.default_rng(3).normal(size=sh.nvox)
+    engine.run(0, 5000, **WAVES)
+    want = engine.tally()
+    fresh = Engine(0)
+    fresh.set_physics(job.physics)
+    fresh.set_scene(job.scene())
+    first = fresh.backward(0, 5000, g)
+    fresh.run(0, 5000)
+    np.testing.assert_array_equal(fresh.tally(), want)
+    again = fresh.backward(0, 5000, g)
+    fresh.close()
+    # sums of up to 1e6 products of both signs in double, in two orders: each is within 1e6 * 2^-53 = 1e-10
+    # of the sum of its terms' sizes, some ten times the largest sum
+    assert np.abs(first).max() > 0
+    np.testing.assert_allclose(again, first, rtol=0, atol=1e-9 * np.abs(first).max())
