@@ -96,6 +96,16 @@ __global__ void k_source(const __grid_constant__ DevCtx C, const SchedState *st)
     }
 }
 
+// A warp goes back to its queue once this many of its lanes are idle. A refill
+// runs at the speed of its loads (the claim, the record, the region: one after
+// another some 2000 cycles) with only the new lanes active, so a refill per
+// lane that ends holds the others up at nearly every step. Slab, 5M histories:
+// 85.1 ms at 1, 78.1 at 4, 75.5 at 8, 75.8 at 16; CT head 5-field plan, 16M:
+// 275.8, 263.4, 258.6, 256.1.
+#ifndef GX_REFILL_IDLE
+#define GX_REFILL_IDLE 12u
+#endif
+
 // ---- persistent consumers with warp regeneration ---------------------------
 // A consumer drains the continuation queue of the previous wave (indices
 // [0, n_cont)) and then its stage queue ([n_cont, n)) through one shared head
@@ -107,7 +117,7 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
     const uint32_t lane = threadIdx.x & 31u;
     unsigned need = __ballot_sync(0xffffffffu, !active);
     uint32_t cnt = __popc(need);
-    if (cnt == 0u || exhausted) return active;
+    if (cnt == 0u || exhausted || cnt < GX_REFILL_IDLE) return active;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&C.q.head[hq], cnt);
     base = __shfl_sync(0xffffffffu, base, 0);
@@ -137,9 +147,10 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
 #ifndef GX_PHOTON_MIN_BLOCKS
 #define GX_PHOTON_MIN_BLOCKS 4
 #endif
-// the near-boundary electron passes: 80 registers
+// the near-boundary electron passes: 128 registers (1.2 % faster than 80 on the
+// CT head 5-field plan, 16M histories, 1.6 % at 1M)
 #ifndef GX_ELECTRON_MIN_BLOCKS
-#define GX_ELECTRON_MIN_BLOCKS 3
+#define GX_ELECTRON_MIN_BLOCKS 2
 #endif
 // the phantom electrons: 64 registers. Its step spills some 280 bytes there
 // against about 100 at 80 registers, yet the fourth block per SM hides more of
@@ -155,10 +166,11 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
 #ifndef GX_PMLC_MIN_BLOCKS
 #define GX_PMLC_MIN_BLOCKS 3
 #endif
-// the first pass of the jaws and MLC electrons, without howfar: 48 registers
-// (5 blocks), 0.3 % faster than 64
+// the first pass of the jaws and MLC electrons, without howfar: 80 registers
+// (3 blocks; CT head 5-field plan, 16M histories: 1.8 % faster than 48, with
+// fewer warps waiting for instructions, and 0.3 % than 64)
 #ifndef GX_EHEAD_MIN_BLOCKS
-#define GX_EHEAD_MIN_BLOCKS 5
+#define GX_EHEAD_MIN_BLOCKS 3
 #endif
 
 // Transport consumer for photons (ELEC false) or electrons of one geometry
