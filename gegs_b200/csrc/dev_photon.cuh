@@ -204,28 +204,27 @@ enum : int {
 };
 
 // One iteration of the PHOTON loop. `vx` is the record of the photon's region,
-// kept from one step to the next. Every way out that scores or queues shares
+// kept from one step to the next, `gle` the logarithm of its energy. Every way out that scores or queues shares
 // one place, and the queueing itself is the caller's, so that the code is small.
 // SH: the {gmfp, cohe} table is staged in shared memory (stage_photon_tables).
 template <int G = GX_GEOM_ALL, bool SH = false>
-static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, int &out)
+static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, float gle, int &out)
 {
     const gegs_physics *P = C.P;
     const unsigned med = vx.med;
     int idisc = 0;
-    bool absorbed = p.e <= pcut_of(C, vx);
-    float dpmfp = 0.0f, cohfac = 0.0f, gle = 0.0f;
+    const float4 m0 = med == GX_VACUUM ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : __ldg(&C.mtab[med]);
+    bool absorbed = p.e <= m0.z;
+    float dpmfp = 0.0f, cohfac = 0.0f;
     int lgle = 0;
     if (!absorbed) {
         if (p.wt <= 0.0f) return STEP_DONE;
         float r1 = U(C, r);
         dpmfp = -gx_log(r1);
-        gle = gx_log(p.e);
         float tstep, gmfp_val = 0.0f;
         if (med == GX_VACUUM) tstep = GX_VACUUM_STEP;
         else {
-            float2 ge = __ldg(reinterpret_cast<const float2 *>(P->ge[med]));
-            lgle = (int)(ge.x + ge.y * gle);
+            lgle = (int)(m0.x + m0.y * gle);
             const float4 t = SH && C.stage_tables ? g_smem_ptab[med * GX_MXGE + lgle] : __ldg(&C.ptab[med * GX_MXGE + lgle]);
             float gmfpr0 = t.x + t.y * gle;
             gmfp_val = gmfpr0 / vx.rhof;
@@ -248,7 +247,7 @@ static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, int
         p.z = p.z + p.w * tstep;
         if (med != GX_VACUUM) dpmfp = fmaxf_(0.0f, dpmfp - tstep / gmfp_val);
         p.region = new_region;
-        absorbed = p.e <= pcut_of(C, vx) || idisc < 0;
+        absorbed = idisc < 0 || (vx.med != med && p.e <= pcut_of(C, vx));   // above its own medium's cut already
     }
     if (absorbed) { escore(C, p, p.region, p.e * p.wt); return STEP_DONE; }
     if ((vx.med != med) || (vx.med == GX_VACUUM) || gx_ge(dpmfp, GX_EPSGMFP)) return STEP_ON;

@@ -127,6 +127,7 @@ __device__ __noinline__ void drain_transport()
     Rng r;
     EState s;
     Vox vx;
+    float gle = 0.0f;
     bool active = false;
     uint32_t steps = 0, taken = 0;
     for (;;) {
@@ -141,6 +142,7 @@ __device__ __noinline__ void drain_transport()
                 p = load_part(slot_part(C, T, i));
                 rng_load(r, p);
                 vx = C.reg[p.region];
+                if (!ELEC) gle = gx_log(p.e);
                 active = true;
                 if (p.status == kGoesOn) {
                     if (ELEC) unpack_estate(*slot_estate(C, T, i), s);
@@ -169,7 +171,7 @@ __device__ __noinline__ void drain_transport()
             else {
                 steps++;
                 rng_window(C, r);
-                const int code = ELEC ? electron_step<G>(C, p, r, s, vx, out) : photon_step<G>(C, p, r, vx, out);
+                const int code = ELEC ? electron_step<G>(C, p, r, s, vx, out) : photon_step<G>(C, p, r, vx, gle, out);
                 if (code == STEP_DONE) active = false;
                 else if (code == STEP_QUEUE) { to = stack_of(out, p); moved = false; }
             }

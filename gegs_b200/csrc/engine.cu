@@ -62,6 +62,7 @@ struct gegs_engine {
 
     gegs_physics *d_P = nullptr;
     float4 *d_ptab = nullptr;          // {gmfp, cohe} per (medium, energy bin) (DevCtx::ptab, kTablePad entries in)
+    float4 *d_mtab = nullptr;          // per medium (DevCtx::mtab)
     float4 *d_etab = nullptr;          // electron tables per bin (DevCtx::etab, kTablePad entries in)
     Vox *d_reg = nullptr;
     float *d_xb = nullptr, *d_yb = nullptr, *d_zb = nullptr;
@@ -244,7 +245,7 @@ void gegs_destroy(gegs_engine *e)
     if (e->stream) cudaStreamSynchronize(e->stream);
     for (int k = 0; k < 2; k++) if (e->gexec[k]) cudaGraphExecDestroy(e->gexec[k]);
     cudaFree(e->d_blw); cudaFree(e->d_gvm); cudaFree(e->d_grad);
-    cudaFree(e->d_P); cudaFree(e->d_ptab); cudaFree(e->d_etab); cudaFree(e->d_reg); cudaFree(e->d_xb); cudaFree(e->d_yb); cudaFree(e->d_zb);
+    cudaFree(e->d_P); cudaFree(e->d_ptab); cudaFree(e->d_etab); cudaFree(e->d_mtab); cudaFree(e->d_reg); cudaFree(e->d_xb); cudaFree(e->d_yb); cudaFree(e->d_zb);
     cudaFree(e->d_timeline);
     cudaFree(e->d_fields); cudaFree(e->d_cross); cudaFree(e->d_jaw_lines); cudaFree(e->d_phsp); cudaFree(e->d_tally);
     cudaFree(e->d_err); cudaFree(e->d_stats); cudaFree(e->d_sched); cudaFree(e->d_qmeta);
@@ -329,6 +330,11 @@ gegs_status gegs_set_physics(gegs_engine *e, const gegs_physics *P)
     }
     CK(cudaMemcpyAsync(e->d_etab + kTablePad, etab.data(), etab.size() * sizeof(float4), cudaMemcpyHostToDevice, e->stream),
        "tables H2D");
+    std::vector<float4> mtab(GEGS_MXMED);
+    for (int m = 0; m < GEGS_MXMED; m++) mtab[m] = make_float4(P->ge[m][0], P->ge[m][1], P->ap[m], P->ae[m]);
+    if (!e->d_mtab) CK(cudaMalloc(&e->d_mtab, mtab.size() * sizeof(float4)), "medium tables");
+    CK(cudaMemcpyAsync(e->d_mtab, mtab.data(), mtab.size() * sizeof(float4), cudaMemcpyHostToDevice, e->stream), "tables H2D");
+    e->ctx.mtab = e->d_mtab;
     CK(cudaStreamSynchronize(e->stream), "physics sync");
     e->have_physics = true;
     e->ctx.P = e->d_P;

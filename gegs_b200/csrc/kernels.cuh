@@ -112,7 +112,7 @@ __global__ void k_source(const __grid_constant__ DevCtx C, const SchedState *st)
 // counter `hq`; idle lanes of a warp are refilled with one atomic.
 template <int Q, bool ELEC>
 __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont, uint32_t n, int qc, bool &exhausted,
-                                       bool active, Part &p, Rng &r, EState &s, Vox &vx, unsigned long long &taken)
+                                       bool active, Part &p, Rng &r, EState &s, Vox &vx, float &gle, unsigned long long &taken)
 {
     const uint32_t lane = threadIdx.x & 31u;
     unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -129,6 +129,7 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
             p = load_part(cont ? &C.q.buf[qc][idx] : &C.q.buf[Q][idx - n_cont]);
             rng_load(r, p);
             vx = C.reg[p.region];
+            if (!ELEC) gle = gx_log(p.e);
             if (cont) {
                 if (ELEC) unpack_estate(C.q.estate[qc - GX_Q_ECONT][idx], s);
             } else {
@@ -245,12 +246,13 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
     Rng r;
     EState s;
     Vox vx;
+    float gle = 0.0f;
     bool active = false, exhausted = false;
     unsigned long long taken = 0, steps = 0;
     uint32_t nst = 0;
     for (;;) {
         const bool was = active;
-        active = refill<Q, ELEC>(C, hq, n_cont, n, qc_in, exhausted, active, p, r, s, vx, taken);
+        active = refill<Q, ELEC>(C, hq, n_cont, n, qc_in, exhausted, active, p, r, s, vx, gle, taken);
         if (active && !was) nst = 0;
         if (!__any_sync(0xffffffffu, active)) break;
         if (active) {
@@ -261,7 +263,7 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
                 rng_window(C, r);
                 const uint32_t ctr0 = r.ctr;
                 const EState s0 = s;
-                const int code = ELEC ? electron_step<G, DEFER, ELEC && NEAR>(C, p, r, s, vx, tq) : photon_step<G, true>(C, p, r, vx, tq);
+                const int code = ELEC ? electron_step<G, DEFER, ELEC && NEAR>(C, p, r, s, vx, tq) : photon_step<G, true>(C, p, r, vx, gle, tq);
                 if (code == STEP_DONE) active = false;
                 else if ((DEFER && code == STEP_NEAR) || (ELEC && NEAR && code == STEP_FAR)) {
                     // needs howfar (to the near-boundary pass) or, in that pass, does
@@ -377,10 +379,11 @@ __global__ void __launch_bounds__(256) k_plain(const __grid_constant__ DevCtx C)
             EState s;
             estate_init(s);
             Vox vx = C.reg[p.region];
+            const float gle = gx_log(p.e);
             uint32_t nst = 0;
             int code, out = 0;
             do {
-                code = Q == ST_PHOTON ? photon_step(C, p, r, vx, out) : electron_step(C, p, r, s, vx, out);
+                code = Q == ST_PHOTON ? photon_step(C, p, r, vx, gle, out) : electron_step(C, p, r, s, vx, out);
                 steps++;
                 if (++nst > GX_STEP_BUDGET) { atomicOr(C.err, GX_ERR_STEP_BUDGET); break; }
             } while (code == STEP_ON);
