@@ -317,6 +317,14 @@ __device__ __forceinline__ float rng_uniform(const DevCtx &C, Rng &r)
     return __uint2float_rn((x >> 8) + 1u) * 5.9604644775390625e-08f;
 }
 
+// The next number of another thread's stream, from its window.
+__device__ __forceinline__ float rng_uniform_of(Rng &r, uint32_t owner)
+{
+    const uint32_t x = g_rng_words[(r.ctr & 7u) * GX_MAX_THREADS + owner];
+    r.ctr++;
+    return __uint2float_rn((x >> 8) + 1u) * 5.9604644775390625e-08f;
+}
+
 // child stream for a particle created by an interaction
 __device__ __forceinline__ void rng_spawn(const DevCtx &C, Rng &parent, Part &child)
 {
@@ -451,6 +459,17 @@ __device__ __forceinline__ void store_part(Part *dst, const Part &p)
     const uint4 *s = reinterpret_cast<const uint4 *>(&p);
     uint4 *d = reinterpret_cast<uint4 *>(dst);
     d[0] = s[0]; d[1] = s[1]; d[2] = s[2]; d[3] = s[3];
+}
+
+// Lane `src`'s particle on every lane of the warp.
+__device__ __forceinline__ Part part_of(const Part &p, int src)
+{
+    Part q;
+    const uint32_t *s = reinterpret_cast<const uint32_t *>(&p);
+    uint32_t *d = reinterpret_cast<uint32_t *>(&q);
+#pragma unroll
+    for (int k = 0; k < 16; k++) d[k] = __shfl_sync(0xffffffffu, s[k], src);
+    return q;
 }
 
 __device__ __forceinline__ Part load_part(const Part *src)

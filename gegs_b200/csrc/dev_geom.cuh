@@ -184,19 +184,42 @@ static __device__ __noinline__ int point_in_polygon(float px, float py, const fl
     return odd;
 }
 
+// The warp's way with one particle: every lane holds the same point (and ray)
+// and takes one edge, so that a polygon costs one edge's time instead of the
+// loop's. All 32 lanes call it; n is at most 30.
+__device__ __forceinline__ int point_in_polygon_warp(float px, float py, const float2 *poly, int n)
+{
+    const int i = (int)(threadIdx.x & 31u);
+    bool left = false;
+    if (i < n) {
+        const float2 a = ld2(&poly[i]), b = ld2(&poly[i ? i - 1 : n - 1]);
+        if ((a.y < py) != (b.y < py) && (a.y >= py || b.y >= py) && (a.x <= px || b.x <= px))
+            left = a.x + (py - a.y) / (b.y - a.y) * (b.x - a.x) < px;
+    }
+    return __popc(__ballot_sync(0xffffffffu, left)) & 1;
+}
+
+template <bool WARP>
+__device__ __forceinline__ int in_polygon(float px, float py, const float2 *poly, int n)
+{
+    return WARP ? point_in_polygon_warp(px, py, poly, n) : point_in_polygon(px, py, poly, n);
+}
+
 __device__ __forceinline__ const float2 *endnode_of(const DevCtx &C, int field, int leaf)
 {
     return reinterpret_cast<const float2 *>(&C.fields[field].endnode[leaf][0][0]);
 }
 
+template <bool WARP = false>
 static __device__ int point_in_leaf(float2 p, const float2 *endn)
 {
     int bank = 0;
-    if (point_in_polygon(p.x, p.y, endn, 17)) bank = 1;
-    else if (point_in_polygon(p.x, p.y, endn + 17, 17)) bank = 2;
+    if (in_polygon<WARP>(p.x, p.y, endn, 17)) bank = 1;
+    else if (in_polygon<WARP>(p.x, p.y, endn + 17, 17)) bank = 2;
     return bank;
 }
 
+template <bool WARP = false>
 static __device__ __noinline__ int index_of_leaf(const DevCtx &C, float2 p)
 {
     int i = GX_OUTMLC, index = GX_OUTMLC;
@@ -218,9 +241,9 @@ static __device__ __noinline__ int index_of_leaf(const DevCtx &C, float2 p)
     else if (x <= C.mlc_x_end)
         i = 58;
     if (i >= 0) {
-        if (point_in_polygon(p.x, p.y, C.crossXZ + i * 16, 14)) index = i;
+        if (in_polygon<WARP>(p.x, p.y, C.crossXZ + i * 16, 14)) index = i;
         else if (i < 59) {
-            if (point_in_polygon(p.x, p.y, C.crossXZ + (i + 1) * 16, 14)) index = i + 1;
+            if (in_polygon<WARP>(p.x, p.y, C.crossXZ + (i + 1) * 16, 14)) index = i + 1;
             else index = -(i + 1);
         } else index = GX_OUTMLC;
     }
@@ -284,19 +307,48 @@ __device__ __forceinline__ float ray_intersect_polygon(float2 p0, float2 v, cons
     return minDist;
 }
 
+// The same by the warp: each lane decides its edge as the loop would.
+__device__ __forceinline__ float ray_intersect_polygon_warp(float2 p0, float2 v, const float2 *poly, int n, int &inside)
+{
+    const int i = (int)(threadIdx.x & 31u);
+    float dist = GX_INFI_DIST + 1;
+    bool hit = false;
+    if (i < n) {
+        float num, den, dn;
+        ray_edge(p0, v, ld2(&poly[i]), ld2(&poly[i + 1 < n ? i + 1 : 0]), num, den, dn);
+        if (den != 0.0f) {
+            const float q = num / den, d = dn / den;
+            hit = q >= 0 && q < 1 && d >= 0;
+            if (hit) dist = fabsf(d);
+        }
+    }
+    inside = __popc(__ballot_sync(0xffffffffu, hit)) & 1;
+    // distances are not negative: they order as their bits
+    const float m = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(dist)));
+    return m < GX_INFI_DIST + 1 ? m : GX_INFI_DIST + 1;
+}
+
+template <bool WARP>
+__device__ __forceinline__ float ray_polygon(float2 p0, float2 v, const float2 *poly, int n, int &inside)
+{
+    return WARP ? ray_intersect_polygon_warp(p0, v, poly, n, inside) : ray_intersect_polygon(p0, v, poly, n, inside);
+}
+
+template <bool WARP = false>
 static __device__ uint32_t inwhere_mlc(const DevCtx &C, int field, float qx, float qy, float qz, int &index, int &bank)
 {
     uint32_t inew = 1;
     float2 p = make_float2(qx, qz);
-    if (index == GX_OUTMLC) index = index_of_leaf(C, p);
+    if (index == GX_OUTMLC) index = index_of_leaf<WARP>(C, p);
     p.x = qy;
     if (index >= 0) {
-        bank = point_in_leaf(p, endnode_of(C, field, index));
+        bank = point_in_leaf<WARP>(p, endnode_of(C, field, index));
         if (bank > 0) inew = 3; else inew = 1;
     }
     return inew;
 }
 
+template <bool WARP = false>
 static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
 {
     const Part p = p0;
@@ -322,7 +374,7 @@ static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
     bool yz = false;
     for (int turn = 0;; turn++) {
         int ins;
-        const float d = ray_intersect_polygon(yz ? p2 : p1, yz ? dir2 : dir1, poly, n, ins);
+        const float d = ray_polygon<WARP>(yz ? p2 : p1, yz ? dir2 : dir1, poly, n, ins);
         if (turn == 0) {
             dis_xz = d;
             inside_xz = ins;
@@ -339,7 +391,7 @@ static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
                 to_new_region = true;
                 break;
             }
-            if (p.leafIndex <= -60) index = index_of_leaf(C, p1);
+            if (p.leafIndex <= -60) index = index_of_leaf<WARP>(C, p1);
             if (index <= -60) break;
             leaf = index >= 0;
             yz = false;
@@ -352,7 +404,7 @@ static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
             } else {
                 // the leaf (or gap) where the ray leaves the MLC; in double, as geom.cu:591
                 const float2 p3 = make_float2(p1.x + dis_xz * dir1.x, p1.y + (dis_xz - 0.001) * dir1.y);
-                limit1 = index_of_leaf(C, p3);
+                limit1 = index_of_leaf<WARP>(C, p3);
                 if (limit1 < 0) limit1 = -limit1;
                 if (dir1.x < 0) { sx = -1; if (limit1 > 0) limit1 -= 1; limit2 = -index + 1; }
                 else { limit2 = limit1; limit1 = -index - 1; }
@@ -374,6 +426,22 @@ static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
             i += sx;
             poly += 16 * sx;
             if (!(i >= limit1 && i <= limit2 && temp1 >= GX_INFI_DIST)) break;
+            if (WARP) {
+                // the rest of the walk, a leaf to a lane: the first that is hit ends it
+                for (; i >= limit1 && i <= limit2; i += 32 * sx) {
+                    const int j = i + sx * (int)(threadIdx.x & 31u);
+                    float dj = GX_INFI_DIST + 1;
+                    if (j >= limit1 && j <= limit2) dj = ray_intersect_polygon(p1, dir1, C.crossXZ + 16 * j, 14, ins);
+                    const unsigned hit = __ballot_sync(0xffffffffu, dj < GX_INFI_DIST);
+                    if (hit) {
+                        const int k = __ffs(hit) - 1;
+                        temp1 = __shfl_sync(0xffffffffu, dj, k);
+                        i += sx * (k + 1);
+                        break;
+                    }
+                }
+                break;
+            }
         }
     }
     if (!to_new_region) {
@@ -404,7 +472,7 @@ static __device__ uint32_t howfar_mlc(const DevCtx &C, Part &p0, float &t)
         } else return inew;
     }
     float qx = p.x + t * p.u, qy = p.y + t * p.v, qz = p.z + t * p.w;
-    inew = inwhere_mlc(C, p.field, qx, qy, qz, index, bank);
+    inew = inwhere_mlc<WARP>(C, p.field, qx, qy, qz, index, bank);
     p0.leafIndex = (int8_t)index;
     p0.bank = (int8_t)bank;
     return inew;
@@ -430,6 +498,7 @@ __device__ __forceinline__ JawPolys jaw_polys(const DevCtx &C, int field, bool x
 // howfar_SecJawsY and howfar_SecJawsX (geom.cu:793-1035) in one: the Y jaws
 // open in x, the X jaws in y. The reference's X routine steps to the opening
 // from the tungsten by the distance to the bounds in YZ; kept.
+template <bool WARP = false>
 static __device__ uint32_t howfar_secjaws(const DevCtx &C, Part &p, float &t)
 {
     const bool xjaw = p.module == GEGS_M_SECJAWX;
@@ -437,39 +506,72 @@ static __device__ uint32_t howfar_secjaws(const DevCtx &C, Part &p, float &t)
     const float2 p1 = make_float2(p.y, p.z), p2 = make_float2(p.x, p.z);
     const float2 dir1 = make_float2(p.v, p.w), dir2 = make_float2(p.u, p.w);
     const float2 q = xjaw ? p1 : p2, dq = xjaw ? dir1 : dir2;
-    // one polygon per turn: the bounds seen from (y, z) and from (x, z); then
-    // from the opening the two jaws around it, from a jaw the opening
     float dis_xz = 0.0f, dis_yz = 0.0f, minBoundaryDist = 0.0f, jaw0 = 0.0f, d;
     int inside_xz = 0, ins;
     bool open = false;
-    float2 o = p1, v = dir1;
-    const float2 *poly = J.bmax;
-    for (int turn = 0;; turn++) {
-        d = ray_intersect_polygon(o, v, poly, 4, ins);
-        if (turn == 0) {
-            dis_xz = d;
-            inside_xz = ins;
-            o = p2;
-            v = dir2;
-        } else if (turn == 1) {
-            dis_yz = d;
-            if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
-            minBoundaryDist = dis_xz < dis_yz ? dis_xz : dis_yz;
-            if (!(inside_xz && ins)) {
-                if (!(t > minBoundaryDist)) return 1;
-                t = minBoundaryDist + GX_EPSTEP;
-                const float y = p.y + t * p.v, x = p.x + t * p.u;
-                if (!point_in_polygon(y, x, J.bmin, 4)) return 0;
-                return point_in_polygon(xjaw ? y : x, p.z + t * p.w, J.geom + 2, 4) ? 1 : 2;
-            }
-            open = point_in_polygon(q.x, q.y, J.geom + 2, 4);
-            o = q;
-            v = dq;
-            poly = open ? J.geom : J.geom + 2;
-        } else if (turn == 2 && open) {
-            jaw0 = d;
-            poly = J.geom + 4;
-        } else break;
+    // outside the bounds: to them, and what lies behind
+    auto from_outside = [&]() -> uint32_t {
+        if (!(t > minBoundaryDist)) return 1;
+        t = minBoundaryDist + GX_EPSTEP;
+        const float y = p.y + t * p.v, x = p.x + t * p.u;
+        if (!in_polygon<WARP>(y, x, J.bmin, 4)) return 0;
+        return in_polygon<WARP>(xjaw ? y : x, p.z + t * p.w, J.geom + 2, 4) ? 1 : 2;
+    };
+    if (WARP) {
+        // all polygons at once, four lanes to each: the bounds seen from (y, z) and
+        // from (x, z), the two jaws, the opening, and the point in the opening
+        const int k = (int)(threadIdx.x & 31u) >> 2, i = (int)threadIdx.x & 3;
+        const float2 o = k == 0 ? p1 : k == 1 ? p2 : q, v = k == 0 ? dir1 : k == 1 ? dir2 : dq;
+        const float2 *poly = k < 2 ? J.bmax : J.geom + (k == 2 ? 0 : k == 3 ? 4 : 2);
+        const float2 a = ld2(&poly[i]), b = ld2(&poly[(i + 1) & 3]);
+        float num, den, dn, dist = GX_INFI_DIST + 1;
+        ray_edge(o, v, a, b, num, den, dn);
+        bool hit = false;
+        if (k == 5) {
+            if ((a.y < q.y) != (b.y < q.y) && (a.y >= q.y || b.y >= q.y) && (a.x <= q.x || b.x <= q.x))
+                hit = b.x + (q.y - b.y) / (a.y - b.y) * (a.x - b.x) < q.x;   // the edge that ends at b, as point_in_polygon takes it
+        } else if (k < 5 && den != 0.0f) {
+            const float u = num / den, e = dn / den;
+            hit = u >= 0 && u < 1 && e >= 0;
+            if (hit) dist = fminf(fabsf(e), GX_INFI_DIST + 1);
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        dist = fminf(dist, __shfl_xor_sync(0xffffffffu, dist, 1));
+        dist = fminf(dist, __shfl_xor_sync(0xffffffffu, dist, 2));
+        dis_xz = __shfl_sync(0xffffffffu, dist, 0);
+        dis_yz = __shfl_sync(0xffffffffu, dist, 4);
+        if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
+        minBoundaryDist = dis_xz < dis_yz ? dis_xz : dis_yz;
+        if (!((__popc(hits & 0xfu) & 1) && (__popc(hits & 0xf0u) & 1))) return from_outside();
+        open = __popc(hits & 0xf00000u) & 1;
+        jaw0 = __shfl_sync(0xffffffffu, dist, 8);
+        d = open ? __shfl_sync(0xffffffffu, dist, 12) : __shfl_sync(0xffffffffu, dist, 16);
+    } else {
+        // one polygon per turn: the bounds seen from (y, z) and from (x, z); then
+        // from the opening the two jaws around it, from a jaw the opening
+        float2 o = p1, v = dir1;
+        const float2 *poly = J.bmax;
+        for (int turn = 0;; turn++) {
+            d = ray_intersect_polygon(o, v, poly, 4, ins);
+            if (turn == 0) {
+                dis_xz = d;
+                inside_xz = ins;
+                o = p2;
+                v = dir2;
+            } else if (turn == 1) {
+                dis_yz = d;
+                if (dis_xz >= GX_INFI_DIST || dis_yz >= GX_INFI_DIST) return 0;
+                minBoundaryDist = dis_xz < dis_yz ? dis_xz : dis_yz;
+                if (!(inside_xz && ins)) return from_outside();
+                open = point_in_polygon(q.x, q.y, J.geom + 2, 4);
+                o = q;
+                v = dq;
+                poly = open ? J.geom : J.geom + 2;
+            } else if (turn == 2 && open) {
+                jaw0 = d;
+                poly = J.geom + 4;
+            } else break;
+        }
     }
     if (open) {
         const float jaw = jaw0 < GX_INFI_DIST ? jaw0 : d;
@@ -737,7 +839,7 @@ __device__ __forceinline__ bool in_geom_class(const Part &p)
     return G == GX_GEOM_ALL || geom_class_of(p.module) == G;
 }
 
-template <int G>
+template <int G, bool WARP = false>
 __device__ __forceinline__ uint32_t howfar_g(const DevCtx &C, Part &p, float &t, bool &ok)
 {
     if (G == GX_GEOM_ALL) return howfar(C, p, t, ok);
@@ -745,9 +847,9 @@ __device__ __forceinline__ uint32_t howfar_g(const DevCtx &C, Part &p, float &t,
     if (G == GX_GEOM_PHANTOM) {
         if (p.module == GEGS_M_PHANTOM) return howfar_phantom(C, p, t);
     } else if (G == GX_GEOM_MLC) {
-        if (p.module == GEGS_M_VARMLC) return howfar_mlc(C, p, t);
+        if (p.module == GEGS_M_VARMLC) return howfar_mlc<WARP>(C, p, t);
     } else {
-        if (p.module == GEGS_M_SECJAWY || p.module == GEGS_M_SECJAWX) return howfar_secjaws(C, p, t);
+        if (p.module == GEGS_M_SECJAWY || p.module == GEGS_M_SECJAWX) return howfar_secjaws<WARP>(C, p, t);
     }
     ok = false;
     return 0;

@@ -207,8 +207,12 @@ enum : int {
 // kept from one step to the next, `gle` the logarithm of its energy. Every way out that scores or queues shares
 // one place, and the queueing itself is the caller's, so that the code is small.
 // SH: the {gmfp, cohe} table is staged in shared memory (stage_photon_tables).
-template <int G = GX_GEOM_ALL, bool SH = false>
-static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, float gle, int &out)
+// WARP: all lanes of the warp hold the same photon, that of the lane with thread
+// index `owner` (whose random window it draws from: a step draws three words at
+// most, and five or more are in the window), and share its polygons; the owner
+// scores.
+template <int G = GX_GEOM_ALL, bool SH = false, bool WARP = false>
+static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, float gle, int &out, uint32_t owner = 0)
 {
     const gegs_physics *P = C.P;
     const unsigned med = vx.med;
@@ -219,7 +223,7 @@ static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, flo
     int lgle = 0;
     if (!absorbed) {
         if (p.wt <= 0.0f) return STEP_DONE;
-        float r1 = U(C, r);
+        float r1 = (WARP ? rng_uniform_of(r, owner) : U(C, r));
         dpmfp = -gx_log(r1);
         float tstep, gmfp_val = 0.0f;
         if (med == GX_VACUUM) tstep = GX_VACUUM_STEP;
@@ -235,7 +239,7 @@ static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, flo
             tstep = gmfp_val * dpmfp;
         }
         bool ok;
-        const uint32_t new_region = howfar_g<G>(C, p, tstep, ok);
+        const uint32_t new_region = howfar_g<G, WARP>(C, p, tstep, ok);
         if (!ok) { atomicOr(C.err, GX_ERR_MODULE); return STEP_DONE; }
         if (new_region != p.region) vx = C.reg[new_region];
         if (new_region == 0) {
@@ -249,17 +253,20 @@ static __device__ int photon_step(const DevCtx &C, Part &p, Rng &r, Vox &vx, flo
         p.region = new_region;
         absorbed = idisc < 0 || (vx.med != med && p.e <= pcut_of(C, vx));   // above its own medium's cut already
     }
-    if (absorbed) { escore(C, p, p.region, p.e * p.wt); return STEP_DONE; }
+    if (absorbed) {
+        if (!WARP || threadIdx.x == owner) escore(C, p, p.region, p.e * p.wt);
+        return STEP_DONE;
+    }
     if ((vx.med != med) || (vx.med == GX_VACUUM) || gx_ge(dpmfp, GX_EPSGMFP)) return STEP_ON;
     if (vx.flags & GEGS_F_RAYLEIGH) {
-        const float r1 = U(C, r);
+        const float r1 = (WARP ? rng_uniform_of(r, owner) : U(C, r));
         if (r1 < 1.0f - cohfac) { out = ST_RAYLEIGH; return STEP_QUEUE; }
     }
     float2 b1 = __ldg(reinterpret_cast<const float2 *>(P->gbr1[vx.med * GX_MXGE + lgle]));
     float2 b2 = __ldg(reinterpret_cast<const float2 *>(P->gbr2[vx.med * GX_MXGE + lgle]));
     float gbr1_val = b1.x + b1.y * gle;
     float gbr2_val = b2.x + b2.y * gle;
-    const float r1 = U(C, r);
+    const float r1 = (WARP ? rng_uniform_of(r, owner) : U(C, r));
     out = (r1 <= gbr1_val) && (p.e > 2.0f * P->rm) ? ST_PAIR : r1 < gbr2_val ? ST_COMPTON : ST_PHOTO;
     return STEP_QUEUE;
 }

@@ -55,6 +55,38 @@ __device__ __forceinline__ void unpack_estate(const EStatePk &k, EState &s)
     s.is_tstep = (k.flags & 2u) != 0;
 }
 
+// One step of each photon of the lanes `act` in turn, by the whole warp: for the
+// few photons that are left when a queue has run out, which otherwise step at
+// the speed of one lane (a photon that goes along a jaw face or a leaf gap for
+// thousands of steps, 1.4 and 8 us each, one edge after another). Their polygon
+// edges are tested side by side. Every lane's random window has been filled.
+#define GX_SHARE_LANES 4
+template <int G>
+__device__ __forceinline__ void share_steps(const DevCtx &C, unsigned act, Part &p, Rng &r, Vox &vx, float gle, int &code, int &out)
+{
+    __syncwarp();
+    for (unsigned m = act; m; m &= m - 1u) {
+        const int src = __ffs(m) - 1;
+        Part q = part_of(p, src);
+        Vox v;
+        v.med = (uint16_t)__shfl_sync(0xffffffffu, (uint32_t)vx.med, src);
+        v.flags = (uint16_t)__shfl_sync(0xffffffffu, (uint32_t)vx.flags, src);
+        v.rhof = __shfl_sync(0xffffffffu, vx.rhof, src);
+        const float g = __shfl_sync(0xffffffffu, gle, src);
+        Rng rq = {};
+        rq.ctr = __shfl_sync(0xffffffffu, r.ctr, src);
+        int to = -1;
+        const int c = photon_step<G, false, true>(C, q, rq, v, g, to, (threadIdx.x & ~31u) + (uint32_t)src);
+        if ((int)(threadIdx.x & 31u) == src) {
+            p = q;
+            vx = v;
+            r.ctr = rq.ctr;
+            code = c;
+            out = to;
+        }
+    }
+}
+
 __device__ __forceinline__ uint32_t queue_len(const DevCtx &C, int q)
 {
     uint32_t n = *((volatile uint32_t *)&C.q.count[q]);

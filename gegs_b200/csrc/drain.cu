@@ -163,15 +163,26 @@ __device__ __noinline__ void drain_transport()
             const uint32_t other = lane < GX_DT_N && (int)lane != T ? w.cnt[lane] : 0u;
             leave = __any_sync(0xffffffffu, other >= 16u);
         }
+        const bool in_class = in_geom_class<G>(p);     // before the step, which may leave it
+        int code = STEP_ON, shared = -1;
+        const bool share = !ELEC && cls < 2 && !leave && __popc(act) <= GX_SHARE_LANES;
+        if (share) {
+            const bool stepping = active && in_class;
+            if (stepping) rng_window(C, r);
+            share_steps<G>(C, __ballot_sync(0xffffffffu, stepping), p, r, vx, gle, code, shared);
+        }
         if (active) {
             int to = -1, out = 0;                 // the stack the particle leaves for; the stage it is new in there
             bool moved = true;
             if (leave) to = T;
-            else if (!in_geom_class<G>(p)) to = (ELEC ? GX_DT_E : GX_DT_P) + geom_class_of(p.module) - GX_GEOM_JAWS;
+            else if (!in_class) to = (ELEC ? GX_DT_E : GX_DT_P) + geom_class_of(p.module) - GX_GEOM_JAWS;
             else {
                 steps++;
-                rng_window(C, r);
-                const int code = ELEC ? electron_step<G>(C, p, r, s, vx, out) : photon_step<G>(C, p, r, vx, gle, out);
+                if (share) out = shared;
+                else {
+                    rng_window(C, r);
+                    code = ELEC ? electron_step<G>(C, p, r, s, vx, out) : photon_step<G>(C, p, r, vx, gle, out);
+                }
                 if (code == STEP_DONE) active = false;
                 else if (code == STEP_QUEUE) { to = stack_of(out, p); moved = false; }
             }

@@ -159,13 +159,16 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
 #ifndef GX_EPHANTOM_MIN_BLOCKS
 #define GX_EPHANTOM_MIN_BLOCKS 4
 #endif
-// the jaws photons (and their long tracks): 48 registers, 0.3 % faster than 64
+// the jaws photons (and their long tracks) and the MLC photons hold a second
+// step, the one the warp shares (share_steps): 80 and 128 registers. With 48 and
+// 80 that step's registers spill in the other one too: CT of 161x117x87, 3
+// fields, 3M histories (two plans) 148.4 ms against 136.0, CT head 5-field plan,
+// 16M (two) 518.4 against 509.9; without the shared step 156.4 and 512.6.
 #ifndef GX_PJAWS_MIN_BLOCKS
-#define GX_PJAWS_MIN_BLOCKS 5
+#define GX_PJAWS_MIN_BLOCKS 3
 #endif
-// the MLC photon kernel, the most divergent, runs best with 80 registers (fewer spills)
 #ifndef GX_PMLC_MIN_BLOCKS
-#define GX_PMLC_MIN_BLOCKS 3
+#define GX_PMLC_MIN_BLOCKS 2
 #endif
 // the first pass of the jaws and MLC electrons, without howfar: 80 registers
 // (3 blocks; CT head 5-field plan, 16M histories: 1.8 % faster than 48, with
@@ -221,23 +224,28 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
     }
     timeline_mark(C, tl, false);
     if (!ELEC) stage_photon_tables(C);
-    // per-class budgets (measured on the CT 5-field plan): photons take 8x their
-    // budget in the jaws and MLC, where a few bounce along leaf gaps for many
-    // steps; electrons take 2x theirs in the phantom
-    const uint32_t budget = (ELEC ? (cls < 2 ? C.electron_budget : 2u * C.electron_budget)
-                                  : (cls < 2 ? 8u * C.photon_budget : C.photon_budget)) << *C.budget_shift;
-    // A jaws photon takes a handful of steps, except the rare one that runs
-    // almost parallel to a jaw face in tens of thousands of tiny steps. Past
-    // its budget such a photon keeps stepping while the other photon consumers
-    // of the wave are still running (up to 64 budgets), so that its long track
-    // advances with the bulk of the work instead of one budget per wave in the
-    // run's tail. Only when the phase's kernels run concurrently (C.overlap).
+    // Per-class budgets (measured on the CT 5-field plan): electrons take 2x their
+    // budget in the phantom. A jaws photon takes a handful of steps, except the
+    // rare one that runs almost parallel to a jaw face in tens of thousands of
+    // tiny steps, and an MLC photon a few, except one in a million that goes
+    // along a leaf gap for thousands, at 8 us each. Past its budget such a photon
+    // keeps stepping while the other transport branches of the wave still run (up
+    // to 64 budgets), so that its long track advances with the bulk of the work
+    // and neither holds a wave up nor is left for the run's tail. The jaws take
+    // 8x the photons' budget before that; the MLC 1x (8x: CT head 5-field plan,
+    // 1M histories, one such photon added 2 ms to each of nine waves). Only when
+    // the phase's kernels run concurrently (C.overlap).
     constexpr bool JAWS_PHOTON = !ELEC && G == GX_GEOM_JAWS;
-    // In the pipelined form the jaws photons step on while any of the five
-    // other transport branches of the wave (both particle types) still runs.
+    constexpr bool EXTEND = !ELEC && cls < 2;
+    const uint32_t budget = (ELEC ? (cls < 2 ? C.electron_budget : 2u * C.electron_budget)
+                                  : (JAWS_PHOTON || (cls < 2 && !C.overlap) ? 8u : 1u) * C.photon_budget)
+                            << *C.budget_shift;
+    // How many of the other branches have to be done for that to end: of both
+    // particle types in the pipelined form, else of the photons; the MLC's own is
+    // not among them, and it does not wait for the jaws photons, which wait for it.
     const volatile uint32_t *others_done = LONG ? C.electron_done : C.photon_done;
     const volatile uint32_t *others_done2 = C.electron_done;
-    const uint32_t others = LONG ? 3u : C.pipelined ? 5u : 2u;
+    const uint32_t others = LONG ? 3u : (C.pipelined ? 5u : 2u) - (JAWS_PHOTON ? 0u : 1u);
     // in the serial persistent form, a jaws photon still going when the photon
     // phase ends moves on to the long-track kernel, which runs beside the
     // electron phase the same way
@@ -255,6 +263,34 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
         active = refill<Q, ELEC>(C, hq, n_cont, n, qc_in, exhausted, active, p, r, s, vx, gle, taken);
         if (active && !was) nst = 0;
         if (!__any_sync(0xffffffffu, active)) break;
+        // (compiled for these kernels alone, and the condition below spelt out twice:
+        // a lambda for it made the phantom's kernels 7 % slower)
+        if constexpr (EXTEND) if (exhausted) {
+            const unsigned act = __ballot_sync(0xffffffffu, active);
+            if (__popc(act) <= GX_SHARE_LANES) {
+                int tq = -1, code = STEP_ON;
+                const bool stepping = active && in_geom_class<G>(p);
+                if (active && !stepping) tq = base + 2 * (geom_class_of(p.module) - GX_GEOM_JAWS) + (int)(par ^ 1u);
+                if (stepping) {
+                    steps++;
+                    rng_window(C, r);
+                }
+                share_steps<G>(C, __ballot_sync(0xffffffffu, stepping), p, r, vx, gle, code, tq);
+                if (stepping) {
+                    if (code == STEP_DONE) active = false;
+                    else if (code == STEP_ON && ++nst >= budget &&
+                             (!EXTEND || !C.overlap || nst >= 64u * budget ||
+                            (((nst - budget) & 15u) == 0u &&
+                             *others_done + (C.pipelined && !LONG ? *others_done2 : 0u) >= others)))
+                        tq = q_limit;
+                }
+                if (tq >= 0) {
+                    queue_particle<false>(C, tq, p, r, s);
+                    active = false;
+                }
+                continue;
+            }
+        }
         if (active) {
             int tq = -1;                          // the queue the particle leaves for
             if (!in_geom_class<G>(p)) tq = base + 2 * (geom_class_of(p.module) - GX_GEOM_JAWS) + (int)(par ^ 1u);
@@ -273,7 +309,7 @@ __device__ __forceinline__ void transport_consumer(const DevCtx &C)
                     tq = DEFER ? GX_Q_ENEAR + cls : qc_out;
                     steps--;
                 } else if (code == STEP_ON && ++nst >= budget &&
-                           (!JAWS_PHOTON || !C.overlap || nst >= 64u * budget ||
+                           (!EXTEND || !C.overlap || nst >= 64u * budget ||
                             (((nst - budget) & 15u) == 0u &&
                              *others_done + (C.pipelined && !LONG ? *others_done2 : 0u) >= others)))
                     tq = ELEC ? qc_out : q_limit;

@@ -62,7 +62,9 @@ typedef struct gegs_run_opts {
     uint32_t max_waves;        /* safety budget (0 = default) */
     uint32_t step_budget;      /* steps per particle per launch before it is continued in the next wave:
                                   bits 0-15 photons, 16-31 electrons (0 = defaults 32 / 8); photons get
-                                  8x theirs in the jaws and MLC, electrons 2x theirs in the phantom */
+                                  8x theirs in the jaws (8x in the MLC too where the wave's kernels run one
+                                  after another), electrons 2x theirs in the phantom; a photon of the jaws or
+                                  the MLC goes on past it while other kernels of its wave run */
     uint32_t refill_below;     /* new histories are injected once fewer than this many particles are in
                                   flight, topping the population up to `batch` (0 = default batch / 4) */
     uint32_t queue_cap;        /* testing aid: at most this many records per event queue (0 = sized from
