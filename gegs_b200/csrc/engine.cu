@@ -11,6 +11,7 @@
 #include <vector>
 #include "kernels.cuh"
 #include "drain.cuh"
+#include "staging.h"
 #include "../../include/gegs.h"
 
 namespace {
@@ -1127,8 +1128,8 @@ extern "C" gegs_status gegs_launch_group(gegs_engine *const *engines, int32_t n,
 extern "C" gegs_status gegs_get_tally(gegs_engine *e, int64_t *out, uint64_t nvox)
 {
     if (!e || !out || nvox != e->nvox || !e->d_tally) return GEGS_ERR_ARG;
-    CK(cudaMemcpyAsync(out, e->d_tally, nvox * 8, cudaMemcpyDeviceToHost, e->stream), "tally D2H");
-    CK(cudaStreamSynchronize(e->stream), "tally sync");
+    CK(cudaSetDevice(e->device), "cudaSetDevice");
+    CK(staged_to_host(out, e->d_tally, nvox * 8, e->stream), "tally D2H");
     return GEGS_OK;
 }
 
@@ -1170,17 +1171,17 @@ extern "C" gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const geg
 extern "C" gegs_status gegs_get_dose(gegs_engine *e, const float *voxel_mass, double dose_unit, double *out, uint64_t nvox)
 {
     if (!e || !out || !voxel_mass || nvox != e->nvox || !e->d_tally) return GEGS_ERR_ARG;
+    CK(cudaSetDevice(e->device), "cudaSetDevice");
     float *d_mass = nullptr;
     double *d_out = nullptr;
-    CK(cudaMallocAsync(&d_mass, nvox * 4, e->stream), "mass");
-    CK(cudaMallocAsync(&d_out, nvox * 8, e->stream), "dose");
-    CK(cudaMemcpyAsync(d_mass, voxel_mass, nvox * 4, cudaMemcpyHostToDevice, e->stream), "mass H2D");
+    CK(scratch_alloc((void **)&d_mass, nvox * 4, e->stream), "mass");
+    CK(scratch_alloc((void **)&d_out, nvox * 8, e->stream), "dose");
+    CK(staged_to_device(d_mass, voxel_mass, nvox * 4, e->stream), "mass H2D");
     k_dose<<<e->nsm * 4, 256, 0, e->stream>>>(e->d_tally, d_mass, dose_unit, d_out, nvox);
     CK(cudaGetLastError(), "dose kernel");
-    CK(cudaMemcpyAsync(out, d_out, nvox * 8, cudaMemcpyDeviceToHost, e->stream), "dose D2H");
+    CK(staged_to_host(out, d_out, nvox * 8, e->stream), "dose D2H");
     cudaFreeAsync(d_mass, e->stream);
     cudaFreeAsync(d_out, e->stream);
-    CK(cudaStreamSynchronize(e->stream), "dose sync");
     return GEGS_OK;
 }
 
@@ -1223,13 +1224,13 @@ extern "C" gegs_status gegs_stat_get(gegs_engine *e, double *mean, double *rel_s
     if (e->stat_batches < 2) { e->err = "gegs_stat_get: at least two folded batches are needed"; return GEGS_ERR_ARG; }
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     double *d_mean = nullptr, *d_rel = nullptr;
-    CK(cudaMallocAsync(&d_mean, nvox * 8, e->stream), "stat output");
-    CK(cudaMallocAsync(&d_rel, nvox * 8, e->stream), "stat output");
+    CK(scratch_alloc((void **)&d_mean, nvox * 8, e->stream), "stat output");
+    CK(scratch_alloc((void **)&d_rel, nvox * 8, e->stream), "stat output");
     k_stat_final<<<e->nsm * 8, 256, 0, e->stream>>>(e->d_stat_s1, e->d_stat_s2, (double)e->stat_batches, d_mean, d_rel,
                                                    nvox);
     CK(cudaGetLastError(), "stat final");
-    CK(cudaMemcpyAsync(mean, d_mean, nvox * 8, cudaMemcpyDeviceToHost, e->stream), "stat D2H");
-    CK(cudaMemcpyAsync(rel_se, d_rel, nvox * 8, cudaMemcpyDeviceToHost, e->stream), "stat D2H");
+    CK(staged_to_host(mean, d_mean, nvox * 8, e->stream), "stat D2H");
+    CK(staged_to_host(rel_se, d_rel, nvox * 8, e->stream), "stat D2H");
     cudaFreeAsync(d_mean, e->stream);
     cudaFreeAsync(d_rel, e->stream);
     CK(cudaStreamSynchronize(e->stream), "stat sync");
@@ -1494,7 +1495,7 @@ extern "C" gegs_status gegs_backward(gegs_engine *e, uint64_t hist_begin, uint64
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     bool fresh = false;
     if (!e->d_gvm) { CK(cudaMalloc(&e->d_gvm, e->nvox * sizeof(double)), "voxel gradient"); fresh = true; }
-    CK(cudaMemcpyAsync(e->d_gvm, voxel_grad, e->nvox * sizeof(double), cudaMemcpyHostToDevice, e->stream), "gvm H2D");
+    CK(staged_to_device(e->d_gvm, voxel_grad, e->nvox * sizeof(double), e->stream), "gvm H2D");
     CK(cudaMemsetAsync(e->d_grad, 0, (size_t)n * GX_GRAD_COPIES * sizeof(double), e->stream), "grad reset");
     // replay the histories with unit fluence weights, scoring into the gradient
     DevCtx saved = e->ctx;

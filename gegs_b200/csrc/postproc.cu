@@ -5,19 +5,22 @@
 //                      agreement) of an evaluated dose against a reference dose;
 //   gegs_ct_ramp       HU -> (medium, density) through a piecewise-linear ramp
 //                      (CTToMedium's 4-material ramp, ctcreate.c:913-970,1057-1104).
-// Host buffers in and out; device memory is allocated per call.
+// Host buffers in and out, through pinned buffers and scratch that the library
+// keeps (staging.cpp); all on the legacy stream.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 #include "../../include/gegs_post.h"
+#include "staging.h"
 
 namespace {
 
 struct DevBuf {
     void *p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
+    ~DevBuf() { if (p) cudaFreeAsync(p, 0); }
 };
 
 // ---- interpolation -------------------------------------------------------
@@ -105,6 +108,35 @@ __global__ void k_gamma(const float *__restrict__ ref, const float *__restrict__
     }
 }
 
+// Largest value, as an integer that orders like the float (0: below every
+// value); out[1] set if any is not a number.
+__host__ __device__ inline uint32_t to_ordered(uint32_t bits) { return bits & 0x80000000u ? ~bits : bits | 0x80000000u; }
+
+inline float from_ordered(uint32_t o)
+{
+    const uint32_t bits = o & 0x80000000u ? o & 0x7fffffffu : ~o;
+    float f;
+    memcpy(&f, &bits, sizeof f);
+    return f;
+}
+
+__global__ void k_max(const float *__restrict__ v, long long n, uint32_t *out)
+{
+    uint32_t top = 0;
+    bool nan = false;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const float f = v[t];
+        nan |= f != f;
+        top = max(top, to_ordered(__float_as_uint(f)));
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    nan = __any_sync(0xffffffffu, nan);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&out[0], top);
+        if (nan) out[1] = 1u;
+    }
+}
+
 // ---- CT ramp --------------------------------------------------------------
 __global__ void k_ct_ramp(const int16_t *__restrict__ hu, long long n, const gegs_ct_ramp_segment *seg, int nseg,
                           double hu_lower, uint16_t *med, float *dens)
@@ -145,8 +177,8 @@ __global__ void k_ct_ramp(const int16_t *__restrict__ hu, long long n, const geg
 template <typename T>
 int dev_copy(DevBuf &b, const T *h, size_t n)
 {
-    PK(cudaMalloc(&b.p, n * sizeof(T) + 16));
-    if (h) PK(cudaMemcpy(b.p, h, n * sizeof(T), cudaMemcpyHostToDevice));
+    PK(scratch_alloc(&b.p, n * sizeof(T) + 16, 0));
+    if (h) PK(staged_to_device(b.p, h, n * sizeof(T), 0));
     return 0;
 }
 
@@ -186,17 +218,37 @@ extern "C" int gegs_interp_dose(int device, const float *dose, int nx, int ny, i
     k_interp<<<grid_for(nout), 256>>>((const float *)dd.p, nx, ny, nz, (const float *)dx.p, (const float *)dy.p,
                                       (const float *)dz.p, x0, y0, z0, sx, sy, sz, mx, my, mz, (float *)dout.p);
     PK(cudaGetLastError());
-    PK(cudaMemcpy(out, dout.p, (size_t)nout * sizeof(float), cudaMemcpyDeviceToHost));
+    PK(staged_to_host(out, dout.p, (size_t)nout * sizeof(float), 0));
     return 0;
 }
 
-extern "C" int gegs_gamma3d(int device, const float *ref, const float *eval, int nx, int ny, int nz, float dx, float dy,
-                            float dz, float dta, float dd_abs, float cutoff_abs, float search_dta, float *gamma,
-                            uint64_t *n_evaluated, uint64_t *n_passed)
+// dd and cutoff: absolute, or (of_max) fractions of the largest reference dose,
+// which the device finds.
+static int gamma3d(int device, const float *ref, const float *eval, int nx, int ny, int nz, float dx, float dy, float dz,
+                   float dta, double dd, double cutoff, bool of_max, float search_dta, float *gamma,
+                   uint64_t *n_evaluated, uint64_t *n_passed)
 {
-    if (!ref || !eval || !gamma || nx <= 0 || ny <= 0 || nz <= 0 || !(dta > 0) || !(dd_abs > 0) || !(search_dta > 0))
-        return 1;
+    if (!ref || !eval || !gamma || nx <= 0 || ny <= 0 || nz <= 0 || !(dta > 0) || !(search_dta > 0)) return 1;
+    float dd_abs = (float)dd, cutoff_abs = (float)cutoff;
+    if (!of_max && !(dd_abs > 0)) return 1;
     PK(cudaSetDevice(device));
+    const long long n = (long long)nx * ny * nz;
+    DevBuf dr, de, dg, doff, dod2, dcnt;
+    int st;
+    if ((st = dev_copy<unsigned long long>(dcnt, nullptr, 2)) || (st = dev_copy(dr, ref, (size_t)n))) return st;
+    PK(cudaMemsetAsync(dcnt.p, 0, 2 * sizeof(unsigned long long), 0));
+    if (of_max) {
+        k_max<<<grid_for(n), 256>>>((const float *)dr.p, n, (uint32_t *)dcnt.p);
+        PK(cudaGetLastError());
+        uint32_t top[2];
+        PK(cudaMemcpy(top, dcnt.p, sizeof top, cudaMemcpyDeviceToHost));
+        if (top[1]) return 1;                        // a dose that is not a number
+        const float rmax = from_ordered(top[0]);
+        dd_abs = (float)(dd * (double)rmax);
+        cutoff_abs = (float)(cutoff * (double)rmax);
+        if (!(dd_abs > 0)) return 1;
+        PK(cudaMemsetAsync(dcnt.p, 0, 2 * sizeof(unsigned long long), 0));
+    }
     // offsets within search_dta * dta, sorted by squared distance (float arithmetic as the kernel's)
     float rmax = search_dta * dta;
     int rx = (int)(rmax / dx), ry = (int)(rmax / dy), rz = (int)(rmax / dz);
@@ -214,24 +266,35 @@ extern "C" int gegs_gamma3d(int device, const float *ref, const float *eval, int
     std::vector<int4> o4(offs.size());
     std::vector<float> o2(offs.size());
     for (size_t k = 0; k < offs.size(); k++) { o4[k] = offs[k].second; o2[k] = offs[k].first; }
-    long long n = (long long)nx * ny * nz;
-    DevBuf dr, de, dg, doff, dod2, dcnt;
-    int st;
-    if ((st = dev_copy(dr, ref, (size_t)n)) || (st = dev_copy(de, eval, (size_t)n)) ||
-        (st = dev_copy<float>(dg, nullptr, (size_t)n)) || (st = dev_copy(doff, o4.data(), o4.size())) ||
-        (st = dev_copy(dod2, o2.data(), o2.size())) || (st = dev_copy<unsigned long long>(dcnt, nullptr, 2)))
+    if ((st = dev_copy(de, eval, (size_t)n)) || (st = dev_copy<float>(dg, nullptr, (size_t)n)) ||
+        (st = dev_copy(doff, o4.data(), o4.size())) || (st = dev_copy(dod2, o2.data(), o2.size())))
         return st;
-    PK(cudaMemset(dcnt.p, 0, 2 * sizeof(unsigned long long)));
     k_gamma<<<grid_for(n), 256>>>((const float *)dr.p, (const float *)de.p, nx, ny, nz, (const int4 *)doff.p,
                                   (const float *)dod2.p, (int)o4.size(), 1.0f / (dta * dta),
                                   1.0f / (dd_abs * dd_abs), cutoff_abs, (float *)dg.p, (unsigned long long *)dcnt.p);
     PK(cudaGetLastError());
     unsigned long long cnt[2];
     PK(cudaMemcpy(cnt, dcnt.p, sizeof cnt, cudaMemcpyDeviceToHost));
-    PK(cudaMemcpy(gamma, dg.p, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
+    PK(staged_to_host(gamma, dg.p, (size_t)n * sizeof(float), 0));
     if (n_evaluated) *n_evaluated = cnt[0];
     if (n_passed) *n_passed = cnt[1];
     return 0;
+}
+
+extern "C" int gegs_gamma3d(int device, const float *ref, const float *eval, int nx, int ny, int nz, float dx, float dy,
+                            float dz, float dta, float dd_abs, float cutoff_abs, float search_dta, float *gamma,
+                            uint64_t *n_evaluated, uint64_t *n_passed)
+{
+    return gamma3d(device, ref, eval, nx, ny, nz, dx, dy, dz, dta, dd_abs, cutoff_abs, false, search_dta, gamma,
+                   n_evaluated, n_passed);
+}
+
+extern "C" int gegs_gamma3d_global(int device, const float *ref, const float *eval, int nx, int ny, int nz, float dx,
+                                   float dy, float dz, float dta, double dd, double cutoff, float search_dta,
+                                   float *gamma, uint64_t *n_evaluated, uint64_t *n_passed)
+{
+    return gamma3d(device, ref, eval, nx, ny, nz, dx, dy, dz, dta, dd, cutoff, true, search_dta, gamma, n_evaluated,
+                   n_passed);
 }
 
 extern "C" int gegs_ct_ramp(int device, const int16_t *hu, uint64_t n, const gegs_ct_ramp_segment *segments,
@@ -247,7 +310,7 @@ extern "C" int gegs_ct_ramp(int device, const int16_t *hu, uint64_t n, const geg
     k_ct_ramp<<<grid_for((long long)n), 256>>>((const int16_t *)dh.p, (long long)n, (const gegs_ct_ramp_segment *)ds.p,
                                                nseg, hu_lower, (uint16_t *)dm.p, (float *)dd.p);
     PK(cudaGetLastError());
-    PK(cudaMemcpy(medium, dm.p, (size_t)n * sizeof(uint16_t), cudaMemcpyDeviceToHost));
-    PK(cudaMemcpy(density, dd.p, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
+    PK(staged_to_host(medium, dm.p, (size_t)n * sizeof(uint16_t), 0));
+    PK(staged_to_host(density, dd.p, (size_t)n * sizeof(float), 0));
     return 0;
 }

@@ -33,6 +33,9 @@ def _lib():
         L.gegs_interp_dose.argtypes = [i, vp, i, i, i, vp, vp, vp, f, f, f, f, f, f, i, i, i, vp]
         L.gegs_gamma3d.argtypes = [i, vp, vp, i, i, i, f, f, f, f, f, f, f, vp, C.POINTER(C.c_uint64),
                                    C.POINTER(C.c_uint64)]
+        L.gegs_gamma3d_global.argtypes = [i, vp, vp, i, i, i, f, f, f, f, C.c_double, C.c_double, f, vp,
+                                          C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]
+        L.gegs_trim.restype = None
         L.gegs_ct_ramp.argtypes = [i, vp, C.c_uint64, vp, i, C.c_double, vp, vp]
         _ready = True
     return L
@@ -76,12 +79,13 @@ def gamma3d(ref, ev, spacing, dta=0.1, dd=0.01, cutoff=0.10, search=3.0, device=
     if r.shape != e.shape or r.ndim != 3:
         raise ValueError("ref and eval must be (nz, ny, nx) arrays of one shape")
     nz, ny, nx = r.shape
-    rmax = float(r.max())
+    if r.size == 0:
+        raise ValueError("gamma of an empty grid")
     g = np.empty(r.size, np.float32)
     ne, npass = C.c_uint64(), C.c_uint64()
-    _check(_lib().gegs_gamma3d(device, r.ctypes.data, e.ctypes.data, nx, ny, nz, *(float(s) for s in spacing),
-                               float(dta), float(dd * rmax), float(cutoff * rmax), float(search), g.ctypes.data,
-                               C.byref(ne), C.byref(npass)), "gegs_gamma3d")
+    _check(_lib().gegs_gamma3d_global(device, r.ctypes.data, e.ctypes.data, nx, ny, nz, *(float(s) for s in spacing),
+                                      float(dta), float(dd), float(cutoff), float(search), g.ctypes.data,
+                                      C.byref(ne), C.byref(npass)), "gegs_gamma3d")
     return g.reshape(r.shape), (npass.value / ne.value if ne.value else float("nan"))
 
 

@@ -1,8 +1,8 @@
 /* Dose post-processing and phantom preparation on the GPU (libgegs_b200.so).
  *
- * Each call takes host buffers, allocates device memory for its own use,
- * and returns 0 on success, 1 for an invalid argument, 2 for a CUDA error
- * and 5 when device memory runs out.
+ * Each call takes host buffers, uses device memory of its own, and returns
+ * 0 on success, 1 for an invalid argument, 2 for a CUDA error and 5 when device
+ * memory runs out.
  */
 #ifndef GEGS_POST_H
 #define GEGS_POST_H
@@ -33,6 +33,13 @@ int gegs_gamma3d(int device, const float *ref, const float *eval, int nx, int ny
                  float dz, float dta, float dd_abs, float cutoff_abs, float search_dta, float *gamma,
                  uint64_t *n_evaluated, uint64_t *n_passed);
 
+/* The same with the dose difference and the cutoff as fractions of the largest
+ * reference dose, which the device finds (1 if that is not above 0, or if a
+ * reference dose is not a number). */
+int gegs_gamma3d_global(int device, const float *ref, const float *eval, int nx, int ny, int nz, float dx, float dy,
+                        float dz, float dta, double dd, double cutoff, float search_dta, float *gamma,
+                        uint64_t *n_evaluated, uint64_t *n_passed);
+
 /* One segment of a CT ramp: HU in (previous upper, hu_upper] maps to medium
  * with density linear from density_lower to density_upper. */
 typedef struct gegs_ct_ramp_segment {
@@ -48,6 +55,11 @@ typedef struct gegs_ct_ramp_segment {
  * density. */
 int gegs_ct_ramp(int device, const int16_t *hu, uint64_t n, const gegs_ct_ramp_segment *segments, int nseg,
                  double hu_lower, uint16_t *medium, float *density);
+
+/* Between calls the library keeps pinned buffers for copies from and to ordinary
+ * host memory (8 MB for each of at most four copies at once) and up to 256 MB
+ * of device scratch per device. Gives back what no call is using. */
+void gegs_trim(void);
 
 #ifdef __cplusplus
 }
