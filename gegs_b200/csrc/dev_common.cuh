@@ -60,7 +60,7 @@ static_assert(sizeof(gegs_field) % 16 == 0, "field record size");
 #define GX_TL_KERNELS 32   // wave timeline slots per wave
 // The drain kernel's particle types: photons and electrons of each geometry
 // class, then the eight interactions in stage order; and the records of one
-// type that a warp's stack holds (fewer than 32 when a warp claims 32 more).
+// type that a warp's stack holds at most (fewer than 32 when a warp claims 32 more).
 #define GX_DT_P 0
 #define GX_DT_E 3
 #define GX_DT_I 6
@@ -206,6 +206,7 @@ struct DevCtx {
     uint32_t photon_budget, electron_budget;   // steps per particle per launch before continuation
     Part *drain_part;       // the drain kernel's stacks: [warp][GX_DT_N][GX_DRAIN_CAP]
     EStatePk *drain_estate; // [warp][3][GX_DRAIN_CAP], step states of the electrons on them
+    uint32_t drain_cap;     // records of one type that a stack takes: GX_DRAIN_CAP, or fewer (gegs_set_drain_stack)
     unsigned long long *timeline;   // [timeline_waves][16][2] first start / last end (ns) per kernel; null: off
     uint32_t timeline_waves;
     QueueSet q;

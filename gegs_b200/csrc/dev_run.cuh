@@ -13,6 +13,7 @@ struct SchedState {
     uint32_t electron_done;           // electron branches finished in this wave
     uint32_t drain_below;             // the drain kernel takes over at this many particles and histories left (0: never)
     uint32_t drain;                   // 1: it does, after this plan
+    uint32_t resume;                  // 1: it left particles in the event queues, and the wave that takes them is planned
     unsigned long long drain_hist;    // histories it has claimed
     uint32_t budget_shift;            // step budgets of the next wave are shifted left by this (tail of a run)
 };

@@ -11,9 +11,10 @@
 // executes one kind of work at a time but waits for nobody. Warps that run low
 // claim more from the event queues, or histories not yet started. There are no
 // barriers and no waits: a warp ends when its stacks and the queues are empty.
-// A stack that is full sends the particle to the event queues, and the host
-// then runs further waves (no plan has been seen to need it; built with stacks
-// of 34 records, which overflow all the time, it gives the same tallies).
+// A stack that is full sends the particle to the event queues, and the run goes
+// on in waves behind the drain kernel, in the same launch (add_wave_loop). With
+// the tables' own single bremsstrahlung photon no plan has been seen to need
+// it; photons split more than 64 ways overflow at once.
 //
 // Bound by the longest cascade of one warp, step after step, and by fetching
 // instructions (all stages in one kernel: 6.9 cycles per issue, issue slots
@@ -93,7 +94,7 @@ __device__ __noinline__ void spill(const DevCtx &C, int type, Part p, const ESta
 __device__ __forceinline__ void stack_push(const DevCtx &C, int type, const Part &p, const EStatePk *k)
 {
     const uint32_t i = atomicAdd(&warp_of().cnt[type], 1u);
-    if (i < GX_DRAIN_CAP) {
+    if (i < C.drain_cap) {
         store_part(slot_part(C, type, i), p);
         if (k) *slot_estate(C, type, i) = *k;
     } else spill(C, type, p, k ? *k : fresh_estate());
@@ -133,7 +134,7 @@ __device__ __noinline__ void drain_transport()
     for (;;) {
         __syncwarp();
         uint32_t act = __ballot_sync(0xffffffffu, active);
-        const uint32_t have = min(w.cnt[T], (uint32_t)GX_DRAIN_CAP);
+        const uint32_t have = min(w.cnt[T], C.drain_cap);
         if (have > 0 && __popc(act) <= 24) {
             const uint32_t take = min(32u - __popc(act), have);
             const uint32_t rank = __popc(~act & ((1u << lane) - 1u));
@@ -214,7 +215,7 @@ __device__ __noinline__ void drain_interaction()
     constexpr int T = GX_DT_I + Q - (Q < ST_ELECTRON ? ST_COMPTON : ST_MOLLER - 4);
     DrainWarp &w = warp_of();
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t have = min(w.cnt[T], (uint32_t)GX_DRAIN_CAP);
+    const uint32_t have = min(w.cnt[T], C.drain_cap);
     const uint32_t take = min(32u, have);
     const bool active = lane < take;
     Part p;
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(kDrainThreads, 6) k_drain(const __grid_constan
         __syncwarp();
         uint32_t c = 0;
         if (lane < GX_DT_N) {
-            c = min(w.cnt[lane], (uint32_t)GX_DRAIN_CAP);
+            c = min(w.cnt[lane], C.drain_cap);
             w.cnt[lane] = c;
         }
         const uint32_t best = __reduce_max_sync(0xffffffffu, c * 32u + lane);

@@ -94,6 +94,7 @@ struct gegs_engine {
     Part *d_drain_part = nullptr;
     EStatePk *d_drain_estate = nullptr;
     int drain_grid = 0;
+    int run_grid = 0, run_threads = 0; // launch shape of the last run's waves
     bool has_head = true;              // the scene's modules include jaws or an MLC (or one this path does not model)
 
     DevCtx ctx{};
@@ -221,6 +222,7 @@ gegs_status gegs_create(int device, gegs_engine **out)
     cudaError_t c = cudaSetDevice(device);
     if (c != cudaSuccess) { gegs_status s = cuda_fail(e, c, "cudaSetDevice"); *out = e; return s; }
     cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device);
+    e->ctx.drain_cap = GX_DRAIN_CAP;
     CK(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "stream");
     e->stream = e->own_stream;
     CK(cudaEventCreate(&e->ev0), "event");
@@ -652,40 +654,57 @@ static void launch_wave_kernels(gegs_engine *e, int grid, int threads)
     join(3);
 }
 
-// Adds an engine's run to g: the first plan, a WHILE node whose body is one
-// wave and whose condition k_plan_cond sets on the device, then the drain
-// kernel for what the plan left to it.
-static gegs_status add_wave_loop(gegs_engine *e, cudaGraph_t g, int grid, int threads)
+// Adds a WHILE node to g, behind `after` (or first), and gives its body.
+static gegs_status add_while(gegs_engine *e, cudaGraph_t g, cudaGraphConditionalHandle handle, const cudaGraphNode_t *after,
+                             cudaGraphNode_t *node, cudaGraph_t *body)
 {
-    cudaGraphConditionalHandle handle;
-    CK(cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault), "conditional handle");
-    cudaGraphNode_t pnode = nullptr;
-    {
-        void *args[] = {(void *)&e->ctx, (void *)&e->d_sched, (void *)&handle};
-        cudaKernelNodeParams kp = {};
-        kp.func = (void *)k_plan_cond;
-        kp.gridDim = dim3(1);
-        kp.blockDim = dim3(32);
-        kp.kernelParams = args;
-        CK(cudaGraphAddKernelNode(&pnode, g, nullptr, 0, &kp), "planner node");
-    }
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    CK(cudaGraphAddNode(&cnode, g, &pnode, 1, &cp), "conditional node");
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CK(cudaStreamBeginCaptureToGraph(e->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
+    CK(cudaGraphAddNode(node, g, after, after ? 1 : 0, &cp), "conditional node");
+    *body = cp.conditional.phGraph_out[0];
+    return GEGS_OK;
+}
+
+// Adds an engine's run to g: the first plan, a WHILE node whose body is one
+// wave and whose condition k_plan_cond sets on the device, then the drain
+// kernel for what the plan left to it. These three are the body of another
+// WHILE node, which goes round once more where the drain kernel's full stacks
+// left particles in the event queues: those then go on in waves. So the run is
+// over when the graph is, and work behind it on the stream sees all of it.
+static gegs_status add_wave_loop(gegs_engine *e, cudaGraph_t g, int grid, int threads)
+{
+    const bool drains = e->drain_grid != 0;     // has any run of this engine left something to the drain kernel?
+    cudaGraphConditionalHandle again, handle;
+    cudaGraphNode_t pnode, cnode;
+    cudaGraph_t run = g, wave, captured;
+    if (drains) {
+        CK(cudaGraphConditionalHandleCreate(&again, g, 1, cudaGraphCondAssignDefault), "conditional handle");
+        gegs_status st = add_while(e, g, again, nullptr, &cnode, &run);
+        if (st != GEGS_OK) return st;
+    }
+    CK(cudaGraphConditionalHandleCreate(&handle, run, 0, 0), "conditional handle");
+    {
+        void *args[] = {(void *)&e->ctx, (void *)&e->d_sched, (void *)&handle};
+        cudaKernelNodeParams kp = {};
+        kp.func = (void *)k_plan_enter;
+        kp.gridDim = dim3(1);
+        kp.blockDim = dim3(32);
+        kp.kernelParams = args;
+        CK(cudaGraphAddKernelNode(&pnode, run, nullptr, 0, &kp), "planner node");
+    }
+    gegs_status st = add_while(e, run, handle, &pnode, &cnode, &wave);
+    if (st != GEGS_OK) return st;
+    CK(cudaStreamBeginCaptureToGraph(e->stream, wave, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
     launch_wave_kernels(e, grid, threads);
     k_plan_cond<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched, handle);
-    cudaGraph_t captured;
     CK(cudaStreamEndCapture(e->stream, &captured), "end capture");
-    if (!e->drain_grid) return GEGS_OK;     // no run of this engine has left anything to the drain kernel yet
-    CK(cudaStreamBeginCaptureToGraph(e->stream, g, &cnode, nullptr, 1, cudaStreamCaptureModeThreadLocal), "capture");
+    if (!drains) return GEGS_OK;
+    CK(cudaStreamBeginCaptureToGraph(e->stream, run, &cnode, nullptr, 1, cudaStreamCaptureModeThreadLocal), "capture");
     launch_drain(e->ctx, e->d_sched, e->has_head, e->drain_grid, e->stream);
-    k_drain_end<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
+    k_drain_end_cond<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched, again);
     CK(cudaStreamEndCapture(e->stream, &captured), "end capture");
     return GEGS_OK;
 }
@@ -827,6 +846,8 @@ static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t his
     R.threads = threads;
     R.max_waves = max_waves;
     R.drain_below = drain_below;
+    e->run_grid = grid;
+    e->run_threads = threads;
     return GEGS_OK;
 }
 
@@ -842,8 +863,10 @@ static gegs_status run_impl(gegs_engine *e, uint64_t hist_begin, uint64_t hist_e
     const int grid = R.grid, threads = R.threads;
     const uint32_t max_waves = R.max_waves;
     for (int k = 0; k < 16; k++) { e->last.stage_ms[k] = 0.0; e->last.stage_launches[k] = 0; }
-    if (o.mode == GEGS_MODE_PERSISTENT && hist_end - hist_begin <= R.drain_below) {
-        // the whole run goes to the drain kernel: no wave loop, so no graph
+    if (o.mode == GEGS_MODE_PERSISTENT && !launch_only && hist_end - hist_begin <= R.drain_below) {
+        // the whole run goes to the drain kernel: no wave loop, so no graph (but for
+        // what its stacks could not hold, run_finish; a launched run is over when
+        // its stream is, so it takes the graph)
         CK(cudaEventRecord(e->ev0, e->stream), "event");
         k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
         launch_drain(e->ctx, e->d_sched, e->has_head, e->drain_grid, e->stream);
@@ -994,10 +1017,11 @@ static gegs_status run_finish(gegs_engine *e)
     e->group.reset();
     SchedState hsr;
     CK(cudaMemcpy(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost), "sched D2H");
-    while (hsr.pending) {
-        // what the drain kernel's full stacks sent to the event queues: further waves
-        launch_wave_kernels(e, e->nsm * 2, 256);
-        k_plan<<<1, 32, 0, e->stream>>>(e->ctx, e->d_sched);
+    if (hsr.resume) {
+        // a run of the drain kernel alone, whose full stacks sent particles to the event queues: on in waves
+        gegs_status st = build_graph(e, e->run_grid, e->run_threads);
+        if (st != GEGS_OK) return st;
+        CK(cudaGraphLaunch(e->gexec[e->slot], e->stream), "graph launch");
         CK(cudaEventRecord(e->ev1, e->stream), "event");
         CK(cudaMemcpyAsync(&hsr, e->d_sched, sizeof hsr, cudaMemcpyDeviceToHost, e->stream), "sched D2H");
         CK(cudaStreamSynchronize(e->stream), "run sync");
@@ -1017,6 +1041,15 @@ static gegs_status run_finish(gegs_engine *e)
 extern "C" gegs_status gegs_run(gegs_engine *e, uint64_t hist_begin, uint64_t hist_end, const gegs_run_opts *opts)
 {
     return run_impl(e, hist_begin, hist_end, opts, false);
+}
+
+extern "C" gegs_status gegs_set_drain_stack(gegs_engine *e, uint32_t records)
+{
+    if (!e) return GEGS_ERR_ARG;
+    if (e->in_flight) { e->err = "a launched run has not been waited for (gegs_wait)"; return GEGS_ERR_ARG; }
+    const uint32_t cap = records && records < GX_DRAIN_CAP ? records : GX_DRAIN_CAP;
+    if (cap != e->ctx.drain_cap) { e->ctx.drain_cap = cap; e->ctx_gen++; }
+    return GEGS_OK;
 }
 
 extern "C" gegs_status gegs_launch(gegs_engine *e, uint64_t hist_begin, uint64_t hist_end, const gegs_run_opts *opts)

@@ -498,13 +498,14 @@ __global__ void k_plan_gated(const __grid_constant__ DevCtx C, SchedState *st)
     plan_wave(C, st);
 }
 
-// Ends a run: if the drain kernel ran, the queues it emptied are reset (their
-// peaks recorded) and the plan says whether it left anything (`pending`).
-__global__ void k_drain_end(const __grid_constant__ DevCtx C, SchedState *st)
+// Behind the drain kernel: if it ran, the queues it emptied are reset (their
+// peaks recorded) and the next wave is planned, for what it left in the event
+// queues. Returns whether it left anything.
+__device__ __forceinline__ uint32_t drain_end(const DevCtx &C, SchedState *st)
 {
     const uint32_t drained = *((volatile uint32_t *)&st->drain);
     __syncwarp();
-    if (drained == 0u) return;
+    if (drained == 0u) return 0u;
     if (threadIdx.x < 8u) {
         const int k = (int)threadIdx.x, q = k < 6 ? GX_Q_PCONT + 2 * k + (int)(*C.wave & 1u) : k == 6 ? ST_PHOTON : ST_ELECTRON;
         if (C.q.peak && C.q.count[q] > C.q.peak[q]) C.q.peak[q] = C.q.count[q];
@@ -517,7 +518,32 @@ __global__ void k_drain_end(const __grid_constant__ DevCtx C, SchedState *st)
         st->drain_hist = 0ull;
     }
     __syncwarp();
-    plan_wave(C, st);
+    const uint32_t left = plan_wave(C, st);
+    if (threadIdx.x == 0) st->resume = left;
+    return left;
+}
+
+__global__ void k_drain_end(const __grid_constant__ DevCtx C, SchedState *st)
+{
+    drain_end(C, st);
+}
+
+__global__ void k_drain_end_cond(const __grid_constant__ DevCtx C, SchedState *st, cudaGraphConditionalHandle handle)
+{
+    const uint32_t left = drain_end(C, st);
+    if (threadIdx.x == 0) cudaGraphSetConditional(handle, left);
+}
+
+// Enters the wave loop: plans its first wave, unless that has been done (drain_end).
+__global__ void k_plan_enter(const __grid_constant__ DevCtx C, SchedState *st, cudaGraphConditionalHandle handle)
+{
+    const uint32_t resume = *((volatile uint32_t *)&st->resume);
+    __syncwarp();
+    const uint32_t pending = resume ? 1u : plan_wave(C, st);
+    if (threadIdx.x == 0) {
+        st->resume = 0u;
+        cudaGraphSetConditional(handle, pending);
+    }
 }
 
 __global__ void k_plan_cond(const __grid_constant__ DevCtx C, SchedState *st, cudaGraphConditionalHandle handle)

@@ -137,11 +137,18 @@ gegs_status gegs_run(gegs_engine *e, uint64_t hist_begin, uint64_t hist_end, con
 /* gegs_run in two halves, for running several engines (plans) at once on one
  * GPU (no counterpart in the reference, which runs fields one after another):
  * gegs_launch queues the persistent-form run on the engine's stream and
- * returns; gegs_wait blocks until it is done and reports like gegs_run. Each
+ * returns (the whole run: the tally is complete for work behind it on the
+ * stream); gegs_wait blocks until it is done and reports like gegs_run. Each
  * engine has its own stream, so runs launched on several engines overlap on
  * the device. One launched run per engine at a time. */
 gegs_status gegs_launch(gegs_engine *e, uint64_t hist_begin, uint64_t hist_end, const gegs_run_opts *opts);
 gegs_status gegs_wait(gegs_engine *e);
+
+/* Testing aid (no counterpart in the reference): the drain kernel's stacks hold
+ * at most this many records of one particle type per warp (0 or more than 64:
+ * 64). A particle for which there is no room goes to the event queues, and the
+ * run goes on in waves: the tally is the same. */
+gegs_status gegs_set_drain_stack(gegs_engine *e, uint32_t records);
 
 /* Replace field `index` of the scene (its gantry cosine and sine, history range,
  * recycling count, jaw and leaf-end polygons) without uploading the phantom

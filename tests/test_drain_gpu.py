@@ -75,3 +75,96 @@ def test_a_gradient_replay_drains_and_leaves_the_forward_run_as_it_was(engine):
     # of the sum of its terms' sizes, some ten times the largest sum
     assert np.abs(first).max() > 0
     np.testing.assert_allclose(again, first, rtol=0, atol=1e-9 * np.abs(first).max())
+
+
+COUNTS = ("processed", "photon_steps", "electron_steps", "photon_steps_class", "electron_steps_class")
+
+
+def _split(job, n):
+    """The plan with every bremsstrahlung photon split n ways."""
+    job.physics = job.physics.copy()
+    job.physics["nbr_split"] = n
+    return job
+
+
+@pytest.mark.parametrize("records", [0, 34, 1])
+@pytest.mark.parametrize("scene,histories,split", [("slab", 4000, 1), ("slab", 20000, 1), ("slab", 3000, 100),
+                                                   ("head", 3000, 1), ("head", 20000, 1), ("head", 400, 100)])
+def test_full_stacks_go_on_in_waves(engine, oracle, scene, histories, split, records):
+    """Stacks of the drain kernel that overflow, because photons are split more
+    ways than a stack holds or because they are small: the tally is the oracle's,
+    and the counts are those of a run in waves."""
+    if scene == "slab":
+        job = _split(W.config2(histories=histories, nphsp=20000, n=30), split)
+    else:
+        job = _split(W.config3(histories=histories, nphsp=20000, dims=(48, 40, 24), angles=(0.0, 72.0, 200.0)), split)
+    sh = _load(engine, job)
+    waves = engine.run(0, histories, **WAVES)
+    engine.reset_tally()
+    engine.set_drain_stack(records)
+    try:
+        drained = engine.run(0, histories)
+    finally:
+        engine.set_drain_stack(0)
+    np.testing.assert_array_equal(engine.tally(), oracle.run(job.physics, sh, 0, histories)[0])
+    assert drained["error_bits"] == 0
+    if histories <= 4000:                              # the overflow is seen by the waves behind the drain kernel
+        assert (drained["waves"] > 2) == (split == 100 or records == 1)
+    for key in COUNTS:
+        assert drained[key] == waves[key], key
+
+
+def _tally_behind(engine, stream, nvox):
+    """The tally as a copy queued on `stream` behind the launched run reads it,
+    without waiting for the run."""
+    import torch
+
+    class View:
+        __cuda_array_interface__ = dict(shape=(nvox,), typestr="<i8", data=(engine.tally_device_ptr(), False), version=3)
+    with torch.cuda.stream(stream):
+        out = torch.as_tensor(View(), device="cuda").clone()
+    stream.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("histories", [3000, 20000])
+def test_a_launched_run_is_whole_for_the_stream(engine, oracle, histories):
+    """What full stacks left over is transported in the launch itself, not when
+    the host waits for it: alone, and in a launch of several plans."""
+    import torch
+    from gegs_b200.engine import Engine, launch_group
+    stream = torch.cuda.Stream()
+    job = _split(W.config2(histories=histories, nphsp=5000, n=30), 100)
+    sh = _load(engine, job)
+    ref, _ = oracle.run(job.physics, sh, 0, histories)
+    other = Engine(0)
+    _load(other, job)
+    engine.set_stream(stream)
+    try:
+        engine.launch(0, histories)
+        np.testing.assert_array_equal(_tally_behind(engine, stream, sh.nvox), ref)
+        assert engine.wait()["error_bits"] == 0
+        engine.reset_tally()
+        launch_group([engine, other], [(0, histories), (0, histories)])
+        np.testing.assert_array_equal(_tally_behind(engine, stream, sh.nvox), ref)
+        np.testing.assert_array_equal(_tally_behind(other, stream, sh.nvox), ref)
+        engine.wait()
+        other.wait()
+    finally:
+        engine.set_stream(None)
+        other.close()
+
+
+def test_a_gradient_replay_with_full_stacks(engine):
+    job = W.config4(histories=5000, nphsp=5000, dims=(40, 40, 20), nb=6, bixel=1.5)
+    sh = _load(engine, job)
+    g = np.random.default_rng(3).normal(size=sh.nvox)
+    for histories in (2000, 5000):
+        want = engine.backward(0, histories, g)
+        engine.set_drain_stack(20)
+        try:
+            got = engine.backward(0, histories, g)
+        finally:
+            engine.set_drain_stack(0)
+        # double sums in another order, as above
+        np.testing.assert_allclose(got, want, rtol=0, atol=1e-9 * np.abs(want).max())
