@@ -66,6 +66,11 @@ static_assert(sizeof(gegs_field) % 16 == 0, "field record size");
 #define GX_DT_I 6
 #define GX_DT_N 14
 #define GX_DRAIN_CAP 64
+// Turns (transport steps of its lanes, and interactions) that a warp of the
+// drain kernel takes before it hands what it still has to the waves, whose
+// number is limited: some ten times the longest track known, tens of thousands
+// of steps along a jaw face, and 0.2 s of such steps.
+#define GX_DRAIN_TURNS (1u << 17)
 #define GX_LOOP_CAP 1000
 // The reference's step constants are double literals (EGSnrc_Parameters.h:91-92,
 // CUDA_EGS.h:34): a step that adds EPSTEP, and a comparison with EPSGMFP or
@@ -207,6 +212,7 @@ struct DevCtx {
     Part *drain_part;       // the drain kernel's stacks: [warp][GX_DT_N][GX_DRAIN_CAP]
     EStatePk *drain_estate; // [warp][3][GX_DRAIN_CAP], step states of the electrons on them
     uint32_t drain_cap;     // records of one type that a stack takes: GX_DRAIN_CAP, or fewer (gegs_set_drain_stack)
+    uint32_t drain_turns;   // GX_DRAIN_TURNS, or fewer (gegs_set_drain_turns)
     unsigned long long *timeline;   // [timeline_waves][16][2] first start / last end (ns) per kernel; null: off
     uint32_t timeline_waves;
     QueueSet q;

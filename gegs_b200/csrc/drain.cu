@@ -10,7 +10,9 @@
 // side, and what they make goes back on its own stacks, so that a warp still
 // executes one kind of work at a time but waits for nobody. Warps that run low
 // claim more from the event queues, or histories not yet started. There are no
-// barriers and no waits: a warp ends when its stacks and the queues are empty.
+// barriers and no waits: a warp ends when its stacks and the queues are empty, or
+// after so many turns (C.drain_turns) that one of its particles may never end;
+// then all it has goes to the event queues, and the waves' budget ends the run.
 // A stack that is full sends the particle to the event queues, and the run goes
 // on in waves behind the drain kernel, in the same launch (add_wave_loop). With
 // the tables' own single bremsstrahlung photon no plan has been seen to need
@@ -31,6 +33,7 @@ constexpr int kWarps = kDrainThreads / 32;
 
 struct DrainWarp {
     uint32_t cnt[GX_DT_N];     // records on each stack
+    uint32_t turns;            // turns that are left to the warp
     uint32_t taken[GX_NSTAGE]; // particles taken per stage
     uint32_t steps[2];         // photon, electron
     uint32_t head_steps[4];    // photon jaws, MLC, electron jaws, MLC
@@ -131,6 +134,8 @@ __device__ __noinline__ void drain_transport()
     float gle = 0.0f;
     bool active = false;
     uint32_t steps = 0, taken = 0;
+    __syncwarp();
+    uint32_t turns = w.turns;
     for (;;) {
         __syncwarp();
         uint32_t act = __ballot_sync(0xffffffffu, active);
@@ -159,10 +164,11 @@ __device__ __noinline__ void drain_transport()
             act = __ballot_sync(0xffffffffu, active);
         }
         if (act == 0u) break;
-        bool leave = false;
+        bool leave = turns == 0u;
+        if (!leave) turns--;
         if (__popc(act) <= 8) {
             const uint32_t other = lane < GX_DT_N && (int)lane != T ? w.cnt[lane] : 0u;
-            leave = __any_sync(0xffffffffu, other >= 16u);
+            leave |= __any_sync(0xffffffffu, other >= 16u);
         }
         const bool in_class = in_geom_class<G>(p);     // before the step, which may leave it
         int code = STEP_ON, shared = -1;
@@ -202,9 +208,21 @@ __device__ __noinline__ void drain_transport()
     steps = __reduce_add_sync(0xffffffffu, steps);
     taken = __reduce_add_sync(0xffffffffu, taken);
     if (lane == 0) {
+        w.turns = turns;
         w.taken[Q] += taken;
         w.steps[ELEC ? 1 : 0] += steps;
         if (cls < 2) w.head_steps[(ELEC ? 2 : 0) + cls] += steps;
+    }
+}
+
+// The transports of the jaws and the MLC; a beam line of the phantom alone has no such particle.
+template <bool HEAD, bool ELEC, int G>
+__device__ __forceinline__ void drain_head()
+{
+    if constexpr (HEAD) drain_transport<ELEC, G>();
+    else if ((threadIdx.x & 31u) == 0u) {
+        warp_of().cnt[(ELEC ? GX_DT_E : GX_DT_P) + G - GX_GEOM_JAWS] = 0u;
+        atomicOr(g_ctx.err, GX_ERR_MODULE);
     }
 }
 
@@ -291,6 +309,25 @@ __device__ __noinline__ bool claim(SchedState *st, uint32_t par, uint32_t per, i
     return false;
 }
 
+// All that is on the warp's stacks goes to the event queues.
+__device__ __noinline__ void spill_stacks()
+{
+    const DevCtx &C = g_ctx;
+    DrainWarp &w = warp_of();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (int type = 0; type < GX_DT_N; type++) {
+        const uint32_t n = min(w.cnt[type], C.drain_cap);
+        for (uint32_t i = lane; i < n; i += 32) {
+            const Part p = load_part(slot_part(C, type, i));
+            const bool state = type >= GX_DT_E && type < GX_DT_I && p.status == kGoesOn;
+            spill(C, type, p, state ? *slot_estate(C, type, i) : fresh_estate());
+        }
+    }
+    __syncwarp();
+    if (lane < GX_DT_N) w.cnt[lane] = 0u;
+    __syncwarp();
+}
+
 template <bool HEAD>
 __global__ void __launch_bounds__(kDrainThreads, 6) k_drain(const __grid_constant__ DevCtx ctx, SchedState *st)
 {
@@ -305,6 +342,7 @@ __global__ void __launch_bounds__(kDrainThreads, 6) k_drain(const __grid_constan
     const uint32_t lane = threadIdx.x & 31u, par = *C.wave & 1u;
     for (uint32_t i = lane; i < sizeof(DrainWarp) / 4; i += 32) reinterpret_cast<uint32_t *>(&w)[i] = 0u;
     __syncwarp();
+    if (lane == 0) w.turns = C.drain_turns;
     // an even share of what there is, so that a small run spreads over the SMs, up to a warp's width
     unsigned long long total = st->end - st->next;
     for (int k = 0; k < kPools; k++) {
@@ -323,9 +361,16 @@ __global__ void __launch_bounds__(kDrainThreads, 6) k_drain(const __grid_constan
         }
         const uint32_t best = __reduce_max_sync(0xffffffffu, c * 32u + lane);
         const uint32_t all = __reduce_add_sync(0xffffffffu, c);
+        const bool over = w.turns == 0u;
         __syncwarp();
+        if (over) {
+            if (all) spill_stacks();
+            if (pool < kPools && claim(st, par, per, pool)) continue;
+            break;
+        }
         if (all < per && pool < kPools && claim(st, par, per, pool)) continue;
         if (all == 0u) break;
+        if (lane == 0) w.turns--;
         switch (best & 31u) {
         case GX_DT_P + 2: drain_transport<false, GX_GEOM_PHANTOM>(); break;
         case GX_DT_E + 2: drain_transport<true, GX_GEOM_PHANTOM>(); break;
@@ -337,10 +382,10 @@ __global__ void __launch_bounds__(kDrainThreads, 6) k_drain(const __grid_constan
         case GX_DT_I + 5: drain_interaction<ST_BREMS>(); break;
         case GX_DT_I + 6: drain_interaction<ST_BHABHA>(); break;
         case GX_DT_I + 7: drain_interaction<ST_ANNIH>(); break;
-        case GX_DT_P + 1: if (HEAD) drain_transport<false, GX_GEOM_MLC>(); break;
-        case GX_DT_E + 1: if (HEAD) drain_transport<true, GX_GEOM_MLC>(); break;
-        case GX_DT_P + 0: if (HEAD) drain_transport<false, GX_GEOM_JAWS>(); break;
-        case GX_DT_E + 0: if (HEAD) drain_transport<true, GX_GEOM_JAWS>(); break;
+        case GX_DT_P + 1: drain_head<HEAD, false, GX_GEOM_MLC>(); break;
+        case GX_DT_E + 1: drain_head<HEAD, true, GX_GEOM_MLC>(); break;
+        case GX_DT_P + 0: drain_head<HEAD, false, GX_GEOM_JAWS>(); break;
+        case GX_DT_E + 0: drain_head<HEAD, true, GX_GEOM_JAWS>(); break;
         }
     }
     if (lane < GX_NSTAGE && w.taken[lane]) atomicAdd(&C.stats[lane], (unsigned long long)w.taken[lane]);

@@ -223,6 +223,7 @@ gegs_status gegs_create(int device, gegs_engine **out)
     if (c != cudaSuccess) { gegs_status s = cuda_fail(e, c, "cudaSetDevice"); *out = e; return s; }
     cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device);
     e->ctx.drain_cap = GX_DRAIN_CAP;
+    e->ctx.drain_turns = GX_DRAIN_TURNS;
     CK(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "stream");
     e->stream = e->own_stream;
     CK(cudaEventCreate(&e->ev0), "event");
@@ -1049,6 +1050,15 @@ extern "C" gegs_status gegs_set_drain_stack(gegs_engine *e, uint32_t records)
     if (e->in_flight) { e->err = "a launched run has not been waited for (gegs_wait)"; return GEGS_ERR_ARG; }
     const uint32_t cap = records && records < GX_DRAIN_CAP ? records : GX_DRAIN_CAP;
     if (cap != e->ctx.drain_cap) { e->ctx.drain_cap = cap; e->ctx_gen++; }
+    return GEGS_OK;
+}
+
+extern "C" gegs_status gegs_set_drain_turns(gegs_engine *e, uint32_t turns)
+{
+    if (!e) return GEGS_ERR_ARG;
+    if (e->in_flight) { e->err = "a launched run has not been waited for (gegs_wait)"; return GEGS_ERR_ARG; }
+    const uint32_t most = turns && turns < GX_DRAIN_TURNS ? turns : GX_DRAIN_TURNS;
+    if (most != e->ctx.drain_turns) { e->ctx.drain_turns = most; e->ctx_gen++; }
     return GEGS_OK;
 }
 

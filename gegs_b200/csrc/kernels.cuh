@@ -26,9 +26,10 @@
 #define GX_TAIL_DIV 256u
 #endif
 
-// steps one particle may take inside one consumer launch before it is dropped
-// and GX_ERR_STEP_BUDGET is raised (guards the persistent loops against a
-// particle that stops making progress)
+// Steps one particle may take inside one launch of the plain form before it is
+// dropped and GX_ERR_STEP_BUDGET is raised: against a particle that stops making
+// progress. (In waves such a particle goes from budget to budget until the run's
+// waves are used up, and the drain kernel hands it to the waves.)
 #define GX_STEP_BUDGET 4000000u
 
 // The last of the `blocks` that took part in draining a queue resets it.

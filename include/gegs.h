@@ -150,6 +150,14 @@ gegs_status gegs_wait(gegs_engine *e);
  * run goes on in waves: the tally is the same. */
 gegs_status gegs_set_drain_stack(gegs_engine *e, uint32_t records);
 
+/* Testing aid (no counterpart in the reference): a warp of the drain kernel
+ * takes at most this many turns (a step of its particles, or one round of
+ * interactions) before all that it still has goes on in waves, so that a
+ * particle that stops making progress ends the run with GEGS_ERR_STEP_BUDGET
+ * once the waves are used up (0 or more than 131072: 131072). The tally is the
+ * same. */
+gegs_status gegs_set_drain_turns(gegs_engine *e, uint32_t turns);
+
 /* Replace field `index` of the scene (its gantry cosine and sine, history range,
  * recycling count, jaw and leaf-end polygons) without uploading the phantom
  * again; the tally is kept. The reference sets a field up before each field's

@@ -168,3 +168,31 @@ def test_a_gradient_replay_with_full_stacks(engine):
             engine.set_drain_stack(0)
         # double sums in another order, as above
         np.testing.assert_allclose(got, want, rtol=0, atol=1e-9 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("turns", [1, 2, 40, 1000])
+@pytest.mark.parametrize("scene,histories", [("slab", 1), ("slab", 4000), ("slab", 20000), ("head", 3553), ("head", 20000)])
+def test_a_warp_out_of_turns_hands_its_particles_to_the_waves(engine, oracle, scene, histories, turns):
+    """The drain kernel ends after a given number of turns whatever its particles
+    do, also before a warp has claimed anything; the rest of the run is the
+    waves', with the oracle's tally and the waves' counts."""
+    if scene == "slab":
+        job = W.config2(histories=histories, nphsp=20000, n=30)
+    else:
+        job = W.config3(histories=histories, nphsp=20000, dims=(48, 40, 24), angles=(0.0, 72.0, 200.0))
+    sh = _load(engine, job)
+    waves = engine.run(0, histories, **WAVES)
+    ref, _ = oracle.run(job.physics, sh, 0, histories)
+    engine.set_drain_turns(turns)
+    try:
+        for kw in ({}, dict(batch=600)):
+            engine.reset_tally()
+            drained = engine.run(0, histories, **kw)
+            np.testing.assert_array_equal(engine.tally(), ref)
+            assert drained["error_bits"] == 0
+            for key in COUNTS:
+                assert drained[key] == waves[key], key
+            if histories <= 4000 and not kw and turns <= (2 if histories == 1 else 40):
+                assert drained["waves"] > 2
+    finally:
+        engine.set_drain_turns(0)
