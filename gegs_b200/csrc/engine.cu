@@ -864,7 +864,7 @@ static gegs_status run_impl(gegs_engine *e, uint64_t hist_begin, uint64_t hist_e
     const int grid = R.grid, threads = R.threads;
     const uint32_t max_waves = R.max_waves;
     for (int k = 0; k < 16; k++) { e->last.stage_ms[k] = 0.0; e->last.stage_launches[k] = 0; }
-    if (o.mode == GEGS_MODE_PERSISTENT && !launch_only && hist_end - hist_begin <= R.drain_below) {
+    if (o.mode == GEGS_MODE_PERSISTENT && !launch_only && R.drain_below && hist_end - hist_begin <= R.drain_below) {
         // the whole run goes to the drain kernel: no wave loop, so no graph (but for
         // what its stacks could not hold, run_finish; a launched run is over when
         // its stream is, so it takes the graph)

@@ -196,3 +196,17 @@ def test_a_warp_out_of_turns_hands_its_particles_to_the_waves(engine, oracle, sc
                 assert drained["waves"] > 2
     finally:
         engine.set_drain_turns(0)
+
+
+@pytest.mark.parametrize("kw", [{}, dict(photon_budget=16), dict(pipelined=False), dict(max_waves=10), dict(batch=1),
+                                dict(mode=1), dict(mode=2)])
+def test_an_empty_range_is_a_run_of_nothing(kw):
+    """The first run of an engine, with the drain kernel and without."""
+    from gegs_b200.engine import Engine
+    e = Engine(0)
+    sh = _load(e, W.config1(histories=100, n=10, voxel=3.0))
+    for h in (0, 50):
+        st = e.run(h, h, **kw)
+        assert st["error_bits"] == 0 and sum(st["processed"]) == 0
+    assert not e.tally().any()
+    e.close()
