@@ -761,18 +761,27 @@ static uint32_t drain_threshold(const gegs_run_opts &o, uint32_t batch)
     return most < batch / 2u ? most : batch / 2u;
 }
 
-static gegs_status ensure_drain(gegs_engine *e)
+// The drain kernel's stacks; false if there is no memory for them (the run then
+// goes on in waves to its end).
+static bool ensure_drain(gegs_engine *e)
 {
     const int grid = e->nsm * drain_blocks_per_sm(e->has_head);
-    if (e->drain_grid == grid) return GEGS_OK;
+    if (e->drain_grid == grid) return true;
     const size_t warps = (size_t)grid * (kDrainThreads / 32);
-    CK(realloc_dev(&e->d_drain_part, warps * GX_DT_N * GX_DRAIN_CAP), "drain stacks");
-    CK(realloc_dev(&e->d_drain_estate, warps * 3 * GX_DRAIN_CAP), "drain stacks");
-    e->drain_grid = grid;
+    if (e->drain_grid) e->ctx_gen++;            // graphs with the old stacks
+    e->drain_grid = 0;
+    if (realloc_dev(&e->d_drain_part, warps * GX_DT_N * GX_DRAIN_CAP) == cudaSuccess &&
+        realloc_dev(&e->d_drain_estate, warps * 3 * GX_DRAIN_CAP) == cudaSuccess) {
+        e->drain_grid = grid;
+        e->ctx_gen++;
+    } else {
+        cudaGetLastError();
+        cudaFree(e->d_drain_part);
+        e->d_drain_part = nullptr;
+    }
     e->ctx.drain_part = e->d_drain_part;
     e->ctx.drain_estate = e->d_drain_estate;
-    e->ctx_gen++;
-    return GEGS_OK;
+    return e->drain_grid != 0;
 }
 
 // Everything a run needs before its kernels: options resolved into the
@@ -817,8 +826,8 @@ static gegs_status prepare_run(gegs_engine *e, uint64_t hist_begin, uint64_t his
     }
     gegs_status st = ensure_queues(e, batch, o.queue_cap);
     if (st != GEGS_OK) return st;
-    const uint32_t drain_below = drain_threshold(o, batch);
-    if (drain_below) { st = ensure_drain(e); if (st != GEGS_OK) return st; }
+    uint32_t drain_below = drain_threshold(o, batch);
+    if (drain_below && !ensure_drain(e)) drain_below = 0u;
     fill_queue_ctx(e);
 
     SchedState hs = {};

@@ -210,3 +210,29 @@ def test_an_empty_range_is_a_run_of_nothing(kw):
         assert st["error_bits"] == 0 and sum(st["processed"]) == 0
     assert not e.tally().any()
     e.close()
+
+
+def test_without_memory_for_the_stacks_a_run_goes_in_waves(oracle):
+    """The queues are there already, and less memory is free than the stacks take (225 MB)."""
+    import torch
+    from gegs_b200.engine import Engine
+    job = W.config3(histories=3000, nphsp=5000, dims=(40, 40, 20))
+    loaded, e = Engine(0), Engine(0)
+    _load(loaded, job)
+    loaded.run(0, 3000)                               # the kernels' own memory
+    loaded.close()
+    sh = _load(e, job)
+    ref, _ = oracle.run(job.physics, sh, 0, 3000)
+    opts = dict(batch=1 << 16)
+    e.run(0, 3000, **opts, **WAVES)
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info(0)[0] - (180 << 20), dtype=torch.uint8, device="cuda")
+    for last in (False, True):
+        for _ in range(2):
+            e.reset_tally()
+            st = e.run(0, 3000, **opts)
+            np.testing.assert_array_equal(e.tally(), ref)
+            assert (st["waves"] == 2) == last
+        held = None
+        torch.cuda.empty_cache()
+    e.close()
