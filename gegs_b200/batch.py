@@ -26,13 +26,13 @@ def choose_options(histories, share_bytes):
     """In-flight batch: a power of two near a quarter of the histories (all of them
     up to 1M: every injection costs a plan another build-up and decline of short
     waves), at most what `share_bytes` of queue memory holds, between 64K and 4M;
-    the default step budgets, with which a plan's end is left to the drain
+    the default step budgets; and a plan's end is left to the drain
     kernel. Six plans of 0.2M to 0.7M histories in one launch: 86.5 to 62.6 ms."""
     near = max(histories / 4, min(histories, 1 << 20), 1)
     want = max(1 << 16, min(1 << 22, 1 << int(np.ceil(np.log2(near)))))
     cap = 1 << int(np.floor(np.log2(max(share_bytes / QUEUE_BYTES_PER_PARTICLE, 1 << 16))))
     b = int(min(want, cap))
-    return dict(batch=b, photon_budget=0, electron_budget=0, refill_below=b // 4)
+    return dict(batch=b, photon_budget=0, electron_budget=0, refill_below=b // 4, drain=True)
 
 
 # The autotuner's search space: each dimension's alternatives to the current
@@ -45,6 +45,7 @@ TUNE_DIMENSIONS = {
     "refill_below": lambda o: [max(o["batch"] // 50, 1), max(o["batch"] // 2, 1)],
     "stage_tables": lambda o: [not o.get("stage_tables", False)],
     "pipelined": lambda o: [not o.get("pipelined", True)],
+    "drain": lambda o: [not o["drain"]],
 }
 
 
@@ -55,8 +56,9 @@ def autotune(engine, job, sample=None, candidates=None, dimensions=None, rounds=
     coordinate descent: starting from choose_options, each dimension of
     TUNE_DIMENSIONS (in-flight batch, grid blocks per SM, photon and electron
     step budgets, refill threshold, whether the photon tables are staged in
-    shared memory, GEGS_RUN_STAGE_TABLES, and whether a wave's two transport
-    phases run at once, GEGS_RUN_SERIAL_WAVES) tries its alternatives with the
+    shared memory, GEGS_RUN_STAGE_TABLES, whether a wave's two transport
+    phases run at once, GEGS_RUN_SERIAL_WAVES, and whether the plan's end goes
+    to the drain kernel, GEGS_RUN_DRAIN) tries its alternatives with the
     others fixed and keeps any that is faster; `rounds` passes over the
     dimensions.
     Every trial first runs a quarter sample untimed (graph build, queue
@@ -82,6 +84,8 @@ def autotune(engine, job, sample=None, candidates=None, dimensions=None, rounds=
         return best, best_t, trials
     best = dict(start) if start is not None else choose_options(job.histories, 64e9)
     best.setdefault("blocks_per_sm", 0)
+    # said by name: left open, a trial's budget or wave order would switch it off as well
+    best.setdefault("drain", not (best.get("photon_budget") or best.get("electron_budget")) and best.get("pipelined", True))
     best_t = timed(best)
     for _ in range(rounds):
         for dim, alts in (dimensions or TUNE_DIMENSIONS).items():

@@ -750,13 +750,14 @@ static gegs_status run_finish(gegs_engine *e);
 // water, 10 000 histories 3.62 / 2.19 / 2.16 / 2.14 / 3.83 (there all of them
 // go to it); slab, 200 000: 11.7 / 9.8 / 9.5 / 10.1 / 10.5; CT head 5-field
 // plan, 1M: 36.1 / 33.4 / 33.5 / 33.3 / 34.1, 16M: 258.2 / 255.5 / 255.6 /
-// 256.0 / 255.9. Never for a run that says how it is to be divided into waves
-// (step or wave budgets, serial waves) or that tests its queues, and at most
-// half the in-flight batch, so that a small batch still runs as asked.
+// 256.0 / 255.9. Unless asked for, not for a run that says how it is to be
+// divided into waves (step or wave budgets, serial waves) or that tests its
+// queues; and at most half the in-flight batch, so that a small batch still runs
+// as asked.
 static uint32_t drain_threshold(const gegs_run_opts &o, uint32_t batch)
 {
-    if (o.mode != GEGS_MODE_PERSISTENT || (o.flags & GEGS_RUN_SERIAL_WAVES) || o.step_budget || o.max_waves || o.queue_cap)
-        return 0u;
+    const bool in_waves = (o.flags & GEGS_RUN_SERIAL_WAVES) || o.step_budget || o.max_waves || o.queue_cap;
+    if (o.mode != GEGS_MODE_PERSISTENT || (o.flags & GEGS_RUN_NO_DRAIN) || (in_waves && !(o.flags & GEGS_RUN_DRAIN))) return 0u;
     const uint32_t most = 4000u;
     return most < batch / 2u ? most : batch / 2u;
 }

@@ -42,6 +42,8 @@ class RunOpts(C.Structure):
 
 RUN_STAGE_TABLES = 1
 RUN_SERIAL_WAVES = 2
+RUN_DRAIN = 4
+RUN_NO_DRAIN = 8
 
 
 # gegs_probe_state (include/gegs.h)
@@ -122,10 +124,12 @@ def check_physics(block: np.ndarray):
         raise GegsError(st, msg.value.decode())
 
 
-def _flags(stage_tables, pipelined):
+def _flags(stage_tables, pipelined, drain):
     """gegs_run_opts.flags; `pipelined` (the default, persistent form): both
-    transport phases of a wave at once, then all interactions."""
-    return (RUN_STAGE_TABLES if stage_tables else 0) | (0 if pipelined else RUN_SERIAL_WAVES)
+    transport phases of a wave at once, then all interactions; `drain`: whether
+    a run's last particles go to the drain kernel (None: the library's rule)."""
+    return ((RUN_STAGE_TABLES if stage_tables else 0) | (0 if pipelined else RUN_SERIAL_WAVES) |
+            (0 if drain is None else RUN_DRAIN if drain else RUN_NO_DRAIN))
 
 
 class Engine:
@@ -190,18 +194,19 @@ class Engine:
 
     def run(self, h0: int, h1: int, mode: int = MODE_PERSISTENT, batch: int = 0, blocks_per_sm: int = 0,
             threads: int = 0, max_waves: int = 0, photon_budget: int = 0, electron_budget: int = 0,
-            refill_below: int = 0, queue_cap: int = 0, stage_tables: bool = False, pipelined: bool = True):
+            refill_below: int = 0, queue_cap: int = 0, stage_tables: bool = False, pipelined: bool = True,
+            drain: bool | None = None):
         o = RunOpts(mode, batch, blocks_per_sm, threads, max_waves, (photon_budget & 0xFFFF) | (electron_budget << 16),
-                    refill_below, queue_cap, _flags(stage_tables, pipelined))
+                    refill_below, queue_cap, _flags(stage_tables, pipelined, drain))
         self._check(self.L.gegs_run(self.h, h0, h1, C.byref(o)))
         return self.stats()
 
     def launch(self, h0: int, h1: int, batch: int = 0, blocks_per_sm: int = 0, threads: int = 0,
                photon_budget: int = 0, electron_budget: int = 0, refill_below: int = 0, stage_tables: bool = False,
-               pipelined: bool = True):
+               pipelined: bool = True, drain: bool | None = None):
         """Queue a persistent-form run and return at once (see wait())."""
         o = RunOpts(MODE_PERSISTENT, batch, blocks_per_sm, threads, 0, (photon_budget & 0xFFFF) | (electron_budget << 16),
-                    refill_below, 0, _flags(stage_tables, pipelined))
+                    refill_below, 0, _flags(stage_tables, pipelined, drain))
         self._check(self.L.gegs_launch(self.h, h0, h1, C.byref(o)))
 
     def wait(self):
@@ -248,7 +253,7 @@ class Engine:
     def _opts(o):
         return RunOpts(MODE_PERSISTENT, o.get("batch", 0), o.get("blocks_per_sm", 0), o.get("threads", 0), 0,
                        (o.get("photon_budget", 0) & 0xFFFF) | (o.get("electron_budget", 0) << 16),
-                       o.get("refill_below", 0), 0, _flags(o.get("stage_tables"), o.get("pipelined", True)))
+                       o.get("refill_below", 0), 0, _flags(o.get("stage_tables"), o.get("pipelined", True), o.get("drain")))
 
 
     def reset_tally(self):

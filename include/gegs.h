@@ -79,11 +79,17 @@ typedef struct gegs_run_opts {
                                   electron interactions in turn, instead of both transports at once and
                                   then all interactions (the default, pipelined: a particle made by an
                                   interaction is transported in the next wave; 1.9 % faster on the CT
-                                  5-field plan). The tally is the same either way */
+                                  5-field plan). The tally is the same either way;
+                                  GEGS_RUN_DRAIN, GEGS_RUN_NO_DRAIN (persistent form): whether the last 4000
+                                  particles and histories go to the drain kernel or on in waves. With neither,
+                                  they go on in waves where the run sets step_budget, max_waves or queue_cap
+                                  or runs serial waves, and else to the drain kernel. The tally is the same */
 } gegs_run_opts;
 
 #define GEGS_RUN_STAGE_TABLES 1u
 #define GEGS_RUN_SERIAL_WAVES 2u
+#define GEGS_RUN_DRAIN 4u
+#define GEGS_RUN_NO_DRAIN 8u
 
 #define GEGS_NQUEUES 25
 

@@ -102,3 +102,36 @@ def test_autotuned_plans_keep_their_tallies(oracle):
     ref, _ = oracle.run(job.physics, job.scene(), 0, job.histories)
     np.testing.assert_array_equal(pb.tallies()[0], ref)
     pb.close()
+
+
+class _Timed:
+    """An engine whose runs take a made-up time: every other one is the fastest so far."""
+    def __init__(self):
+        self.runs = []
+
+    def run(self, h0, h1, **o):
+        self.runs.append(o)
+        return dict(device_ms=1000.0 - len(self.runs) if len(self.runs) % 4 else 2000.0)
+
+    def reset_tally(self):
+        pass
+
+
+@pytest.mark.parametrize("start", [None, dict(batch=1 << 17), dict(batch=1 << 17, photon_budget=8)])
+def test_the_autotuner_changes_one_thing_at_a_time(start):
+    """Whether a plan's end goes to the drain kernel is a dimension of its own:
+    a trial of a step budget or of the wave order says so by name, and does not
+    switch it by the way."""
+    from gegs_b200.batch import autotune
+    job = W.config1(histories=5000, n=8, voxel=3.0)
+    e = _Timed()
+    best, best_ms, trials = autotune(e, job, start=start)
+    assert {o["drain"] for o, _ in trials} == {True, False}
+    assert trials[0][0]["drain"] == (start is None or "photon_budget" not in start)
+    base, t0 = trials[0]
+    for o, t in trials[1:]:
+        d = {k for k in set(o) | set(base) if o.get(k) != base.get(k)}
+        assert len(d - {"refill_below"}) == 1 or d == {"refill_below"}, (base, o)
+        if t < t0:
+            base, t0 = o, t
+    assert (best, best_ms) == (base, t0)

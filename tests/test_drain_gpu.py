@@ -236,3 +236,46 @@ def test_without_memory_for_the_stacks_a_run_goes_in_waves(oracle):
         held = None
         torch.cuda.empty_cache()
     e.close()
+
+
+@pytest.mark.parametrize("kw", [dict(photon_budget=2, electron_budget=1), dict(pipelined=False), dict(max_waves=1000),
+                                dict(pipelined=False, photon_budget=3, stage_tables=True), {}])
+def test_drain_and_no_drain_by_name(engine, oracle, kw):
+    """Beside every option that otherwise decides it, both ways, alone and launched."""
+    from gegs_b200.engine import launch_group
+    for histories in (3000, 9000):
+        job = W.config3(histories=histories, nphsp=20000, dims=(48, 40, 24), angles=(0.0, 72.0, 200.0))
+        sh = _load(engine, job)
+        ref, _ = oracle.run(job.physics, sh, 0, histories)
+        small = histories <= 4000
+        for drain in (True, False):
+            engine.reset_tally()
+            st = engine.run(0, histories, drain=drain, **kw)
+            np.testing.assert_array_equal(engine.tally(), ref)
+            assert (st["waves"] == 2) == (drain and small)
+            if "max_waves" in kw:
+                continue                               # not an option of launched runs
+            engine.reset_tally()
+            engine.launch(0, histories, drain=drain, **kw)
+            assert (engine.wait()["waves"] == 2) == (drain and small)
+            np.testing.assert_array_equal(engine.tally(), ref)
+            engine.reset_tally()
+            launch_group([engine], [(0, histories)], [dict(drain=drain, **kw)])
+            assert (engine.wait()["waves"] == 2) == (drain and small)
+            np.testing.assert_array_equal(engine.tally(), ref)
+
+
+def test_a_particle_that_does_not_end_uses_up_the_waves(engine):
+    """What the drain kernel hands over comes under the wave budget: with two
+    turns a warp and six waves, an ordinary plan is such a one."""
+    from gegs_b200.engine import GegsError
+    job = W.config2(histories=2000, nphsp=2000, n=30)
+    _load(engine, job)
+    engine.set_drain_turns(2)
+    try:
+        with pytest.raises(GegsError) as err:
+            engine.run(0, 2000, max_waves=6, drain=True)
+    finally:
+        engine.set_drain_turns(0)
+    assert err.value.status == 6                      # GEGS_ERR_STEP_BUDGET
+    assert engine.stats()["waves"] == 6
