@@ -20,25 +20,37 @@ import numpy as np
 from .engine import Engine, launch_group
 
 QUEUE_BYTES_PER_PARTICLE = 5.2e3      # event queues + electron step state per particle of `batch`
+DRAIN_BYTES = 2.3e8                   # an engine's drain kernel stacks
+LEAST_BATCH, MOST_BATCH = 1 << 16, 1 << 22
+
+
+def memory_limits(share_bytes):
+    """What `share_bytes` of device memory hold: the largest in-flight batch (a
+    power of two, at least the smallest one), and whether there is room for the
+    drain kernel's stacks beside the smallest batch's queues."""
+    drain = share_bytes >= DRAIN_BYTES + LEAST_BATCH * QUEUE_BYTES_PER_PARTICLE
+    fit = (share_bytes - (DRAIN_BYTES if drain else 0.0)) / QUEUE_BYTES_PER_PARTICLE
+    return 1 << int(np.floor(np.log2(max(fit, LEAST_BATCH)))), drain
 
 
 def choose_options(histories, share_bytes):
     """In-flight batch: a power of two near a quarter of the histories (all of them
     up to 1M: every injection costs a plan another build-up and decline of short
-    waves), at most what `share_bytes` of queue memory holds, between 64K and 4M;
-    the default step budgets; and a plan's end is left to the drain
-    kernel. Six plans of 0.2M to 0.7M histories in one launch: 86.5 to 62.6 ms."""
+    waves), at most what `share_bytes` hold, between 64K and 4M; the default step
+    budgets; and a plan's end is left to the drain kernel, where the share has
+    room for its stacks. Six plans of 0.2M to 0.7M histories in one launch: 86.5
+    to 62.6 ms."""
     near = max(histories / 4, min(histories, 1 << 20), 1)
-    want = max(1 << 16, min(1 << 22, 1 << int(np.ceil(np.log2(near)))))
-    cap = 1 << int(np.floor(np.log2(max(share_bytes / QUEUE_BYTES_PER_PARTICLE, 1 << 16))))
+    want = max(LEAST_BATCH, min(MOST_BATCH, 1 << int(np.ceil(np.log2(near)))))
+    cap, drain = memory_limits(share_bytes)
     b = int(min(want, cap))
-    return dict(batch=b, photon_budget=0, electron_budget=0, refill_below=b // 4, drain=True)
+    return dict(batch=b, photon_budget=0, electron_budget=0, refill_below=b // 4, drain=drain)
 
 
 # The autotuner's search space: each dimension's alternatives to the current
 # setting (coordinate descent from the defaults of choose_options).
 TUNE_DIMENSIONS = {
-    "batch": lambda o: [max(o["batch"] // 2, 1 << 16), min(o["batch"] * 2, 1 << 22)],
+    "batch": lambda o: [max(o["batch"] // 2, LEAST_BATCH), min(o["batch"] * 2, MOST_BATCH)],
     "blocks_per_sm": lambda o: [4, 8],
     "photon_budget": lambda o: [16, 64],
     "electron_budget": lambda o: [4, 16],
@@ -106,8 +118,9 @@ class PlanBatch:
     def __init__(self, jobs, device=0, memory_budget_gb=40.0, tune_sample=0, tune_fraction=0.0):
         """One engine per plan. With tune_sample (histories) or tune_fraction
         (of each plan's histories, at least 1e5), each plan's run options come
-        from the coordinate-descent autotuner, kept within the plan's share of
-        the queue-memory budget."""
+        from the coordinate-descent autotuner. Event queues and drain stacks stay
+        within the plan's share of the memory budget (but for the smallest batch's
+        queues, 340 MB, which every plan has)."""
         self.jobs = list(jobs)
         self.engines, self.options, self.tune_ms = [], [], []
         total = float(sum(j.histories for j in self.jobs)) or 1.0
@@ -119,9 +132,11 @@ class PlanBatch:
             opts = choose_options(job.histories, share)
             sample = tune_sample or (int(max(1e5, tune_fraction * job.histories)) if tune_fraction > 0 else 0)
             if sample:
-                cap = 1 << int(np.floor(np.log2(max(share / QUEUE_BYTES_PER_PARTICLE, 1 << 16))))  # what the share holds
+                cap, drain = memory_limits(share)
                 dims = dict(TUNE_DIMENSIONS)
-                dims["batch"] = lambda o: [b for b in (max(o["batch"] // 2, 1 << 16), o["batch"] * 2) if b <= cap]
+                dims["batch"] = lambda o: [b for b in (max(o["batch"] // 2, LEAST_BATCH), o["batch"] * 2) if b <= cap]
+                if not drain:
+                    del dims["drain"]
                 opts, t, _ = autotune(e, job, sample=sample, dimensions=dims, start=opts)
                 self.tune_ms.append(t)
             self.engines.append(e)

@@ -104,6 +104,35 @@ def test_autotuned_plans_keep_their_tallies(oracle):
     pb.close()
 
 
+@pytest.mark.parametrize("histories", [10_000, 300_000, 5_000_000, 100_000_000])
+def test_a_plans_memory_stays_within_its_share(histories):
+    """Queues and drain stacks together, down to the smallest batch's queues."""
+    stacks = 3552 * (14 * 64 * 64 + 3 * 64 * 32)        # warps of the drain kernel x records, on the B200
+    for share in (1e8, 3.5e8, 5.6e8, 5.8e8, 6.25e8, 7e8, 9e8, 1.4e9, 3e9, 6e9, 2.2e10, 4e10):
+        o = choose_options(histories, share)
+        used = o["batch"] * 5.2e3 + (stacks if o["drain"] else 0)
+        assert used <= max(share, (1 << 16) * 5.2e3), (share, o)
+        assert o["drain"] == (share >= 5.8e8)           # where both fit
+
+
+@pytest.mark.gpu
+def test_a_batch_of_plans_stays_within_its_budget():
+    import torch
+    from gegs_b200.batch import PlanBatch
+    jobs = [W.config1(histories=300_000, n=10, voxel=3.0) for _ in range(8)]
+    warm = PlanBatch(jobs[:1], memory_budget_gb=1.0)     # the kernels' own memory
+    warm.run([1000])
+    warm.close()
+    for budget in (8 * 0.7, 8 * 0.4):
+        before = torch.cuda.mem_get_info(0)[0]
+        pb = PlanBatch(jobs, memory_budget_gb=budget)
+        stats = pb.run([2000] * 8)
+        used = before - torch.cuda.mem_get_info(0)[0]
+        pb.close()
+        assert all((s["waves"] == 2) == (budget > 5) for s in stats)   # drained where the stacks fit
+        assert used < budget * 1e9 + 8 * 30e6            # tables (5 MB), scene and graph of a plan besides
+
+
 class _Timed:
     """An engine whose runs take a made-up time: every other one is the fastest so far."""
     def __init__(self):
