@@ -527,15 +527,23 @@ static uint32_t default_batch(gegs_engine *e, uint64_t histories)
 static gegs_status ensure_queues(gegs_engine *e, uint32_t batch, uint32_t queue_cap)
 {
     if (batch == e->batch && queue_cap == e->queue_cap) return GEGS_OK;
-    for (int q = 0; q < GX_NQ; q++) {
+    e->batch = 0;                       // until all of them are there
+    cudaError_t c = cudaSuccess;
+    for (int q = 0; q < GX_NQ && c == cudaSuccess; q++) {
         uint64_t cap = (uint64_t)(kCapFactor[q] * (float)batch) + 4096;
         if (cap > 0xFFFFFFF0ull) cap = 0xFFFFFFF0ull;
         if (queue_cap && cap > queue_cap) cap = queue_cap;
-        CK(realloc_dev(&e->d_qbuf[q], (size_t)cap), "queue buffer");
+        c = realloc_dev(&e->d_qbuf[q], (size_t)cap);
         e->qcap[q] = (uint32_t)cap;
     }
-    for (int k = 0; k < GX_NESTATE; k++)
-        CK(realloc_dev(&e->d_estate[k], (size_t)e->qcap[GX_Q_ECONT + k]), "electron state");
+    for (int k = 0; k < GX_NESTATE && c == cudaSuccess; k++)
+        c = realloc_dev(&e->d_estate[k], (size_t)e->qcap[GX_Q_ECONT + k]);
+    if (c != cudaSuccess) {
+        cudaGetLastError();
+        for (int q = 0; q < GX_NQ; q++) realloc_dev(&e->d_qbuf[q], 0);
+        for (int k = 0; k < GX_NESTATE; k++) realloc_dev(&e->d_estate[k], 0);
+    }
+    CK(c, "queue buffers");
     e->batch = batch;
     e->queue_cap = queue_cap;
     e->ctx_gen++;

@@ -178,3 +178,24 @@ def test_history_outside_every_field_returns_source_error(engine, oracle):
         engine.run(0, job.histories + 50)
     assert err.value.status == ERR_SOURCE
     _assert_normal_run_matches_oracle(engine, oracle, job, sh)
+
+
+@pytest.mark.gpu
+def test_a_batch_too_large_for_the_device_leaves_the_engine_usable(oracle):
+    """The queues of the refused run are given back, and none of their pointers
+    is left for a run with the batch of before."""
+    import torch
+    from gegs_b200.engine import Engine
+    job = W.config1(histories=3000, n=16, voxel=2.0)
+    e = Engine(0)
+    sh = _fresh(e, job)
+    e.run(0, 3000, batch=4000)
+    free = torch.cuda.mem_get_info(0)[0]
+    with pytest.raises(GegsError) as err:
+        e.run(0, 3000, batch=100_000_000)             # 520 GB
+    assert err.value.status == 5                      # GEGS_ERR_NOMEM
+    assert torch.cuda.mem_get_info(0)[0] >= free
+    e.reset_tally()
+    e.run(0, 3000, batch=4000)
+    np.testing.assert_array_equal(e.tally(), oracle.run(job.physics, sh, 0, 3000)[0])
+    e.close()
