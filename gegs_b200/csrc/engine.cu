@@ -1203,8 +1203,10 @@ extern "C" gegs_status gegs_set_tally(gegs_engine *e, const int64_t *in, uint64_
     return GEGS_OK;
 }
 
-extern "C" gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
-                                           uint32_t *far_region, float *far_t, gegs_probe_state *far_out, float *near_t)
+// The probes of the geometry: the routines as they stand, or (with ranges) the forms that some steps take.
+static gegs_status probe_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
+                                  const float *range, uint32_t *far_region, float *far_t, gegs_probe_state *far_out,
+                                  float *near_t)
 {
     if (!e || !e->have_scene || !in || !t_in || !far_region || !far_t || !far_out || !near_t) return GEGS_ERR_ARG;
     if (e->in_flight) { e->err = "a launched run has not been waited for (gegs_wait)"; return GEGS_ERR_ARG; }
@@ -1212,13 +1214,16 @@ extern "C" gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const geg
     CK(cudaSetDevice(e->device), "cudaSetDevice");
     const size_t ns = (size_t)n * sizeof(gegs_probe_state), nf = (size_t)n * 4;
     char *d = nullptr;
-    CK(cudaMallocAsync(&d, 2 * ns + 4 * nf, e->stream), "probe buffers");
+    CK(cudaMallocAsync(&d, 2 * ns + 5 * nf, e->stream), "probe buffers");
     gegs_probe_state *d_in = (gegs_probe_state *)d, *d_out = (gegs_probe_state *)(d + ns);
-    float *d_t = (float *)(d + 2 * ns), *d_ft = d_t + n, *d_near = d_t + 2 * (size_t)n;
+    float *d_t = (float *)(d + 2 * ns), *d_ft = d_t + n, *d_near = d_t + 2 * (size_t)n, *d_range = d_t + 4 * (size_t)n;
     uint32_t *d_reg = (uint32_t *)(d_t + 3 * (size_t)n);
     CK(cudaMemcpyAsync(d_in, in, ns, cudaMemcpyHostToDevice, e->stream), "probe H2D");
     CK(cudaMemcpyAsync(d_t, t_in, nf, cudaMemcpyHostToDevice, e->stream), "probe H2D");
-    k_probe_geometry<<<(n + 127) / 128, 128, 0, e->stream>>>(e->ctx, n, d_in, d_t, d_reg, d_ft, d_out, d_near);
+    if (range) {
+        CK(cudaMemcpyAsync(d_range, range, nf, cudaMemcpyHostToDevice, e->stream), "probe H2D");
+        k_probe_step_geometry<<<(n + 127) / 128, 128, 0, e->stream>>>(e->ctx, n, d_in, d_t, d_range, d_reg, d_ft, d_out, d_near);
+    } else k_probe_geometry<<<(n + 127) / 128, 128, 0, e->stream>>>(e->ctx, n, d_in, d_t, d_reg, d_ft, d_out, d_near);
     CK(cudaGetLastError(), "probe kernel");
     CK(cudaMemcpyAsync(far_region, d_reg, nf, cudaMemcpyDeviceToHost, e->stream), "probe D2H");
     CK(cudaMemcpyAsync(far_t, d_ft, nf, cudaMemcpyDeviceToHost, e->stream), "probe D2H");
@@ -1227,6 +1232,20 @@ extern "C" gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const geg
     cudaFreeAsync(d, e->stream);
     CK(cudaStreamSynchronize(e->stream), "probe sync");
     return GEGS_OK;
+}
+
+extern "C" gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
+                                           uint32_t *far_region, float *far_t, gegs_probe_state *far_out, float *near_t)
+{
+    return probe_geometry(e, n, in, t_in, nullptr, far_region, far_t, far_out, near_t);
+}
+
+extern "C" gegs_status gegs_probe_step_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
+                                                const float *range, uint32_t *far_region, float *far_t,
+                                                gegs_probe_state *far_out, float *near_t)
+{
+    if (!range) return GEGS_ERR_ARG;
+    return probe_geometry(e, n, in, t_in, range, far_region, far_t, far_out, near_t);
 }
 
 extern "C" gegs_status gegs_get_dose(gegs_engine *e, const float *voxel_mass, double dose_unit, double *out, uint64_t nvox)

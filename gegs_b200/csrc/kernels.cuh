@@ -584,6 +584,55 @@ __global__ void k_probe_geometry(const __grid_constant__ DevCtx C, uint32_t n, c
     near_t[i] = tp;
 }
 
+// The forms of the same routines that only some steps take: howfar by the whole
+// warp, one state after another (share_steps), and hownear as an electron step
+// with tustep t_in and the given range (negative: no range rejection) uses it.
+__global__ void k_probe_step_geometry(const __grid_constant__ DevCtx C, uint32_t n, const gegs_probe_state *in,
+                                      const float *t_in, const float *range, uint32_t *far_region, float *far_t,
+                                      gegs_probe_state *far_out, float *near_t)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool have = i < n;
+    gegs_probe_state s = {};
+    if (have) s = in[i];
+    const Part p = probe_part(s);
+    const float t = have ? t_in[i] : 0.0f;
+    for (unsigned m = __ballot_sync(0xffffffffu, have); m; m &= m - 1u) {
+        const int src = __ffs(m) - 1;
+        Part q = part_of(p, src);
+        float tq = __shfl_sync(0xffffffffu, t, src);
+        bool ok;
+        uint32_t region;
+        switch (geom_class_of(q.module)) {
+        case GX_GEOM_JAWS: region = howfar_g<GX_GEOM_JAWS, true>(C, q, tq, ok); break;
+        case GX_GEOM_MLC: region = howfar_g<GX_GEOM_MLC, true>(C, q, tq, ok); break;
+        default: region = howfar(C, q, tq, ok);
+        }
+        __syncwarp();
+        if ((int)(threadIdx.x & 31u) == src) {
+            far_region[i] = region;
+            far_t[i] = tq;
+            gegs_probe_state o = s;
+            o.leafIndex = q.leafIndex; o.bank = q.bank; o.module = q.module;
+            far_out[i] = o;
+        }
+    }
+    if (!have) return;
+    Part q = p;
+    NearUse use;
+    use.rr = range[i] >= 0.0f;
+    use.range = range[i];
+    use.tustep = t;
+    float tp = 0.0f;
+    bool ok;
+    switch (geom_class_of(q.module)) {
+    case GX_GEOM_JAWS: hownear_g<GX_GEOM_JAWS>(C, q, tp, ok, use); break;
+    case GX_GEOM_MLC: hownear_g<GX_GEOM_MLC>(C, q, tp, ok, use); break;
+    default: hownear(C, q, tp, ok);
+    }
+    near_t[i] = tp;
+}
+
 __global__ void k_dose(const unsigned long long *tally, const float *mass, double unit, double *out, uint64_t n)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {

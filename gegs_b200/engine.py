@@ -22,7 +22,7 @@ EXPORTS = ["gegs_set_trace", "gegs_get_trace", "gegs_set_timeline", "gegs_get_ti
            "gegs_run", "gegs_reset_tally", "gegs_get_tally", "gegs_set_tally", "gegs_get_dose", "gegs_get_stats",
            "gegs_tally_device_ptr", "gegs_run_noalloc", "gegs_launch", "gegs_wait", "gegs_launch_group", "gegs_probe_geometry", "gegs_set_stream", "gegs_set_field", "gegs_set_beamlet_weights", "gegs_backward", "gegs_sizeof_physics", "gegs_sizeof_scene", "gegs_sizeof_field", "gegs_version",
            "gegs_check_physics", "gegs_stat_begin", "gegs_stat_fold", "gegs_stat_get", "gegs_set_drain_stack",
-           "gegs_set_drain_turns"]
+           "gegs_set_drain_turns", "gegs_probe_step_geometry"]
 
 
 TRACE_DTYPE = np.dtype([("kind_stage", "<u4"), ("hist_lo", "<u4"), ("sid_lo", "<u4"), ("sid_hi", "<u4"),
@@ -85,6 +85,7 @@ def load_library(path=None):
     L.gegs_wait.argtypes = [vp]
     L.gegs_launch_group.argtypes = [vp, C.c_int32, vp, vp, vp]
     L.gegs_probe_geometry.argtypes = [vp, C.c_uint32, vp, vp, vp, vp, vp, vp]
+    L.gegs_probe_step_geometry.argtypes = [vp, C.c_uint32, vp, vp, vp, vp, vp, vp, vp]
     L.gegs_set_stream.argtypes = [vp, vp]
     L.gegs_set_drain_stack.argtypes = [vp, C.c_uint32]
     L.gegs_set_drain_turns.argtypes = [vp, C.c_uint32]
@@ -234,10 +235,12 @@ class Engine:
         handle = getattr(stream, "cuda_stream", stream)
         self._check(self.L.gegs_set_stream(self.h, handle))
 
-    def probe_geometry(self, states, t_in):
+    def probe_geometry(self, states, t_in, limit=None):
         """howfar (step t_in) and hownear of each state on the device
         (gegs_probe_geometry): region entered, step, state after howfar, and
-        the distance to the nearest boundary."""
+        the distance to the nearest boundary. With `limit`, the electron range
+        per state (negative: no range rejection), the forms that only some
+        steps take (gegs_probe_step_geometry)."""
         s = np.ascontiguousarray(states, PROBE_DTYPE)
         t = np.ascontiguousarray(t_in, np.float32)
         n = len(s)
@@ -245,8 +248,16 @@ class Engine:
         ft = np.zeros(n, np.float32)
         out = np.zeros(n, PROBE_DTYPE)
         near = np.zeros(n, np.float32)
-        self._check(self.L.gegs_probe_geometry(self.h, n, s.ctypes.data, t.ctypes.data, reg.ctypes.data,
-                                               ft.ctypes.data, out.ctypes.data, near.ctypes.data))
+        if limit is None:
+            self._check(self.L.gegs_probe_geometry(self.h, n, s.ctypes.data, t.ctypes.data, reg.ctypes.data,
+                                                   ft.ctypes.data, out.ctypes.data, near.ctypes.data))
+        else:
+            r = np.ascontiguousarray(limit, np.float32)
+            if r.shape != t.shape:
+                raise ValueError("one range per state")
+            self._check(self.L.gegs_probe_step_geometry(self.h, n, s.ctypes.data, t.ctypes.data, r.ctypes.data,
+                                                        reg.ctypes.data, ft.ctypes.data, out.ctypes.data,
+                                                        near.ctypes.data))
         return dict(region=reg, t=ft, particle=out, tperp=near)
 
     @staticmethod

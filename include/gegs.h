@@ -278,6 +278,15 @@ typedef struct gegs_probe_state {
 gegs_status gegs_probe_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
                                 uint32_t *far_region, float *far_t, gegs_probe_state *far_out, float *near_t);
 
+/* The same for the forms of these routines that only some steps take: howfar as
+ * a warp computes it together for a few photons left over, and hownear as an
+ * electron step t_in[i] of the given range (negative: without range rejection)
+ * uses it, where a value that leaves both comparisons as they are may stand in
+ * for the distance. */
+gegs_status gegs_probe_step_geometry(gegs_engine *e, uint32_t n, const gegs_probe_state *in, const float *t_in,
+                                     const float *range, uint32_t *far_region, float *far_t,
+                                     gegs_probe_state *far_out, float *near_t);
+
 /* Device pointer of the tally (for callers that keep results in HBM). */
 gegs_status gegs_tally_device_ptr(gegs_engine *e, void **out);
 
