@@ -256,7 +256,7 @@ __device__ __forceinline__ bool at_rest_mark(const Part &p) { return p.e == 0.0f
 // scoring and the ways out of all branches meet at one place each. Inlined per
 // branch they made kernels of 210 to 280 KB that waited for instructions more
 // than for anything else (22 cycles per issue in the jaws, 7 in the MLC); now
-// they take 83 to 92 KB. With the polygon routines (dev_geom.cuh) and the random
+// they take 79 to 93 KB. With the polygon routines (dev_geom.cuh) and the random
 // window in shared memory: CT head 5-field plan, 16M histories, 381 to 285 ms;
 // 1M histories 70 to 52 ms; slab, 5M histories, 96 to 90 ms.
 template <int G = GX_GEOM_ALL, bool DEFER = false, bool ONLY_NEAR = false>

@@ -161,7 +161,8 @@ static __device__ void hownear_phantom(const DevCtx &C, const Part &p0, float &t
 // loop over its polygons, the loops over edges stay rolled and without
 // branches, and what only few edges need (the divisions) follows for those
 // edges alone, picked out by a bit mask. The photon kernels of the jaws and the
-// MLC went from 97 and 83 KB to 30 and 33 KB (times: electron_step).
+// MLC went from 97 and 83 KB to 30 and 33 KB, 50 and 62 KB with the second step
+// that the warp shares (share_steps; times: electron_step).
 __device__ __forceinline__ float2 ld2(const float2 *a) { return __ldg(a); }
 
 static __device__ __noinline__ int point_in_polygon(float px, float py, const float2 *poly, int n)
@@ -594,7 +595,6 @@ static __device__ uint32_t howfar_secjaws(const DevCtx &C, Part &p, float &t)
 
 // ---- hownear -----------------------------------------------------------------
 __device__ __forceinline__ float dist2p(float2 v, float2 w) { return (v.x - w.x) * (v.x - w.x) + (v.y - w.y) * (v.y - w.y); }
-__device__ __forceinline__ float distp(float2 v, float2 w) { return sqrtf((v.x - w.x) * (v.x - w.x) + (v.y - w.y) * (v.y - w.y)); }
 
 // Squared distance whose sqrtf is point_dist_to_segment(p, v, w), term for term.
 __device__ __forceinline__ float point_dist2_to_segment(float2 p, float2 v, float2 w)

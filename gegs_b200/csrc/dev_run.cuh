@@ -164,8 +164,8 @@ __device__ __forceinline__ void run_interaction(const DevCtx &C, const Part &p, 
     }
 }
 
-// Entries an interaction kernel counts as processed: all but the positrons
-// handed over at rest (counted nowhere in the serial form either).
+// Entries an interaction kernel counts as processed: all but the positrons that
+// stopped in the electron transport (`processed` counts annihilations in flight).
 template <int Q>
 __device__ __forceinline__ unsigned counted(const Part &p)
 {

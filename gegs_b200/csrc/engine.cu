@@ -154,7 +154,7 @@ static cudaError_t realloc_dev(T **p, size_t n)
 }
 
 // Unit normal form (a, b, c), a*x + b*y = c, of the line through each edge of
-// the polygons that hownear_secjaws_y / _x measure (the bounding polygon and
+// the polygons that hownear_secjaws measures (the bounding polygon and
 // the jaw opening), per field and jaw: [field][jaw: Y, X][8]. |a*x + b*y - c|
 // is at most the distance to the edge, so the smallest over the eight lines
 // bounds hownear from below (jaws_near_lower_bound). A zero-length edge gets

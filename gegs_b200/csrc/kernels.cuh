@@ -154,9 +154,10 @@ __device__ __forceinline__ bool refill(const DevCtx &C, int hq, uint32_t n_cont,
 #ifndef GX_ELECTRON_MIN_BLOCKS
 #define GX_ELECTRON_MIN_BLOCKS 2
 #endif
-// the phantom electrons: 64 registers. Its step spills some 280 bytes there
-// against about 100 at 80 registers, yet the fourth block per SM hides more of
-// the loads' latency: 2.1 % faster on C3 (5 blocks, 48 registers: 2.2 % slower)
+// the phantom electrons: 64 registers. Its step spills there (224 bytes of
+// stores, 428 of loads; 160 and 224 at 80 registers), yet the fourth block per
+// SM hides as much of the loads' latency: the same time at 3 blocks, 3.5 %
+// slower at 5 (48 registers)
 #ifndef GX_EPHANTOM_MIN_BLOCKS
 #define GX_EPHANTOM_MIN_BLOCKS 4
 #endif
