@@ -658,12 +658,14 @@ def main():
         cpu = {"value": crate, "unit": "histories/s", "cores": cores, "kind": "port",
                "sample": f"{cn} C3 histories in {cdt:.1f} s on {cores} host threads (CPU oracle, same inputs)",
                "value_1_core": r1, "sample_1_core": f"{n1} C3 histories in {dt1:.1f} s on 1 thread"}
-    # per step: the first planner launch, then per wave the kernels of one wave and the planner.
-    # Plain form: source + 10 stage kernels + planner. Timed form: source, photon jaws / MLC /
-    # phantom, 4 photon interactions, electron jaws + near pass, MLC + near pass, phantom, 4
-    # electron interactions, planner. Persistent form: the same plus the long jaws-photon kernel.
-    per_wave = {"plain": 12, "timed": 18}.get(args.mode, 19)
-    launches_per_step = [1 + per_wave * (st["waves"] - 1) for st in stats]
+    # per step: the first planner launch, then per wave the kernels of one wave and the planner
+    # (`waves` counts the plans). Plain form: source + 10 stage kernels + planner. Timed and
+    # persistent form: source, photon jaws / MLC / phantom, 4 photon interactions, electron jaws +
+    # near pass, MLC + near pass, phantom, 4 electron interactions, planner. In the persistent form
+    # without step budgets the drain kernel follows, and one that plans once more behind it.
+    per_wave = 12 if args.mode == "plain" else 18
+    drains = args.mode == "persistent" and not (args.photon_budget or args.electron_budget)
+    launches_per_step = [1 + per_wave * (st["waves"] - 1 - drains) + 2 * drains for st in stats]
     line = {
         "metric": METRIC, "value": value, "unit": "histories/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": elapsed_s * 1e3 / args.steps, "higher_is_better": True,
