@@ -409,6 +409,18 @@ int drain_blocks_per_sm(bool head)
     return c == cudaSuccess && n > 0 ? n : 1;
 }
 
+size_t drain_frames(bool head)
+{
+    cudaFuncAttributes a;
+    int device = 0, sms = 0, threads = 0;
+    if ((head ? cudaFuncGetAttributes(&a, k_drain<true>) : cudaFuncGetAttributes(&a, k_drain<false>)) != cudaSuccess ||
+        cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&threads, cudaDevAttrMaxThreadsPerMultiProcessor, device) != cudaSuccess)
+        return (size_t)1 << 30;
+    return a.localSizeBytes * (size_t)sms * (size_t)threads + ((size_t)64 << 20);
+}
+
 void launch_drain(const DevCtx &C, SchedState *st, bool head, int grid, cudaStream_t s)
 {
     if (head) k_drain<true><<<grid, kDrainThreads, 0, s>>>(C, st);

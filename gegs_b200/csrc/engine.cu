@@ -770,8 +770,13 @@ static uint32_t drain_threshold(const gegs_run_opts &o, uint32_t batch)
     return most < batch / 2u ? most : batch / 2u;
 }
 
-// The drain kernel's stacks; false if there is no memory for them (the run then
-// goes on in waves to its end).
+// The drain kernel's stacks; false if there is no room for them (the run then goes
+// on in waves to its end). There has to be room for the frames of the kernel's
+// threads besides, which the driver sets aside at a process's first launch of it
+// (whether it has is not known, so 0.5 GB each time): a launch for which it cannot
+// do so fails, and a graph launched after that has accessed frames that were gone.
+// So that the room is still there when they are set aside, the kernel is launched
+// here, with nothing to drain.
 static bool ensure_drain(gegs_engine *e)
 {
     const int grid = e->nsm * drain_blocks_per_sm(e->has_head);
@@ -779,14 +784,27 @@ static bool ensure_drain(gegs_engine *e)
     const size_t warps = (size_t)grid * (kDrainThreads / 32);
     if (e->drain_grid) e->ctx_gen++;            // graphs with the old stacks
     e->drain_grid = 0;
-    if (realloc_dev(&e->d_drain_part, warps * GX_DT_N * GX_DRAIN_CAP) == cudaSuccess &&
-        realloc_dev(&e->d_drain_estate, warps * 3 * GX_DRAIN_CAP) == cudaSuccess) {
+    const size_t parts = warps * GX_DT_N * GX_DRAIN_CAP, states = warps * 3 * GX_DRAIN_CAP;
+    realloc_dev(&e->d_drain_part, 0);
+    realloc_dev(&e->d_drain_estate, 0);
+    size_t free_b = 0, total_b = 0;
+    cudaError_t c = cudaMemGetInfo(&free_b, &total_b);
+    if (c == cudaSuccess && free_b < parts * sizeof(Part) + states * sizeof(EStatePk) + drain_frames(e->has_head))
+        c = cudaErrorMemoryAllocation;
+    if (c == cudaSuccess) c = realloc_dev(&e->d_drain_part, parts);
+    if (c == cudaSuccess) c = realloc_dev(&e->d_drain_estate, states);
+    if (c == cudaSuccess) c = cudaMemsetAsync(e->d_sched, 0, sizeof(SchedState), e->stream);
+    if (c == cudaSuccess) {
+        launch_drain(e->ctx, e->d_sched, e->has_head, grid, e->stream);
+        c = cudaGetLastError();
+    }
+    if (c == cudaSuccess) {
         e->drain_grid = grid;
         e->ctx_gen++;
     } else {
         cudaGetLastError();
-        cudaFree(e->d_drain_part);
-        e->d_drain_part = nullptr;
+        realloc_dev(&e->d_drain_part, 0);
+        realloc_dev(&e->d_drain_estate, 0);
     }
     e->ctx.drain_part = e->d_drain_part;
     e->ctx.drain_estate = e->d_drain_estate;

@@ -279,3 +279,38 @@ def test_a_particle_that_does_not_end_uses_up_the_waves(engine):
         engine.set_drain_turns(0)
     assert err.value.status == 6                      # GEGS_ERR_STEP_BUDGET
     assert engine.stats()["waves"] == 6
+
+
+def test_without_memory_for_the_kernels_own_frames_a_run_goes_in_waves():
+    """A process whose first run of the drain kernel would find room for the stacks
+    (228 MB), but not for the frames of its threads (190 MB more): it must not be
+    launched."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import numpy as np, torch
+from gegs_b200 import workloads as W
+from gegs_b200.engine import Engine
+job = W.config3(histories=3000, nphsp=5000, dims=(40, 40, 20))
+e = Engine(0)
+e.set_physics(job.physics)
+e.set_scene(job.scene())
+e.run(0, 3000, batch=1 << 16, drain=False)
+want = e.tally()
+held = torch.empty(torch.cuda.mem_get_info(0)[0] - (300 << 20), dtype=torch.uint8, device="cuda")
+for last in (False, True):
+    for _ in range(2):
+        e.reset_tally()
+        st = e.run(0, 3000, batch=1 << 16)
+        np.testing.assert_array_equal(e.tally(), want)
+        assert (st["waves"] == 2) == last, st["waves"]
+    held = None
+    torch.cuda.empty_cache()
+e.close()
+print("as it should be")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "as it should be" in r.stdout, r.stdout + r.stderr
