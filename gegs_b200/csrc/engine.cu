@@ -94,6 +94,7 @@ struct gegs_engine {
     Part *d_drain_part = nullptr;
     EStatePk *d_drain_estate = nullptr;
     int drain_grid = 0;
+    bool drain_head = false;           // room was made for the kernel with the jaws and the MLC (the larger frames)
     int run_grid = 0, run_threads = 0; // launch shape of the last run's waves
     bool has_head = true;              // the scene's modules include jaws or an MLC (or one this path does not model)
 
@@ -780,7 +781,7 @@ static uint32_t drain_threshold(const gegs_run_opts &o, uint32_t batch)
 static bool ensure_drain(gegs_engine *e)
 {
     const int grid = e->nsm * drain_blocks_per_sm(e->has_head);
-    if (e->drain_grid == grid) return true;
+    if (e->drain_grid == grid && (e->drain_head || !e->has_head)) return true;
     const size_t warps = (size_t)grid * (kDrainThreads / 32);
     if (e->drain_grid) e->ctx_gen++;            // graphs with the old stacks
     e->drain_grid = 0;
@@ -800,6 +801,7 @@ static bool ensure_drain(gegs_engine *e)
     }
     if (c == cudaSuccess) {
         e->drain_grid = grid;
+        e->drain_head = e->has_head;
         e->ctx_gen++;
     } else {
         cudaGetLastError();

@@ -281,19 +281,26 @@ def test_a_particle_that_does_not_end_uses_up_the_waves(engine):
     assert engine.stats()["waves"] == 6
 
 
-def test_without_memory_for_the_kernels_own_frames_a_run_goes_in_waves():
+@pytest.mark.parametrize("phantom_first", [False, True])
+def test_without_memory_for_the_kernels_own_frames_a_run_goes_in_waves(phantom_first):
     """A process whose first run of the drain kernel would find room for the stacks
     (228 MB), but not for the frames of its threads (190 MB more): it must not be
-    launched."""
+    launched. With `phantom_first` the engine has drained a plan without jaws and
+    MLC, whose kernel has smaller frames."""
     import os
     import subprocess
     import sys
-    code = """
+    code = f"phantom_first = {phantom_first}" + """
 import numpy as np, torch
 from gegs_b200 import workloads as W
 from gegs_b200.engine import Engine
 job = W.config3(histories=3000, nphsp=5000, dims=(40, 40, 20))
 e = Engine(0)
+if phantom_first:
+    slab = W.config2(histories=1000, nphsp=1000, n=20)
+    e.set_physics(slab.physics)
+    e.set_scene(slab.scene())
+    assert e.run(0, 1000, batch=1 << 16)["waves"] == 2
 e.set_physics(job.physics)
 e.set_scene(job.scene())
 e.run(0, 3000, batch=1 << 16, drain=False)
